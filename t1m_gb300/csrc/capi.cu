@@ -279,7 +279,10 @@ int choose_splits(const t1m_context* ctx, int method, int dtype, int64_t M, int6
   const int64_t tiles = ((M + bm - 1) / bm) * ((N + bn - 1) / bn);
   const int64_t ksteps = (K + bk - 1) / bk;
   int64_t s = 1;
-  if (ctx->split_k > 0) {
+  if (method == T1M_METHOD_PLAIN && ctx->split_k == 0 &&
+      (dtype == T1M_FLOAT64 || dtype == T1M_COMPLEX128)) {
+    s = fp64_form(dtype, M, N, K, 0).splits;
+  } else if (ctx->split_k > 0) {
     s = ctx->split_k;
   } else {
     const int64_t target = int64_t(ctx->num_sms) * per_sm;

@@ -1,0 +1,301 @@
+// float64 / complex128 contraction in FP64 FMAs on small output tiles.
+//
+// GB300 issues two FP64 FMAs per clock and SM (1.25 TFLOP/s nominal), so a
+// warp's FMA occupies its scheduler for 64 clocks and everything else of the
+// loop (shared-memory reads, copies, address arithmetic) hides behind it even
+// with one output per thread.  What bounds a product is how evenly its FMAs
+// spread over the 152 SMs and how many of them are padding.  Hence the small
+// tiles: a 128 x 64 tile of 256 threads (the FP32 kernel's shape) takes an SM
+// 16 us per 8 k of float64, whatever part of it lies inside the output.
+//   16 x 16 outputs: two per thread;
+//   8 x 8 outputs:   one per thread, the two halves of the block taking
+//                    alternate k and added in a fixed order at the end, for
+//                    outputs with too few tiles to occupy every SM.
+// Steps past K are not computed, and a warp whose outputs all lie past the edge
+// computes nothing.
+// Measured (GB300): complex128 1024^3 8.23 -> 6.95 ms (1.24 TFLOP/s), float64
+// 9216 x 96 x 96 283 -> 195 us per synchronous call, 98% of the 2-FMA rate in
+// the first.
+//
+// Tiles are gathered through the scatter vectors as in simt.cu (the plain
+// form; replaces the reference's include/t1m/t1m.h:432-557 in FP64), each
+// operand's unit-stride direction on consecutive threads, through a
+// three-stage cp.async ring.  Consecutive threads write along C's unit stride.
+#include <algorithm>
+#include <cstdint>
+
+#include "internal.h"
+#include "simt_common.h"
+#include "t1m_capi.h"
+
+namespace t1m {
+namespace gb300 {
+namespace {
+
+constexpr int kThreads64 = 128;
+constexpr int kBK64 = 16;      // k per stage
+constexpr int kStages64 = 3;
+
+// Conjugation by the sign bit: a floating negation of a value that is not an
+// FMA operand would go through the FP64 pipe (measured: half as many FP64
+// instructions again, complex128 1024^3 10.5 ms against 7.1).
+__device__ __forceinline__ double flip(double v, uint64_t) { return v; }
+__device__ __forceinline__ double2 flip(double2 v, uint64_t sign) {
+  v.y = __longlong_as_double(__double_as_longlong(v.y) ^ static_cast<long long>(sign));
+  return v;
+}
+
+template <class T, int kTile>
+struct Smem64 {
+  static constexpr int kPad = 32 / sizeof(T);
+  T a[kStages64][kBK64][kTile + kPad];
+  T b[kStages64][kBK64][kTile + kPad];
+  T part[kTile * kTile];  // the second k slice's sums (8 x 8 form)
+  int64_t row_a[kTile], col_b[kTile];
+};
+
+// One output tile over the K range of `split`.  kTile: 16 or 8 rows and
+// columns.  kNFast: consecutive threads along n (C unit stride along its
+// columns), else along m.
+template <class T, int kTile, bool kNFast>
+__device__ __forceinline__ void fp64_tile(const GemmArgs& args, int64_t tile, int64_t split,
+                                          Smem64<T, kTile>& sm) {
+  constexpr int kOut = kTile * kTile >= kThreads64 ? kTile * kTile / kThreads64 : 1;
+  constexpr int kSlices = kThreads64 * kOut / (kTile * kTile);  // k slices of the block
+  constexpr int kSlow = kTile / kOut;                           // step between a thread's outputs
+  auto& As = sm.a;
+  auto& Bs = sm.b;
+  int64_t* const rowA = sm.row_a;
+  int64_t* const colB = sm.col_b;
+
+  const T* __restrict__ A = static_cast<const T*>(args.A);
+  const T* __restrict__ B = static_cast<const T*>(args.B);
+  const int64_t M = args.M, N = args.N;
+  const int64_t tiles_m = (M + kTile - 1) / kTile, tiles_n = (N + kTile - 1) / kTile;
+  const int64_t kb = split * args.k_per_split;
+  const int64_t K = min(args.K, kb + args.k_per_split);
+  T* __restrict__ C = static_cast<T*>(args.C) + split * args.c_split_stride;
+  const uint64_t signA = args.flags & kFlagConjA ? uint64_t(1) << 63 : 0;
+  const uint64_t signB = args.flags & kFlagConjB ? uint64_t(1) << 63 : 0;
+  // Groups of 32 M-tiles sweep N, so blocks running together share operands.
+  constexpr int64_t G = 32;
+  const int64_t first_m = (tile / (G * tiles_n)) * G;
+  const int64_t gsize = min(G, tiles_m - first_m);
+  const int64_t r = tile % (G * tiles_n);
+  const int64_t m0 = (first_m + r % gsize) * kTile, n0 = (r / gsize) * kTile;
+
+  const int tid = threadIdx.x;
+  if (tid < kTile) {
+    rowA[tid] = m0 + tid < M ? offs(args.rsA, args.uA_m, m0 + tid) : 0;
+  } else if (tid < 2 * kTile) {
+    const int n = tid - kTile;
+    colB[n] = n0 + n < N ? offs(args.csB, args.uB_n, n0 + n) : 0;
+  }
+  __syncthreads();
+
+  const bool a_kfast = args.uA_k == 1;
+  const bool b_kfast = args.uB_k == 1 || args.uB_n != 1;
+  constexpr int kPer = kTile * kBK64 / kThreads64;
+  static_assert(kPer * kThreads64 == kTile * kBK64, "stage copies");
+  auto issue = [&](int64_t k0, int buf) {
+#pragma unroll
+    for (int p = 0; p < kPer; ++p) {
+      const int idx = tid + p * kThreads64;
+      const int m = a_kfast ? idx / kBK64 : idx % kTile;
+      const int k = a_kfast ? idx % kBK64 : idx / kTile;
+      const bool in = m0 + m < M && k0 + k < K;
+      cp_async_elem<sizeof(T)>(&As[buf][k][m],
+                               in ? A + rowA[m] + offs(args.csA, args.uA_k, k0 + k) : A, in);
+    }
+#pragma unroll
+    for (int p = 0; p < kPer; ++p) {
+      const int idx = tid + p * kThreads64;
+      const int n = b_kfast ? idx / kBK64 : idx % kTile;
+      const int k = b_kfast ? idx % kBK64 : idx / kTile;
+      const bool in = n0 + n < N && k0 + k < K;
+      cp_async_elem<sizeof(T)>(&Bs[buf][k][n],
+                               in ? B + offs(args.rsB, args.uB_k, k0 + k) + colB[n] : B, in);
+    }
+  };
+
+  // Outputs of this thread: index `f` along the fast dimension, s + kSlow j
+  // along the other.
+  const int f = tid % kTile, s = (tid / kTile) % kSlow, slice = tid / (kTile * kSlow);
+  const int64_t fast_n = (kNFast ? N - n0 : M - m0), slow_n = (kNFast ? M - m0 : N - n0);
+  bool live[kOut];
+#pragma unroll
+  for (int j = 0; j < kOut; ++j) live[j] = f < fast_n && s + kSlow * j < slow_n;
+  // Four FMA chains per output (k mod 4, over the slices), added at the end:
+  // shorter chains than one per K range round less.
+  constexpr int kChains = 4 / kSlices;
+  T part[kOut][kChains];
+#pragma unroll
+  for (int j = 0; j < kOut; ++j)
+#pragma unroll
+    for (int u = 0; u < kChains; ++u) part[j][u] = zero<T>();
+
+  const int64_t ksteps = K > kb ? (K - kb + kBK64 - 1) / kBK64 : 0;
+#pragma unroll
+  for (int st = 0; st < kStages64 - 1; ++st) {
+    if (st < ksteps) issue(kb + st * kBK64, st);
+    cp_async_commit_group();
+  }
+  for (int64_t st = 0; st < ksteps; ++st) {
+    const int buf = static_cast<int>(st % kStages64);
+    cp_async_wait_group<kStages64 - 2>();
+    __syncthreads();  // stage st has landed for every thread; stage st - 1 is consumed
+    const int64_t nxt = st + kStages64 - 1;
+    if (nxt < ksteps) issue(kb + nxt * kBK64, static_cast<int>(nxt % kStages64));
+    cp_async_commit_group();
+    const int kn = static_cast<int>(min(static_cast<int64_t>(kBK64), K - kb - st * kBK64));
+    auto step = [&](int k, int u) {
+      const T x = kNFast ? flip(Bs[buf][k][f], signB) : flip(As[buf][k][f], signA);
+#pragma unroll
+      for (int j = 0; j < kOut; ++j) {
+        if (!live[j]) continue;
+        const T y = kNFast ? flip(As[buf][k][s + kSlow * j], signA)
+                           : flip(Bs[buf][k][s + kSlow * j], signB);
+        if (kNFast) mac(part[j][u], y, x); else mac(part[j][u], x, y);
+      }
+    };
+    if (kn == kBK64) {
+#pragma unroll
+      for (int k = 0; k < kBK64; k += 4)
+#pragma unroll
+        for (int u = 0; u < kChains; ++u) step(k + u * kSlices + slice, u);
+    } else {
+      for (int k = 0; k < kn; k += 4)
+#pragma unroll
+        for (int u = 0; u < kChains; ++u)
+          if (k + u * kSlices + slice < kn) step(k + u * kSlices + slice, u);
+    }
+  }
+  cp_async_wait_group<0>();
+
+  T acc[kOut];
+#pragma unroll
+  for (int j = 0; j < kOut; ++j) {
+    acc[j] = part[j][0];
+#pragma unroll
+    for (int u = 1; u < kChains; ++u) acc[j] = add(acc[j], part[j][u]);
+  }
+  if constexpr (kSlices > 1) {
+    static_assert(kOut == 1 && kSlices == 2, "two k slices of one output per thread");
+    if (slice > 0) sm.part[tid % (kTile * kTile)] = acc[0];
+    __syncthreads();
+    if (slice > 0) return;
+    acc[0] = add(acc[0], sm.part[tid]);
+  }
+
+  const T alpha = scal<T>(args.alpha), beta = scal<T>(args.beta);
+  const bool accumulate = args.flags & kFlagAccumulate;
+  const bool beta_zero = args.flags & kFlagBetaZero;
+#pragma unroll
+  for (int j = 0; j < kOut; ++j) {
+    if (!live[j]) continue;
+    const int64_t m = m0 + (kNFast ? s + kSlow * j : f), n = n0 + (kNFast ? f : s + kSlow * j);
+    T* p = C + offs(args.rsC, args.uC_m, m) + offs(args.csC, args.uC_n, n);
+    const T ab = mul(alpha, acc[j]);
+    if (accumulate)
+      *p = add(*p, ab);
+    else if (beta_zero)
+      *p = ab;
+    else
+      *p = add(ab, mul(beta, *p));
+  }
+}
+
+// Grouped launches: blockIdx.x indexes the concatenated tile lists of
+// group[0..nprob) (sorted by tile_begin, split-major within a problem);
+// otherwise it is a tile of args0 and blockIdx.y its split.
+template <class T, int kTile, bool kGroup>
+__global__ void __launch_bounds__(kThreads64)
+fp64_contract(const GemmArgs args0, const SimtProblem* group, int nprob) {
+  __shared__ __align__(16) Smem64<T, kTile> sm;
+  __shared__ GemmArgs group_args;
+  int64_t tile = blockIdx.x, split = blockIdx.y;
+  if constexpr (kGroup) {
+    int lo = 0, hi = nprob - 1;
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (group[mid].tile_begin <= tile) lo = mid; else hi = mid - 1;
+    }
+    tile -= group[lo].tile_begin;
+    if (threadIdx.x == 0) group_args = group[lo].g;
+    __syncthreads();
+    const int64_t per = ((group_args.M + kTile - 1) / kTile) * ((group_args.N + kTile - 1) / kTile);
+    split = tile / per;
+    tile -= split * per;
+  }
+  const GemmArgs& args = kGroup ? group_args : args0;
+  if (args.uC_n == 1 && args.uC_m != 1)
+    fp64_tile<T, kTile, true>(args, tile, split, sm);
+  else
+    fp64_tile<T, kTile, false>(args, tile, split, sm);
+}
+
+template <class T>
+cudaError_t launch(const GemmArgs& g, int tile, int splits, cudaStream_t stream) {
+  const int64_t tiles = ((g.M + tile - 1) / tile) * ((g.N + tile - 1) / tile);
+  if (tiles == 0) return cudaSuccess;
+  if (tiles > 0x7fffffffLL || splits < 1 || splits > 65535) return cudaErrorInvalidConfiguration;
+  const dim3 grid(static_cast<unsigned>(tiles), static_cast<unsigned>(splits));
+  if (tile == 16)
+    fp64_contract<T, 16, false><<<grid, kThreads64, 0, stream>>>(g, nullptr, 0);
+  else
+    fp64_contract<T, 8, false><<<grid, kThreads64, 0, stream>>>(g, nullptr, 0);
+  return cudaGetLastError();
+}
+
+}  // namespace
+
+Fp64Form fp64_form(int dtype, int64_t M, int64_t N, int64_t K, int64_t forced) {
+  // Clocks of the busiest SM: whole blocks per SM times a block's FMAs at two
+  // per clock (four per complex product), plus 2000 for the fill of the copy
+  // ring and the epilogue, plus, when split, 6000 for the reduction launch
+  // and 1 per 8 bytes x SM of partials written and read back.
+  constexpr double kSms = 152;
+  const double fma = dtype == T1M_COMPLEX128 ? 4 : 1, es = dtype == T1M_COMPLEX128 ? 16 : 8;
+  const int64_t ksteps = std::max<int64_t>(1, (K + kBK64 - 1) / kBK64);
+  Fp64Form best{16, 1, ksteps * kBK64};
+  double best_cost = 1e300;
+  for (int tile : {16, 8}) {
+    const double tiles = double((M + tile - 1) / tile) * double((N + tile - 1) / tile);
+    for (int64_t s = forced > 0 ? forced : 1; s <= (forced > 0 ? forced : 64); ++s) {
+      if (s > 1 && s > ksteps) break;
+      const int64_t per = (ksteps + s - 1) / s;
+      const int64_t used = (ksteps + per - 1) / per;
+      if (forced <= 0 && used != s) continue;  // the same partition as a smaller s
+      const double waves = double(static_cast<int64_t>((tiles * used + kSms - 1) / kSms));
+      double cost = waves * tile * tile * double(std::min(K, per * kBK64)) * fma / 2 + 2000;
+      if (used > 1) cost += 6000 + 2.0 * double(used) * double(M) * double(N) * es / (8 * kSms);
+      if (cost < best_cost) {
+        best_cost = cost;
+        best = {tile, static_cast<int>(used), per * kBK64};
+      }
+    }
+  }
+  return best;
+}
+
+cudaError_t launch_fp64(int dtype, const GemmArgs& g, int splits, cudaStream_t stream) {
+  const int tile = fp64_form(dtype, g.M, g.N, g.K, splits).tile;
+  return dtype == T1M_COMPLEX128 ? launch<double2>(g, tile, splits, stream)
+                                 : launch<double>(g, tile, splits, stream);
+}
+
+cudaError_t launch_fp64_group(int dtype, const SimtProblem* dev, int nprob, int64_t total_tiles,
+                              cudaStream_t stream) {
+  if (total_tiles <= 0) return cudaSuccess;
+  if (total_tiles > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
+  const GemmArgs none{};
+  const unsigned grid = static_cast<unsigned>(total_tiles);
+  if (dtype == T1M_COMPLEX128)
+    fp64_contract<double2, kFp64Tile, true><<<grid, kThreads64, 0, stream>>>(none, dev, nprob);
+  else
+    fp64_contract<double, kFp64Tile, true><<<grid, kThreads64, 0, stream>>>(none, dev, nprob);
+  return cudaGetLastError();
+}
+
+}  // namespace gb300
+}  // namespace t1m

@@ -151,6 +151,21 @@ cudaError_t launch_simt(int dtype, const GemmArgs& args, int splits, cudaStream_
 // Output tile sizes of the plain kernel for a dtype (for split decisions).
 void simt_tile(int dtype, int* bm, int* bn, int* bk);
 
+// fp64.cu: the plain kernel of float64 / complex128.  Tile (16 or 8 rows and
+// columns), split count and K per split (a multiple of 16) of a product; with
+// `forced` > 0 that split count.
+struct Fp64Form {
+  int tile;
+  int splits;
+  int64_t k_per_split;
+};
+constexpr int kFp64Tile = 16;  // tile of grouped launches
+Fp64Form fp64_form(int dtype, int64_t M, int64_t N, int64_t K, int64_t forced);
+cudaError_t launch_fp64(int dtype, const GemmArgs& args, int splits, cudaStream_t stream);
+struct SimtProblem;
+cudaError_t launch_fp64_group(int dtype, const SimtProblem* dev, int nprob, int64_t total_tiles,
+                              cudaStream_t stream);
+
 // One contraction of a grouped plain launch (device array, sorted by
 // tile_begin).  Its tiles are numbered split-major: g.k_per_split and
 // g.c_split_stride describe split-K exactly as for a single launch, and the
