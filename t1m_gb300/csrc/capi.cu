@@ -410,13 +410,15 @@ int launch_product(t1m_context* ctx, int method, int dtype, size_t es, const Hos
         return ctx->opt_work_limit < 0 || bytes <= static_cast<size_t>(ctx->opt_work_limit);
       };
       // The panel workspace also holds operand pieces where they run.
-      const size_t pcb = tc_pieces_count(method, dtype, gm, hp, form) > 0
-                             ? tc_pieces_bytes(dtype, method, gm.M, gm.N, gm.K, ready)
-                             : 0;
-      const size_t pb = std::max(tc_panel_bytes(dtype, gm.M, gm.N, gm.K), pcb);
-      const bool pan = pb > 0 && within(pb) &&
-                       ensure_opt_work(s, &ctx->panel[slot], &ctx->panel_bytes[slot], pb);
-      const size_t kb = tc_pack_bytes(dtype, hp);
+      // Products over pieces need no dense packs.
+      const size_t pcb = tc_pieces_bytes(dtype, tc_pieces_count(method, dtype, gm, hp, form),
+                                         gm.M, gm.N, gm.K, ready);
+      const bool pieces = pcb > 0 && within(pcb) &&
+                          ensure_opt_work(s, &ctx->panel[slot], &ctx->panel_bytes[slot], pcb);
+      const size_t pb = tc_panel_bytes(dtype, gm.M, gm.N, gm.K);
+      const bool pan = pieces || (pb > 0 && within(pb) &&
+                                  ensure_opt_work(s, &ctx->panel[slot], &ctx->panel_bytes[slot], pb));
+      const size_t kb = pieces ? 0 : tc_pack_bytes(dtype, hp);
       const bool pk = kb > 0 && within(kb) &&
                       ensure_opt_work(s, &ctx->pack[slot], &ctx->pack_bytes[slot], kb);
       // Arrival counters for the persistent kernel's in-kernel reduction of
@@ -647,22 +649,23 @@ int run_pipelined(t1m_context* ctx, int method, int dtype, size_t es, const Host
   // split once, half by half after its copy (on the context stream), into
   // its own workspace; every block then splits only its streamed slab.
   const int npieces = tc_pieces_count(method, dtype, block_args(0, 0), hp, ctx->tile_form);
-  const int64_t ppitch = tc_pieces_pitch(hp.K);
-  const int64_t prows = sl.along_n ? 2 * hp.M : hp.N;   // rows of the resident pieces
-  const size_t pbytes = size_t(npieces) * size_t(prows) * size_t(ppitch) * 2u;
+  const int64_t pgroups = tc_pieces_groups(dtype, sl.along_n, sl.along_n ? hp.M : hp.N);
+  const size_t pbytes = tc_pieces_array_bytes(dtype, npieces, pgroups, hp.K);
   const bool res_pieces =
       npieces > 0 && (ctx->opt_work_limit < 0 || pbytes <= size_t(ctx->opt_work_limit)) &&
       ensure_opt_work(s, &ctx->res_pieces, &ctx->res_pieces_bytes, pbytes);
-  // Element offset of half h's first row in the resident pieces.
-  auto pieces_row0 = [&](int h) -> int64_t {
+  // Row groups start 512 bytes apart; halves and slabs are multiples of 128 rows.
+  auto groups_at = [](void* base, int64_t groups) -> void* {
+    return static_cast<unsigned char*>(base) + groups * 512;
+  };
+  auto res_at = [&](int h) -> void* {  // half h of the resident pieces
     const int64_t hlo = split ? h * half : 0;
-    return (sl.along_n ? 2 * hlo : hlo) * ppitch;
+    return groups_at(ctx->res_pieces, tc_pieces_groups(dtype, sl.along_n, hlo));
   };
   auto split_resident = [&](int h) -> cudaError_t {
     cudaStreamWaitEvent(s, ctx->pev[kEvRes + h], 0);
-    void* out = static_cast<uint16_t*>(ctx->res_pieces) + pieces_row0(h);
-    const cudaError_t r =
-        tc_split_operand(npieces, sl.along_n, block_args(0, h), out, prows * ppitch, s);
+    const cudaError_t r = tc_split_operand(dtype, npieces, sl.along_n, block_args(0, h), hp,
+                                           res_at(h), pgroups, s);
     if (r == cudaSuccess) ++kernels;
     cudaEventRecord(ctx->pev[kEvResPieces + h], s);
     return r;
@@ -671,15 +674,14 @@ int run_pipelined(t1m_context* ctx, int method, int dtype, size_t es, const Host
   // slab is used by two blocks; its first block splits it once into its own
   // rows of this workspace and the other block reuses them (the per-block
   // split did it twice: 16 splits of 42 MB moved at 4096^3 instead of 8).
-  const int64_t srows = sl.along_n ? hp.N : 2 * hp.M;  // rows of the streamed pieces
-  const size_t sbytes = size_t(npieces) * size_t(srows) * size_t(ppitch) * 2u;
+  const int64_t sgroups = tc_pieces_groups(dtype, !sl.along_n, sl.along_n ? hp.N : hp.M);
+  const size_t sbytes = tc_pieces_array_bytes(dtype, npieces, sgroups, hp.K);
   const bool slab_pieces =
       res_pieces && split &&
       (ctx->opt_work_limit < 0 || pbytes + sbytes <= size_t(ctx->opt_work_limit)) &&
       ensure_opt_work(s, &ctx->slab_pieces, &ctx->slab_pieces_bytes, sbytes);
-  auto slab_row0 = [&](int i) -> int64_t {
-    const int64_t lo = i * sl.width;
-    return (sl.along_n ? lo : 2 * lo) * ppitch;
+  auto slab_at = [&](int i) -> void* {
+    return groups_at(ctx->slab_pieces, tc_pieces_groups(dtype, !sl.along_n, i * sl.width));
   };
   std::vector<char> slab_split(sl.count, 0);
   auto launch_block = [&](int i, int h) -> int {
@@ -690,19 +692,18 @@ int run_pipelined(t1m_context* ctx, int method, int dtype, size_t es, const Host
     const GemmArgs gs = block_args(i, h);
     PiecesReady ready;
     if (res_pieces) {
-      const void* p = static_cast<const uint16_t*>(ctx->res_pieces) + pieces_row0(h);
       if (sl.along_n) {
-        ready.a = p;
-        ready.a_plane = prows * ppitch;
+        ready.a = res_at(h);
+        ready.a_groups = pgroups;
       } else {
-        ready.b = p;
-        ready.b_plane = prows * ppitch;
+        ready.b = res_at(h);
+        ready.b_groups = pgroups;
       }
     }
     if (slab_pieces) {
-      void* sp = static_cast<uint16_t*>(ctx->slab_pieces) + slab_row0(i);
+      void* sp = slab_at(i);
       if (!slab_split[i]) {
-        const cudaError_t r = tc_split_operand(npieces, !sl.along_n, gs, sp, srows * ppitch, cs);
+        const cudaError_t r = tc_split_operand(dtype, npieces, !sl.along_n, gs, hp, sp, sgroups, cs);
         if (r != cudaSuccess) return cuda_fail(ctx, r, "split streamed slab");
         ++kernels;
         cudaEventRecord(ctx->pev[kEvSlabPieces + i], cs);
@@ -712,10 +713,10 @@ int run_pipelined(t1m_context* ctx, int method, int dtype, size_t es, const Host
       }
       if (sl.along_n) {
         ready.b = sp;
-        ready.b_plane = srows * ppitch;
+        ready.b_groups = sgroups;
       } else {
         ready.a = sp;
-        ready.a_plane = srows * ppitch;
+        ready.a_groups = sgroups;
       }
     }
     if (int st = launch_product(ctx, method, dtype, es, hp, gs, cs, &kernels, &used_method,
@@ -1455,10 +1456,10 @@ bool tuned_product(t1m_context* ctx, int method, int dtype, size_t es, const Hos
         gm.c_split_stride = sp > 1 ? g.M * g.N : 0;
         GemmArgs red = gm;
         red.C = work + size_t(sp) * size_t(g.M) * size_t(g.N) * es;
-        const size_t pb = std::max(tc_panel_bytes(dtype, gm.M, gm.N, gm.K),
-                                   tc_pieces_count(method, dtype, gm, hp, f) > 0
-                                       ? tc_pieces_bytes(dtype, method, gm.M, gm.N, gm.K)
-                                       : size_t(0));
+        const size_t pb =
+            std::max(tc_panel_bytes(dtype, gm.M, gm.N, gm.K),
+                     tc_pieces_bytes(dtype, tc_pieces_count(method, dtype, gm, hp, f), gm.M, gm.N,
+                                     gm.K));
         const bool pan = pb > 0 && (ctx->opt_work_limit < 0 || pb <= size_t(ctx->opt_work_limit)) &&
                          ensure_opt_work(s, &ctx->panel[slot], &ctx->panel_bytes[slot], pb);
         const size_t kb = tc_pack_bytes(dtype, hp);

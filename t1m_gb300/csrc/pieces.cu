@@ -1,0 +1,901 @@
+// Operand pieces: products of complex64 / float32 operands split once into
+// bf16 pieces, on CTA pairs whose MMAs read both operands from shared memory.
+//
+// split_pieces writes every operand element's P bf16 pieces (the split of
+// tc_common.h, conjugation first) in the layout of pieces.h: for complex A the
+// 1M rows [re, -im, ...] and [im, re, ...] of every row (t1m.h:309-325), for
+// B the row [re, im, ...] of every column, real k = 2 k + part; for real
+// operands the rows themselves.  It replaces the reference's per-block
+// packing (t1m.h:309-337): once per operand instead of once per tile.
+//
+// tc1m_pieces then runs the real GEMM on clusters of two CTAs
+// (tcgen05.mma.cta_group::2, M = 256 real rows per pair), persistent over the
+// tiles of one product or of a batch.  Per accumulator the MMAs run in the
+// order of tc.cu's pair form (the main product x0 y0 into a chunk
+// accumulator, restarted every 16 MMAs and folded into FP32 registers with
+// round-to-nearest adds; the corrections x0y1, x1y0 [, x1y1, x0y2, x2y0] into
+// one accumulator for the whole K range), so both give the same bits.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cstdint>
+#include <cstring>
+#include <mutex>
+
+#include "internal.h"
+#include "pieces.h"
+#include "ptx.h"
+#include "t1m_capi.h"
+#include "tc_common.h"
+
+namespace t1m {
+namespace gb300 {
+namespace {
+
+// ------------------------------------------------------------- split pass ---
+
+struct SplitPair {
+  PieceSplit op[2];
+  int n;
+};
+
+// Pieces of 8 consecutive real k (v, already conjugated) into one 16-byte
+// chunk per piece.  `at`: byte offset of the chunk in piece 0, pieces
+// `stride` bytes apart.
+template <int P>
+__device__ __forceinline__ void put_chunk(uint8_t* out, int64_t at, int64_t stride,
+                                          const float (&v)[8]) {
+  uint32_t w[3][4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) split_bf16<P>(v[2 * j], v[2 * j + 1], w[0][j], w[1][j], w[2][j]);
+#pragma unroll
+  for (int p = 0; p < P; ++p)
+    *reinterpret_cast<uint4*>(out + at + p * stride) = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
+}
+
+// Byte offset of chunk c of real row rr in the piece-0 atom of stage ks.
+template <int P>
+__device__ __forceinline__ int64_t chunk_at(int64_t rg, int64_t ks, int64_t rr, int c) {
+  const int rl = static_cast<int>(rr & 7);
+  return (ks * P * rg + (rr >> 3)) * kPieceAtom + rl * 64 + ((c ^ ((rl >> 1) & 3)) << 4);
+}
+
+// Chunk c of source row r in stage ks from shared memory (`src`: its 4
+// complex or 8 real values, consecutive k).
+template <int P, bool kReal>
+__device__ __forceinline__ void split_row_chunk(const PieceSplit& o, int64_t ks, int64_t r, int c,
+                                                const float* src) {
+  const int64_t stride = o.rg * kPieceAtom;
+  float v[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) v[j] = src[j];
+  if constexpr (kReal) {
+    put_chunk<P>(o.out, chunk_at<P>(o.rg, ks, r, c), stride, v);
+  } else {
+    if (o.conj) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) v[2 * j + 1] = -v[2 * j + 1];
+    }
+    if (!o.expand) {
+      put_chunk<P>(o.out, chunk_at<P>(o.rg, ks, r, c), stride, v);
+    } else {
+      float x[8];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        x[2 * j] = v[2 * j];
+        x[2 * j + 1] = -v[2 * j + 1];
+      }
+      put_chunk<P>(o.out, chunk_at<P>(o.rg, ks, 2 * r, c), stride, x);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        x[2 * j] = v[2 * j + 1];
+        x[2 * j + 1] = v[2 * j];
+      }
+      put_chunk<P>(o.out, chunk_at<P>(o.rg, ks, 2 * r + 1, c), stride, x);
+    }
+  }
+}
+
+constexpr int kSplitRowsPer = 32;                                // source rows per block
+template <bool kReal>
+constexpr int split_k() { return kReal ? 64 : 32; }              // k per block: two stages
+
+// Blocks of 32 rows x two stages: read through shared memory along the
+// source's unit-stride direction, written as whole atoms (a warp writes the
+// four chunks of eight rows).  Bound by HBM; k past K is written as zeros, rows past
+// R are not written.
+template <int P, bool kReal>
+__global__ void __launch_bounds__(256)
+split_pieces(const SplitPair pair, const PieceSplit* dev, int n) {
+  using T = typename std::conditional<kReal, float, float2>::type;
+  constexpr int KB = split_k<kReal>();
+  __shared__ T tile[kSplitRowsPer][KB + 1];
+  __shared__ PieceSplit so;
+  if (dev) {
+    int lo = 0, hi = n - 1;
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (dev[mid].block_begin <= blockIdx.x) lo = mid; else hi = mid - 1;
+    }
+    if (threadIdx.x == 0) so = dev[lo];
+    __syncthreads();
+  }
+  const PieceSplit& o =
+      dev ? so : (pair.n > 1 && blockIdx.x >= pair.op[1].block_begin ? pair.op[1] : pair.op[0]);
+  const int64_t bid = blockIdx.x - o.block_begin;
+  const int64_t kblocks = (o.K + KB - 1) / KB;
+  const int64_t r0 = (bid / kblocks) * kSplitRowsPer, k0 = (bid % kblocks) * KB;
+  const T* __restrict__ src = static_cast<const T*>(o.src);
+  const int t = threadIdx.x;
+  constexpr int kPer = kSplitRowsPer * KB / 256;
+  if (o.mode == kSplitRows) {
+    const int r = t & 31;
+    const bool rin = r0 + r < o.R;
+    const T* __restrict__ row = src + (rin ? offs(o.ro, o.ur, r0 + r) : 0);
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+      const int k = (t >> 5) + 8 * i;
+      T v{};
+      if (rin && k0 + k < o.K) v = row[offs(o.ko, o.uk, k0 + k)];
+      tile[r][k] = v;
+    }
+  } else {
+    const int k = t & (KB - 1);
+    const bool kin = k0 + k < o.K;
+    const T* __restrict__ col = src + (kin ? offs(o.ko, o.uk, k0 + k) : 0);
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+      const int r = t / KB + (256 / KB) * i;
+      T v{};
+      if (kin && r0 + r < o.R) v = col[offs(o.ro, o.ur, r0 + r)];
+      tile[r][k] = v;
+    }
+  }
+  __syncthreads();
+  // 32 rows x 8 chunks: thread t takes chunk t & 3 of row (t >> 2) & 31 in
+  // stage t >> 7 of the block's two.
+  const int c = t & 3, r = (t >> 2) & 31, st = t >> 7;
+  constexpr int kStageE = kReal ? 32 : 16;  // elements per stage
+  const int64_t ks = k0 / kStageE + st;
+  if (r0 + r >= o.R || ks * kStageE >= o.K) return;
+  float v[8];
+  constexpr int kChunkE = kReal ? 8 : 4;
+#pragma unroll
+  for (int j = 0; j < kChunkE; ++j) {
+    const T x = tile[r][st * kStageE + c * kChunkE + j];
+    if constexpr (kReal) {
+      v[j] = x;
+    } else {
+      v[2 * j] = x.x;
+      v[2 * j + 1] = x.y;
+    }
+  }
+  split_row_chunk<P, kReal>(o, ks, r0 + r, c, v);
+}
+
+// kSplitStep: the source is contiguous along k_hi (k = k_lo + step * k_hi).
+// Blocks of 8 rows x one stage of k_lo x 32 k_hi: reads are runs of 32
+// elements, writes whole atoms (one stage of every k_hi).
+template <int P, bool kReal>
+__global__ void __launch_bounds__(256)
+split_pieces_step(const PieceSplit o) {
+  using T = typename std::conditional<kReal, float, float2>::type;
+  constexpr int KL = kReal ? 32 : 16, KH = 32, R = 8;
+  // Rows padded by one element and k_hi planes by one more: neither the
+  // stores along k_hi nor the chunk reads conflict.
+  constexpr int kRow = KL + 1, kPlane = R * kRow + 1;
+  __shared__ T tile[KH * kPlane];
+  const int64_t nhi = o.K / o.step, nlo = o.step / KL;
+  const int64_t hblocks = (nhi + KH - 1) / KH;
+  int64_t b = blockIdx.x;
+  const int64_t h0 = (b % hblocks) * KH;
+  b /= hblocks;
+  const int64_t l0 = (b % nlo) * KL, r0 = (b / nlo) * R;
+  const T* __restrict__ src = static_cast<const T*>(o.src);
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  // Offsets are linear in the mode indices and `step` spans whole modes.
+  const bool hin = h0 + lane < nhi;
+  const int64_t oh = hin ? offs(o.ko, o.uk, o.step * (h0 + lane)) : 0;
+  const bool rin = r0 + warp < o.R;
+  const T* __restrict__ row = src + (rin ? offs(o.ro, o.ur, r0 + warp) : 0) + oh;
+#pragma unroll 8
+  for (int l = 0; l < KL; ++l) {
+    T v{};
+    if (hin && rin) v = row[offs(o.ko, o.uk, l0 + l)];
+    tile[lane * kPlane + warp * kRow + l] = v;
+  }
+  __syncthreads();
+  const int c = lane & 3, r = lane >> 2;
+  if (r0 + r >= o.R) return;
+  constexpr int kChunkE = kReal ? 8 : 4;
+#pragma unroll
+  for (int i = 0; i < KH / 8; ++i) {
+    const int h = warp + 8 * i;
+    if (h0 + h >= nhi) break;
+    const T* s = tile + h * kPlane + r * kRow + c * kChunkE;
+    float v[8];
+#pragma unroll
+    for (int j = 0; j < kChunkE; ++j) {
+      if constexpr (kReal) {
+        v[j] = s[j];
+      } else {
+        v[2 * j] = s[j].x;
+        v[2 * j + 1] = s[j].y;
+      }
+    }
+    split_row_chunk<P, kReal>(o, (l0 + o.step * (h0 + h)) / KL, r0 + r, c, v);
+  }
+}
+
+// ---------------------------------------------------------------- product ---
+
+constexpr int kPcThreads = 640;        // warp 0 MMA, 1 loads, 2 relay, 4-19 epilogue
+constexpr int kPcEpiBase = 128;
+constexpr int kPcEpiWarps = 16;
+constexpr uint32_t kPcTmemCols = 512;
+constexpr int kPcBarriers = 256;
+constexpr int kPcARows = 128;          // real rows of A per CTA
+constexpr int kPcABytes = kPcARows * 64;
+constexpr int kPcFold = 8;             // stages per main chunk: 16 MMAs of K = 16
+
+// kWide: tiles of 160 to 256 columns, one chunk and one correction
+// accumulator of 256 columns; otherwise up to 128 columns and two of each.
+// Ring stages: as many as 227 KB hold.
+template <int P, bool kWide>
+struct PcShape {
+  static constexpr int kMaxN = kWide ? 256 : 128;
+  static constexpr int kBufs = kWide ? 1 : 2;
+  static constexpr int kBBytes = kMaxN / 2 * 64;            // one piece of this CTA's columns
+  static constexpr int kStage = P * (kPcABytes + kBBytes);  // 48 / 36 KB for three pieces
+  static constexpr int kStages = kWide ? (P == 3 ? 4 : 6) : (P == 3 ? 6 : 8);
+  static constexpr int kSmem = 1024 + kStages * kStage + kPcBarriers;
+  static_assert(kSmem <= 227 * 1024, "shared memory budget");
+  static_assert(8 * (2 * kStages + 4 * kBufs + 2) <= kPcBarriers, "barrier area");
+  __device__ static constexpr uint32_t chunk_col(int b) { return 128u * b; }
+  __device__ static constexpr uint32_t corr_col(int b) { return 256u + 128u * b; }
+};
+
+struct PcTile {
+  const PieceProblem* p;
+  int64_t tm, n0, kb, steps;  // steps: K = 16 MMA steps of this tile
+  int64_t split;
+  int tn;
+};
+
+// Tiles of a problem are numbered split-major; within a split, groups of 8
+// pair tiles along M sweep N, so pairs running together share both operands
+// in L2.
+template <bool kReal>
+__device__ __forceinline__ PcTile pc_locate(const PieceProblem* single, const PieceProblem* group,
+                                            int nprob, int64_t t, int& hint) {
+  const PieceProblem* p = single;
+  if (group) {
+    int lo = hint;
+    while (lo + 1 < nprob && group[lo + 1].tile_begin <= t) ++lo;
+    hint = lo;
+    p = group + lo;
+  }
+  // Tile counts of a launch fit 32 bits (launch_piece_products).
+  const int lt = static_cast<int>(t - p->tile_begin);
+  const int tiles_m = p->tiles_m, tiles_n = p->tiles_n;
+  const int per_split = tiles_m * tiles_n;
+  const int split = p->splits > 1 ? lt / per_split : 0, r = lt - split * per_split;
+  constexpr int G = 8;
+  const int grp = r / (G * tiles_n), in = r - grp * (G * tiles_n);
+  const int first_m = grp * G;
+  const int gsize = min(G, tiles_m - first_m);
+  const int col = in / gsize;
+  PcTile x;
+  x.p = p;
+  x.split = split;
+  x.tm = first_m + in - col * gsize;
+  x.tn = p->tile_n;
+  x.n0 = int64_t(col) * x.tn;
+  constexpr int64_t f = kReal ? 1 : 2;
+  const int64_t kb = int64_t(split) * p->g.k_per_split;
+  const int64_t ke = min(p->g.K, kb + p->g.k_per_split);
+  x.kb = f * kb;
+  x.steps = (f * (ke - kb) + 15) / 16;
+  return x;
+}
+
+// C <- alpha * acc (+ beta * C, or + C when accumulating) for the 16 columns
+// [n0, n0 + 16) below N of complex row at Cr: lane pairs hold its real (part
+// 0) and imaginary row.  As store_tile, but old values are read together
+// before any is written, so accumulating products wait once per group
+// instead of once per access.
+__device__ __forceinline__ void pc_store16(const GemmArgs& g, float2* __restrict__ Cr, bool row_ok,
+                                           int64_t n0, int part, const float* acc) {
+  const uint32_t flags = g.flags;
+  const bool accumulate = flags & kFlagAccumulate, read = accumulate || !(flags & kFlagBetaZero);
+  const bool col16 = flags & kFlagCCol16;
+  const float ar = (float)g.alpha[0], ai = (float)g.alpha[1];
+  const float br = (float)g.beta[0], bi = (float)g.beta[1];
+  const int64_t N = g.N;
+  if (n0 >= N) return;  // uniform over the warp
+  float2 v[8];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const float s0 = part ? acc[4 * q] : acc[4 * q + 2];
+    const float s1 = part ? acc[4 * q + 1] : acc[4 * q + 3];
+    const float r0 = __shfl_xor_sync(0xffffffffu, s0, 1);
+    const float r1 = __shfl_xor_sync(0xffffffffu, s1, 1);
+    const float re0 = part ? r0 : acc[4 * q], im0 = part ? acc[4 * q + 2] : r0;
+    const float re1 = part ? r1 : acc[4 * q + 1], im1 = part ? acc[4 * q + 3] : r1;
+    v[2 * q] = make_float2(ar * re0 - ai * im0, ar * im0 + ai * re0);
+    v[2 * q + 1] = make_float2(ar * re1 - ai * im1, ar * im1 + ai * re1);
+  }
+  if (!row_ok) return;
+  auto combine = [&](float2 t, float2 o) {
+    return accumulate ? make_float2(o.x + t.x, o.y + t.y)
+                      : make_float2(t.x + (br * o.x - bi * o.y), t.y + (br * o.y + bi * o.x));
+  };
+  // Value 2 q + e belongs to column n0 + 4 q + 2 part + e.
+  if ((flags & kFlagCPairs) && col16 && n0 + 16 <= N) {
+    float4* p = reinterpret_cast<float4*>(Cr + offs(g.csC, g.uC_n, n0) + 2 * part);
+    if (read) {
+      float4 o[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) o[q] = p[2 * q];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        v[2 * q] = combine(v[2 * q], make_float2(o[q].x, o[q].y));
+        v[2 * q + 1] = combine(v[2 * q + 1], make_float2(o[q].z, o[q].w));
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      p[2 * q] = make_float4(v[2 * q].x, v[2 * q].y, v[2 * q + 1].x, v[2 * q + 1].y);
+  } else {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {  // four values at a time
+      float2* p[4];
+      bool in[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int64_t n = n0 + 8 * h + 4 * (i >> 1) + 2 * part + (i & 1);
+        in[i] = n < N;
+        p[i] = Cr + (in[i] ? offs(g.csC, g.uC_n, n) : 0);
+      }
+      if (read) {
+        float2 o[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) o[i] = in[i] ? *p[i] : make_float2(0.f, 0.f);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[4 * h + i] = combine(v[4 * h + i], o[i]);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (in[i]) *p[i] = v[4 * h + i];
+    }
+  }
+}
+
+// The real form: columns [n0, n0 + 16) of one real row per lane.
+__device__ __forceinline__ void pc_store16_real(const GemmArgs& g, float* __restrict__ Cr,
+                                                int64_t n0, const float* acc) {
+  const uint32_t flags = g.flags;
+  const bool accumulate = flags & kFlagAccumulate, read = accumulate || !(flags & kFlagBetaZero);
+  const float ar = (float)g.alpha[0], br = (float)g.beta[0];
+  const int64_t N = g.N;
+  if (n0 >= N) return;
+  auto combine = [&](float t, float o) { return accumulate ? o + t : t + br * o; };
+  if ((flags & kFlagCPairs) && (flags & kFlagCCol16) && n0 + 16 <= N) {
+    float4* p = reinterpret_cast<float4*>(Cr + offs(g.csC, g.uC_n, n0));
+    float4 o[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) o[q] = read ? p[q] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      float4 t = make_float4(ar * acc[4 * q], ar * acc[4 * q + 1], ar * acc[4 * q + 2],
+                             ar * acc[4 * q + 3]);
+      if (read)
+        t = make_float4(combine(t.x, o[q].x), combine(t.y, o[q].y), combine(t.z, o[q].z),
+                        combine(t.w, o[q].w));
+      p[q] = t;
+    }
+  } else {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {  // eight values at a time
+      float* p[8];
+      bool in[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int64_t n = n0 + 8 * h + i;
+        in[i] = n < N;
+        p[i] = Cr + (in[i] ? offs(g.csC, g.uC_n, n) : 0);
+      }
+      float o[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) o[i] = read && in[i] ? *p[i] : 0.f;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float t = ar * acc[8 * h + i];
+        if (in[i]) *p[i] = read ? combine(t, o[i]) : t;
+      }
+    }
+  }
+}
+
+// Persistent over the launch's tiles, one cluster of two CTAs per pair of
+// SMs.  Warp 0 (even CTA, one lane) issues every MMA; warp 1 (one lane per
+// CTA) loads the CTA's 128 rows of A and half of the tile's columns of B;
+// warp 2 (odd CTA, one lane) relays the arrival of its stage to the MMA
+// thread; warps 4-19 fold chunks and write C (one TMEM lane per thread, the
+// four warpgroups taking the tile's 16-column units in turn).
+//
+// Overlap.  Loads run ahead over tile borders.  With tiles of up to 128
+// columns both chunk and correction accumulators are doubled, so a tile's
+// MMAs start while the previous tile is still being read and written.  Wide
+// tiles fill TMEM with one set: a chunk is folded while the corrections of
+// its last two stages run (their main products are issued first), and the
+// next tile starts as soon as the accumulators are in registers, before C is
+// written.
+//
+// Tile widths from 32 to 256 columns let the tiles of a product fill whole
+// waves of the 76 pairs (piece_tile_n).  Measured at complex64 4096^3,
+// BF16x6: 1.86 ms (one 128-column tile per pair, 64-k stages, MMAs issued
+// from a lane-0 branch) -> 1.52 ms, 361 TFLOP/s of 8MNK.
+template <int P, bool kReal, bool kWide>
+__global__ void __launch_bounds__(kPcThreads, 1)
+tc1m_pieces(const __grid_constant__ PieceProblem single, const PieceProblem* group, int nprob,
+            int64_t total_tiles, int* err_flag) {
+  using Sh = PcShape<P, kWide>;
+  constexpr int S = Sh::kStages, kBufs = Sh::kBufs;
+  constexpr int kUnits = Sh::kMaxN / 16 / (kPcEpiWarps / 4);  // 16-column units per thread
+
+  extern __shared__ __align__(16) uint8_t smem_raw[];
+  const uint32_t base = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
+  uint8_t* const base_ptr = smem_raw + (base - ptx::smem_u32(smem_raw));
+  const uint32_t bars = base + S * Sh::kStage;
+  auto full_bar = [&](int s) { return bars + 8u * s; };
+  auto empty_bar = [&](int s) { return bars + 8u * (S + s); };
+  auto chunk_full = [&](int b) { return bars + 8u * (2 * S + b); };
+  auto chunk_empty = [&](int b) { return bars + 8u * (2 * S + kBufs + b); };
+  auto corr_full = [&](int b) { return bars + 8u * (2 * S + 2 * kBufs + b); };
+  auto corr_empty = [&](int b) { return bars + 8u * (2 * S + 3 * kBufs + b); };
+  const uint32_t end_bar = bars + 8u * (2 * S + 4 * kBufs);
+  const uint32_t tmem_slot = end_bar + 8u;
+  volatile uint32_t* tmem_slot_ptr =
+      reinterpret_cast<volatile uint32_t*>(base_ptr + (tmem_slot - base));
+
+  const int tid = threadIdx.x;
+  // Broadcast from lane 0, so the compiler knows the roles are warp-uniform.
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+  const uint32_t rank = __shfl_sync(0xffffffffu, ptx::cluster_ctarank(), 0);
+  if (warp == 0) {
+    ptx::tmem_alloc2(tmem_slot, kPcTmemCols);
+    ptx::tmem_relinquish2();
+  }
+  if (tid == 32) {
+    // A stage is full on the even CTA once its own copies and, through the
+    // odd CTA's relay, the peer's have landed.
+    for (int s = 0; s < S; ++s) {
+      ptx::mbar_init(full_bar(s), rank == 0 ? 2 : 1);
+      ptx::mbar_init(empty_bar(s), 1);
+    }
+    for (int b = 0; b < kBufs; ++b) {
+      ptx::mbar_init(chunk_full(b), 1);
+      ptx::mbar_init(chunk_empty(b), 2 * kPcEpiWarps);
+      ptx::mbar_init(corr_full(b), 1);
+      ptx::mbar_init(corr_empty(b), 2 * kPcEpiWarps);
+    }
+    ptx::mbar_init(end_bar, 1);
+    ptx::fence_mbar_init();
+  }
+  ptx::tc_fence_before();
+  ptx::cluster_sync();
+  ptx::tc_fence_after();
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot_ptr, 0);
+
+  // Everything above may overlap the end of the split pass; the descriptors,
+  // pieces and C below may have been written by earlier kernels.
+  ptx::grid_dependency_wait();
+  const int64_t first = blockIdx.x >> 1, stride = gridDim.x >> 1;
+  if (warp == 0) {
+    // ---------------------------------------------------------- MMA issue ---
+    // The whole warp runs this loop and one elected lane issues: with
+    // warp-uniform control flow the descriptors stay in uniform registers.
+    // Issued from a lane-0 branch an MMA cost its thread 75 clocks and a stage
+    // 850 more, whatever the tile width (128-column tiles ran at half the
+    // tensor rate).
+    if (rank == 0) {
+      const uint64_t desc0 = ptx::smem_desc_sw64(base);
+      const bool issue = ptx::elect_one();
+      int slot = 0, tile_cnt = 0, chunk = 0, hint = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      int x_tn = 0, x_steps = 0, x_swap = 0;
+      auto look = [&](int64_t t) {
+        const PcTile x = pc_locate<kReal>(&single, group, nprob, t, hint);
+        x_tn = __shfl_sync(0xffffffffu, x.tn, 0);
+        x_steps = __shfl_sync(0xffffffffu, static_cast<int>(x.steps), 0);
+        x_swap = __shfl_sync(0xffffffffu, x.p->swapped, 0);
+      };
+      // Products of one ring slot.  Piece p, K = 16 step kk: A at +p x 8 KB,
+      // B after the A pieces, +32 bytes per step inside the 64-byte rows.
+      auto mains = [&](int st, int nkk, uint32_t d, uint32_t idesc, bool first_of_chunk) {
+        const uint64_t ds = desc0 + static_cast<uint32_t>((st * Sh::kStage) >> 4);
+        if (issue) {
+#pragma unroll
+          for (int kk = 0; kk < 2; ++kk)
+            if (kk < nkk)
+              ptx::mma_f16_ss2(d, ds + ((32 * kk) >> 4), ds + ((P * kPcABytes + 32 * kk) >> 4),
+                               idesc, (first_of_chunk && kk == 0) ? 0u : 1u);
+        }
+      };
+      auto corrections = [&](int st, int nkk, uint32_t d, uint32_t idesc, bool first_of_tile,
+                             bool swapped) {
+        const uint64_t ds = desc0 + static_cast<uint32_t>((st * Sh::kStage) >> 4);
+        // Product of pieces px of the x operand and py of y: x is A, or B
+        // where the operands are exchanged.
+        auto mma = [&](int px, int py, int kk, uint32_t acc) {
+          const int pa = swapped ? py : px, pb = swapped ? px : py;
+          ptx::mma_f16_ss2(d, ds + ((pa * kPcABytes + 32 * kk) >> 4),
+                           ds + ((P * kPcABytes + pb * Sh::kBBytes + 32 * kk) >> 4), idesc, acc);
+        };
+        if (issue) {
+#pragma unroll
+          for (int kk = 0; kk < 2; ++kk) {
+            if (kk < nkk) {
+              mma(0, 1, kk, (first_of_tile && kk == 0) ? 0u : 1u);
+              mma(1, 0, kk, 1u);
+              if (P == 3) {
+                mma(1, 1, kk, 1u);
+                mma(0, 2, kk, 1u);
+                mma(2, 0, kk, 1u);
+              }
+            }
+          }
+          ptx::mma_commit2(empty_bar(st));
+        }
+      };
+      if (first < total_tiles) look(first);
+      for (int64_t t = first; t < total_tiles && ok; t += stride) {
+        const int steps = x_steps;
+        const bool swapped = x_swap != 0;
+        const uint32_t idesc = ptx::idesc_f32acc(1u /*BF16*/, 256u, static_cast<uint32_t>(x_tn));
+        const int ns = (steps + 1) / 2;
+        const int cb = tile_cnt % kBufs;
+        const uint32_t d_corr = tmem + Sh::corr_col(cb);
+        uint32_t d_main = 0;
+        int buf = 0;
+        for (int s = 0; s < ns;) {
+          if (s % kPcFold == 0) {
+            buf = chunk % kBufs;
+            d_main = tmem + Sh::chunk_col(buf);
+            if (chunk >= kBufs &&
+                !ptx::mbar_wait(chunk_empty(buf), static_cast<uint32_t>((chunk / kBufs - 1) & 1))) {
+              record_error(err_flag, kErrChunkWait);
+              ok = false;
+              break;
+            }
+          }
+          // The last two stages of a chunk issue their main products
+          // together, so its fold overlaps two stages of corrections.
+          const bool two = s % kPcFold == kPcFold - 2 && s + 1 < ns;
+          const int slot2 = slot + 1 == S ? 0 : slot + 1;
+          const uint32_t phase2 = slot + 1 == S ? phase ^ 1u : phase;
+          if (!ptx::mbar_wait(full_bar(slot), phase) ||
+              (two && !ptx::mbar_wait(full_bar(slot2), phase2))) {
+            record_error(err_flag, kErrFullWait);
+            ok = false;
+            break;
+          }
+          ptx::tc_fence_after();
+          const int nkk = steps - 2 * s >= 2 ? 2 : 1, nkk2 = steps - 2 * s >= 4 ? 2 : 1;
+          mains(slot, nkk, d_main, idesc, s % kPcFold == 0);
+          if (two) mains(slot2, nkk2, d_main, idesc, false);
+          const int last = s + (two ? 1 : 0);
+          if (last % kPcFold == kPcFold - 1 || last == ns - 1) {
+            if (issue) ptx::mma_commit2(chunk_full(buf));
+            ++chunk;
+          }
+          if (s == 0 && tile_cnt >= kBufs) {
+            if (!ptx::mbar_wait(corr_empty(cb), static_cast<uint32_t>((tile_cnt / kBufs - 1) & 1))) {
+              record_error(err_flag, kErrAccEmptyWait);
+              ok = false;
+              break;
+            }
+            ptx::tc_fence_after();
+          }
+          corrections(slot, nkk, d_corr, idesc, s == 0, swapped);
+          if (two) corrections(slot2, nkk2, d_corr, idesc, false, swapped);
+          // The next tile is looked up while this tile's MMAs run.
+          if (s == 0 && t + stride < total_tiles) look(t + stride);
+          slot = two ? slot2 : slot;
+          phase = two ? phase2 : phase;
+          s += two ? 2 : 1;
+          if (++slot == S) {
+            slot = 0;
+            phase ^= 1u;
+          }
+        }
+        if (!ok) break;
+        if (issue) ptx::mma_commit2(corr_full(cb));
+        ++tile_cnt;
+      }
+      // No MMA may still write TMEM (or read shared memory) when the CTAs leave.
+      if (issue) ptx::mma_commit2(end_bar);
+      if (!ptx::mbar_wait(end_bar, 0)) record_error(err_flag, kErrAccWait);
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    // -------------------------------------------------------------- loads ---
+    if (lane == 0) {
+      int64_t it = 0;
+      int hint = 0;
+      bool ok = true;
+      for (int64_t t = first; t < total_tiles && ok; t += stride) {
+        const PcTile x = pc_locate<kReal>(&single, group, nprob, t, hint);
+        const PieceProblem* p = x.p;
+        // Row groups of this CTA's rows and columns that exist (the rest of
+        // the stage keeps old bytes: rows and columns nobody writes to C).
+        const int64_t ga = (2 * x.tm + rank) * (kPcARows / 8);
+        const int64_t gb = (x.n0 + rank * (x.tn / 2)) / 8;
+        const int64_t na = min(int64_t(kPcARows / 8), p->rg_a - ga);
+        const int64_t nb = min(int64_t(x.tn / 16), p->rg_b - gb);
+        const uint32_t abytes = na > 0 ? static_cast<uint32_t>(na) * kPieceAtom : 0u;
+        const uint32_t bbytes = nb > 0 ? static_cast<uint32_t>(nb) * kPieceAtom : 0u;
+        const int64_t ks0 = x.kb / kPieceStageK, ns = (x.steps + 1) / 2;
+        const uint8_t* a = p->a + (ks0 * P * p->rg_a + ga) * kPieceAtom;
+        const uint8_t* b = p->b + (ks0 * P * p->rg_b + gb) * kPieceAtom;
+        const int64_t pa = p->rg_a * kPieceAtom, pb = p->rg_b * kPieceAtom;
+        for (int64_t s = 0; s < ns; ++s, ++it) {
+          const int st = static_cast<int>(it % S);
+          if (!ptx::mbar_wait(empty_bar(st), static_cast<uint32_t>((it / S) & 1) ^ 1u)) {
+            record_error(err_flag, kErrRawWait);
+            ok = false;
+            break;
+          }
+          const uint32_t dst = base + st * Sh::kStage;
+          ptx::mbar_arrive_expect_tx(full_bar(st), P * (abytes + bbytes));
+#pragma unroll
+          for (int q = 0; q < P; ++q) {
+            if (abytes) ptx::bulk_load(dst + q * kPcABytes, a, abytes, full_bar(st));
+            if (bbytes)
+              ptx::bulk_load(dst + P * kPcABytes + q * Sh::kBBytes, b, bbytes, full_bar(st));
+            a += pa;
+            b += pb;
+          }
+        }
+      }
+    }
+    __syncwarp();
+  } else if (warp == 2) {
+    // -------------------------------------------------------------- relay ---
+    if (lane == 0 && rank == 1) {
+      int64_t it = 0;
+      int hint = 0;
+      bool ok = true;
+      for (int64_t t = first; t < total_tiles && ok; t += stride) {
+        const PcTile x = pc_locate<kReal>(&single, group, nprob, t, hint);
+        const int64_t ns = (x.steps + 1) / 2;
+        for (int64_t s = 0; s < ns; ++s, ++it) {
+          const int st = static_cast<int>(it % S);
+          if (!ptx::mbar_wait(full_bar(st), static_cast<uint32_t>((it / S) & 1))) {
+            record_error(err_flag, kErrFullWait);
+            ok = false;
+            break;
+          }
+          ptx::mbar_arrive_cluster(ptx::mapa(full_bar(st), 0));
+        }
+      }
+    }
+    __syncwarp();
+  } else if (tid >= kPcEpiBase) {
+    // ------------------------------------------------- fold and epilogue ---
+    const int pt = tid - kPcEpiBase;
+    const int wg = pt >> 7;
+    const int q = (pt >> 5) & 3;
+    const int rho = 32 * q + lane;  // real row of this CTA's 128 = TMEM lane
+    const uint32_t lane_base = static_cast<uint32_t>(32 * q) << 16;
+    int64_t chunk = 0, tile_cnt = 0;
+    int hint = 0;
+    for (int64_t t = first; t < total_tiles; t += stride, ++tile_cnt) {
+      const PcTile x = pc_locate<kReal>(&single, group, nprob, t, hint);
+      float master[kUnits][16];
+#pragma unroll
+      for (int u = 0; u < kUnits; ++u)
+#pragma unroll
+        for (int j = 0; j < 16; ++j) master[u][j] = 0.f;
+      auto unit_col = [&](int u) { return 16 * (wg + 4 * u); };
+      auto fold = [&](uint32_t col) {
+#pragma unroll
+        for (int u = 0; u < kUnits; ++u) {
+          if (unit_col(u) < x.tn) {
+            uint32_t r[16];
+            ptx::tmem_ld16_sync(tmem + lane_base + col + unit_col(u), r);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) master[u][j] += __uint_as_float(r[j]);
+          }
+        }
+      };
+      auto release = [&](uint32_t bar) {
+        ptx::tc_fence_before();
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive_cluster(ptx::mapa(bar, 0));
+      };
+      const int64_t nchunks = (x.steps + 2 * kPcFold - 1) / (2 * kPcFold);
+      bool ok = true;
+      for (int64_t c = 0; c < nchunks; ++c, ++chunk) {
+        const int buf = static_cast<int>(chunk % kBufs);
+        if (!ptx::mbar_wait(chunk_full(buf), static_cast<uint32_t>((chunk / kBufs) & 1))) {
+          record_error(err_flag, kErrChunkWait);
+          ok = false;
+          break;
+        }
+        ptx::tc_fence_after();
+        fold(Sh::chunk_col(buf));
+        release(chunk_empty(buf));
+      }
+      if (!ok) break;
+      const int cb = static_cast<int>(tile_cnt % kBufs);
+      if (!ptx::mbar_wait(corr_full(cb), static_cast<uint32_t>((tile_cnt / kBufs) & 1))) {
+        record_error(err_flag, kErrAccWait);
+        break;
+      }
+      ptx::tc_fence_after();
+      fold(Sh::corr_col(cb));
+      release(corr_empty(cb));
+      const GemmArgs& g = x.p->g;
+      if constexpr (kReal) {
+        const int64_t row = (2 * x.tm + rank) * kPcARows + rho;
+        if (row < g.M) {
+          float* Cr = static_cast<float*>(g.C) + x.split * g.c_split_stride +
+                      offs(g.rsC, g.uC_m, row);
+#pragma unroll
+          for (int u = 0; u < kUnits; ++u)
+            if (unit_col(u) < x.tn) pc_store16_real(g, Cr, x.n0 + unit_col(u), master[u]);
+        }
+      } else {
+        const int64_t row = (2 * x.tm + rank) * (kPcARows / 2) + (rho >> 1);
+        const bool row_ok = row < g.M;
+        float2* Cr = static_cast<float2*>(g.C) + x.split * g.c_split_stride +
+                     (row_ok ? offs(g.rsC, g.uC_m, row) : 0);
+#pragma unroll
+        for (int u = 0; u < kUnits; ++u)
+          if (unit_col(u) < x.tn) pc_store16(g, Cr, row_ok, x.n0 + unit_col(u), rho & 1, master[u]);
+      }
+    }
+  }
+
+  ptx::tc_fence_before();
+  __syncwarp();
+  ptx::cluster_sync();
+  if (warp == 0) {
+    ptx::tc_fence_after();
+    ptx::tmem_dealloc2(tmem, kPcTmemCols);
+  }
+}
+
+template <int P, bool kReal, bool kWide>
+cudaError_t launch_products(const PieceProblem* single, const PieceProblem* dev, int nprob,
+                            int64_t total_tiles, cudaStream_t stream, int* err_flag) {
+  constexpr int kSmem = PcShape<P, kWide>::kSmem;
+  static std::once_flag once;
+  static cudaError_t attr = cudaSuccess;
+  std::call_once(once, [] {
+    attr = cudaFuncSetAttribute(tc1m_pieces<P, kReal, kWide>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+  });
+  if (attr != cudaSuccess) return attr;
+  PieceProblem none;
+  if (!single) {
+    std::memset(static_cast<void*>(&none), 0, sizeof(none));
+    single = &none;
+  }
+  constexpr int64_t kPairs = 76;  // pairs of SMs
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(2 * std::min<int64_t>(total_tiles, kPairs)));
+  cfg.blockDim = dim3(kPcThreads);
+  cfg.dynamicSmemBytes = kSmem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attrs[2];
+  attrs[0].id = cudaLaunchAttributeClusterDimension;
+  attrs[0].val.clusterDim.x = 2;
+  attrs[0].val.clusterDim.y = 1;
+  attrs[0].val.clusterDim.z = 1;
+  attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attrs[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attrs;
+  cfg.numAttrs = 2;
+  return cudaLaunchKernelEx(&cfg, tc1m_pieces<P, kReal, kWide>, *single, dev, nprob, total_tiles,
+                            err_flag);
+}
+
+template <int P, bool kReal>
+cudaError_t launch_products_w(bool wide, const PieceProblem* single, const PieceProblem* dev,
+                              int nprob, int64_t tiles, cudaStream_t stream, int* err_flag) {
+  return wide ? launch_products<P, kReal, true>(single, dev, nprob, tiles, stream, err_flag)
+              : launch_products<P, kReal, false>(single, dev, nprob, tiles, stream, err_flag);
+}
+
+template <int P, bool kReal>
+cudaError_t launch_split_t(const PieceSplit* ops, int n, const PieceSplit* dev, int64_t blocks,
+                           cudaStream_t stream) {
+  if (!dev && n == 1 && ops[0].mode == kSplitStep) {
+    split_pieces_step<P, kReal><<<static_cast<unsigned>(blocks), 256, 0, stream>>>(ops[0]);
+    return cudaGetLastError();
+  }
+  SplitPair pair;
+  std::memset(static_cast<void*>(&pair), 0, sizeof(pair));
+  if (!dev) {
+    if (n > 2) return cudaErrorInvalidValue;
+    for (int i = 0; i < n; ++i) pair.op[i] = ops[i];
+    pair.n = n;
+  }
+  split_pieces<P, kReal><<<static_cast<unsigned>(blocks), 256, 0, stream>>>(pair, dev, n);
+  return cudaGetLastError();
+}
+
+}  // namespace
+
+int64_t piece_split_blocks(bool real, const PieceSplit& s) {
+  if (s.mode == kSplitStep) {
+    const int64_t nhi = s.K / s.step, nlo = s.step / (real ? 32 : 16);
+    return (s.R + 7) / 8 * nlo * ((nhi + 31) / 32);
+  }
+  const int64_t kb = real ? split_k<true>() : split_k<false>();
+  return (s.R + kSplitRowsPer - 1) / kSplitRowsPer * ((s.K + kb - 1) / kb);
+}
+
+cudaError_t launch_piece_split(int pieces, bool real, const PieceSplit* ops, int n,
+                               const PieceSplit* dev, int64_t blocks, cudaStream_t stream) {
+  if (blocks <= 0) return cudaSuccess;
+  if (blocks >= (int64_t(1) << 31)) return cudaErrorInvalidConfiguration;
+  if (pieces == 2)
+    return real ? launch_split_t<2, true>(ops, n, dev, blocks, stream)
+                : launch_split_t<2, false>(ops, n, dev, blocks, stream);
+  return real ? launch_split_t<3, true>(ops, n, dev, blocks, stream)
+              : launch_split_t<3, false>(ops, n, dev, blocks, stream);
+}
+
+int piece_tile_n(bool real, int64_t M, int64_t N, int64_t K, int splits) {
+  // Clocks of the busiest pair: its tiles times a tile's MMAs, plus a per-tile
+  // cost that wide tiles do not hide (reading the accumulators) and one
+  // epilogue.  An MMA of K = 16 measured 138, 105, 72 and 61 clocks at 256,
+  // 192, 128 and 64 columns (complex64 4096^3; below 110 columns the reads of
+  // A bound it), so widths differ mostly in how evenly their tiles fill the
+  // 76 pairs: complex64 2304^3 takes 290 us at 192 columns (216 tiles), 322
+  // at 128 (324) and 372 at 256 (162); 1024^3 38 us at 128, 66 at 256.
+  const int64_t rows = real ? 256 : 128;
+  const int64_t tm = (M + rows - 1) / rows;
+  const double steps = double((real ? 1 : 2) * K) / 16 / std::max(1, splits);
+  int best = 128;
+  double best_cost = 1e300;
+  for (int w = 256; w >= 32; w -= 32) {
+    const int64_t tiles = tm * ((N + w - 1) / w) * splits;
+    const int64_t waves = (tiles + 75) / 76;
+    const double mma = steps * 6 * std::max(60.0, 0.55 * w);
+    const double cost = double(waves) * (mma + (w > 128 ? 1500 : 300)) + 30.0 * w;
+    if (cost < best_cost) {
+      best_cost = cost;
+      best = w;
+    }
+  }
+  return best;
+}
+
+void piece_set_tiles(bool real, PieceProblem* p, int tile_n, int splits) {
+  const int64_t rows = real ? 256 : 128;
+  p->tile_n = tile_n;
+  p->tiles_m = static_cast<int32_t>((p->g.M + rows - 1) / rows);
+  p->tiles_n = static_cast<int32_t>((p->g.N + tile_n - 1) / tile_n);
+  p->splits = splits;
+}
+
+cudaError_t launch_piece_products(int pieces, bool real, bool wide, const PieceProblem* single,
+                                  const PieceProblem* dev, int nprob, int64_t total_tiles,
+                                  cudaStream_t stream, int* err_flag) {
+  if (total_tiles <= 0) return cudaSuccess;
+  if (total_tiles >= (int64_t(1) << 31)) return cudaErrorInvalidConfiguration;
+  if (pieces == 2)
+    return real ? launch_products_w<2, true>(wide, single, dev, nprob, total_tiles, stream, err_flag)
+                : launch_products_w<2, false>(wide, single, dev, nprob, total_tiles, stream, err_flag);
+  return real ? launch_products_w<3, true>(wide, single, dev, nprob, total_tiles, stream, err_flag)
+              : launch_products_w<3, false>(wide, single, dev, nprob, total_tiles, stream, err_flag);
+}
+
+}  // namespace gb300
+}  // namespace t1m

@@ -1,0 +1,88 @@
+// Operand pieces (pieces.cu): descriptors of the split pass and of the
+// CTA-pair product, shared with the dispatch (tc.cu) and the grouped launches.
+#pragma once
+
+#include <cstdint>
+
+#include "internal.h"
+
+namespace t1m {
+namespace gb300 {
+
+// Layout of an operand's pieces.  An operand of R real rows (A: the two 1M
+// rows of every complex row, or the rows of a real A; B: its columns) and Kr
+// real k (2 K complex, K real) is stored as atoms of 8 rows x 32 k bf16 (512
+// bytes): piece p of stage ks (k in [32 ks, 32 ks + 32)) and row group rg is
+// atom (ks * P + p) * rg_count + rg.  Inside an atom, row r holds 64 bytes;
+// its 16-byte chunk c lies at chunk c ^ ((r >> 1) & 3).  That is the MMA's
+// 64-byte-swizzled K-major shared-memory layout, so a tile's rows of one
+// stage and piece are ONE contiguous copy of 512 bytes per row group: no
+// tensor maps (a grouped launch needs one descriptor per product, not three)
+// and every access is whole lines.
+constexpr int kPieceStageK = 32;   // real k per stage
+constexpr int kPieceAtom = 512;    // bytes
+inline int64_t piece_groups(int64_t rows) { return (rows + 7) / 8; }
+inline int64_t piece_stages(int64_t kreal) { return (kreal + kPieceStageK - 1) / kPieceStageK; }
+inline size_t piece_bytes(int pieces, int64_t rows, int64_t kreal) {
+  return size_t(pieces) * size_t(piece_groups(rows)) * size_t(piece_stages(kreal)) * kPieceAtom;
+}
+
+// Split pass of one operand: element (r, k) at src + ro(r) + ko(k).
+enum : int32_t {
+  kSplitRows = 0,  // consecutive threads along the rows (unit-stride runs of rows)
+  kSplitK = 1,     // along k
+  kSplitStep = 2   // along k_hi, where k = k_lo + step * k_hi and the source is
+                   // contiguous in k_hi (step a multiple of a stage)
+};
+struct PieceSplit {
+  const void* src;
+  const int64_t *ro, *ko;  // offsets, or uniform strides ur / uk where >= 0
+  int64_t ur, uk;
+  int64_t R, K;            // source rows, elements of K
+  int64_t step;
+  uint8_t* out;
+  int64_t rg;              // row groups of `out` (may exceed this operand's own)
+  int64_t block_begin;     // first block of this operand in the launch
+  int32_t expand;          // complex A: the two 1M rows of every row
+  int32_t conj;
+  int32_t mode;
+  int32_t pad;
+};
+
+// One product over pieces.  g: C, its offsets and epilogue, M, N, K,
+// k_per_split and c_split_stride in elements.
+struct PieceProblem {
+  GemmArgs g;
+  const uint8_t* a;
+  const uint8_t* b;
+  int64_t rg_a, rg_b;
+  int64_t tile_begin;      // first tile of this problem in the launch
+  int32_t tiles_m, tiles_n, splits;
+  int32_t tile_n;          // output columns of a tile, a multiple of 32 up to 256
+  // The operands (and M and N, C's offsets) are exchanged: the product
+  // pairs run in the order of the unexchanged form, x0y1 before x1y0 of its x
+  // and y, so every output sums the same values in the same order.
+  int32_t swapped;
+  int32_t pad;
+};
+
+// Blocks of the split pass of one operand.
+int64_t piece_split_blocks(bool real, const PieceSplit& s);
+// Split `n` operands in one launch (none of them kSplitStep when n > 1 or
+// dev is given): `ops` by value (n <= 2) or the device array `dev`.
+cudaError_t launch_piece_split(int pieces, bool real, const PieceSplit* ops, int n,
+                               const PieceSplit* dev, int64_t blocks, cudaStream_t stream);
+// Tile width of a product and its tile counts (from g and splits).
+int piece_tile_n(bool real, int64_t M, int64_t N, int64_t K, int splits);
+void piece_set_tiles(bool real, PieceProblem* p, int tile_n, int splits);
+inline int64_t piece_tiles(const PieceProblem& p) {
+  return int64_t(p.tiles_m) * p.tiles_n * p.splits;
+}
+// One launch over `total_tiles` tiles of `single`, or of the device array
+// dev[0..nprob) (sorted by tile_begin); wide: every tile_n above 128 columns.
+cudaError_t launch_piece_products(int pieces, bool real, bool wide, const PieceProblem* single,
+                                  const PieceProblem* dev, int nprob, int64_t total_tiles,
+                                  cudaStream_t stream, int* err_flag);
+
+}  // namespace gb300
+}  // namespace t1m

@@ -67,6 +67,12 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
   return true;
 }
 
+// Programmatic dependent launch: wait until the kernels this one depends on
+// have finished and their writes are visible (returns at once otherwise).
+__device__ __forceinline__ void grid_dependency_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // Per-warpgroup register budget (every warp of the warpgroup executes it).
 template <uint32_t kRegs>
 __device__ __forceinline__ void regs_dec() {
@@ -196,6 +202,13 @@ __device__ __forceinline__ void mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uin
       : "memory");
 }
 
+// One lane of a converged warp (true in that lane).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n .reg .pred q;\n elect.sync _|q, 0xffffffff;\n selp.b32 %0, 1, 0, q;\n}" : "=r"(p));
+  return p != 0;
+}
+
 // Arrive on an mbarrier when all previously issued MMAs of this thread finish.
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
   asm volatile(
@@ -213,6 +226,19 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t saddr) {
   d |= static_cast<uint64_t>(1024u >> 4) << 32;               // stride byte offset
   d |= static_cast<uint64_t>(1u) << 46;                        // descriptor version
   d |= static_cast<uint64_t>(2u) << 61;                        // SWIZZLE_128B
+  return d;
+}
+
+// The same for the 64-byte swizzle: 8-row atoms of 512 bytes, rows of 64
+// bytes whose four 16-byte chunks are XOR-permuted by bits 1-2 of the row
+// index within the atom.
+__device__ __forceinline__ uint64_t smem_desc_sw64(uint32_t saddr) {
+  uint64_t d = 0;
+  d |= static_cast<uint64_t>((saddr >> 4) & 0x3FFFu);
+  d |= static_cast<uint64_t>(1u) << 16;
+  d |= static_cast<uint64_t>(512u >> 4) << 32;
+  d |= static_cast<uint64_t>(1u) << 46;
+  d |= static_cast<uint64_t>(4u) << 61;  // SWIZZLE_64B
   return d;
 }
 
@@ -344,6 +370,17 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const void* tmap, int 
       "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes"
       " [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
       "l"(reinterpret_cast<uint64_t>(tmap)), "r"(c0), "r"(c1), "r"(c2), "r"(bar)
+      : "memory");
+}
+
+// Contiguous bulk copy into this CTA's shared memory (both addresses and the
+// size multiples of 16 bytes); completion as transaction bytes on `bar`.
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes,
+                                          uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::
+          "r"(dst),
+      "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes), "r"(bar)
       : "memory");
 }
 

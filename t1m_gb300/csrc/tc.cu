@@ -65,9 +65,11 @@
 #include <vector>
 
 #include "internal.h"
+#include "pieces.h"
 #include "ptx.h"
 #include "t1m_capi.h"
 #include "tc.h"
+#include "tc_common.h"
 
 namespace t1m {
 namespace gb300 {
@@ -111,20 +113,6 @@ static_assert(kAStageCol + 64 * kStages <= kTmemCols, "TMEM budget");
 static_assert(kSmemBytes <= 227 * 1024, "shared memory budget");
 static_assert(kRawABytes % 1024 == 0 && kRawBBytes % 1024 == 0, "TMA swizzle alignment");
 
-enum : int {
-  kErrFullWait = 1,
-  kErrEmptyWait = 2,
-  kErrAccWait = 3,
-  kErrChunkWait = 4,
-  kErrRawWait = 5,
-  kErrAccEmptyWait = 6,
-  kErrDepWait = 7
-};
-
-__device__ __forceinline__ int64_t offs(const int64_t* v, int64_t u, int64_t i) {
-  return u >= 0 ? i * u : __ldg(v + i);
-}
-
 // Byte offset of complex element (row r, complex k) in a 128 B-swizzled tile
 // of 128-byte rows: 16-byte chunk (k/2) of row r lands at chunk (k/2)^(r%8);
 // rows are grouped in 1024-byte atoms.  This is both the TMA SWIZZLE_128B
@@ -132,10 +120,6 @@ __device__ __forceinline__ int64_t offs(const int64_t* v, int64_t u, int64_t i) 
 __device__ __forceinline__ uint32_t swz128(int r, int k) {
   return static_cast<uint32_t>((r >> 3) * 1024 + (r & 7) * 128 +
                                ((((k >> 1) ^ (r & 7)) & 7) << 4) + (k & 1) * 8);
-}
-
-__device__ __forceinline__ void record_error(int* flag, int code) {
-  if (flag) atomicCAS(flag, 0, code);
 }
 
 struct Split {
@@ -153,34 +137,6 @@ __device__ __forceinline__ Split split_tf32(float x) {
   const float h = __fsub_rn(c, __fsub_rn(c, x));
   const float l = __fsub_rn(x, h);
   return {__float_as_uint(h), __float_as_uint(l)};
-}
-
-// Split-product precision of the one-tile-per-CTA kernel.
-//   TF32x3: x = hi + lo (TF32), products hi*hi + hi*lo + lo*hi (kind::tf32).
-//   BF16x3: x = x0 + x1 (bf16, 8 significant bits each), products
-//           x0*y0 + x0*y1 + x1*y0 (kind::f16): about 16 correct bits.
-//   BF16x6: x = x0 + x1 + x2, products x0*y0 + x0*y1 + x1*y0 + x1*y1 +
-//           x0*y2 + x2*y0: about 24 correct bits (FP32-class).
-// The bf16 forms are the split-and-sum scheme of Henry, Tang and Heinecke,
-// "Leveraging the bfloat16 artificial intelligence datatype for
-// higher-precision computations" (ARITH 2019).
-enum : int { kPrecTF32x3 = 0, kPrecBF16x3 = 1, kPrecBF16x6 = 2 };
-
-// Split a pair of floats (consecutive K) into P packed bf16x2 words: piece 0
-// is the round-to-nearest bf16 of the value, each further piece the bf16 of
-// the remainder (x - x0 is exact in FP32).  Low half = x, high half = y.
-template <int P>
-__device__ __forceinline__ void split_bf16(float x, float y, uint32_t& w0, uint32_t& w1,
-                                           uint32_t& w2) {
-  w0 = ptx::cvt_bf16x2(x, y);
-  const float rx = __fsub_rn(x, __uint_as_float(w0 << 16));
-  const float ry = __fsub_rn(y, __uint_as_float(w0 & 0xFFFF0000u));
-  w1 = ptx::cvt_bf16x2(rx, ry);
-  if (P == 3) {
-    const float sx = __fsub_rn(rx, __uint_as_float(w1 << 16));
-    const float sy = __fsub_rn(ry, __uint_as_float(w1 & 0xFFFF0000u));
-    w2 = ptx::cvt_bf16x2(sx, sy);
-  }
 }
 
 __device__ __forceinline__ float lds32(uint32_t addr) {
@@ -354,146 +310,6 @@ __device__ __forceinline__ void gather_b_stage_real(const GemmArgs& g, uint32_t 
       if (i0 + j < kPer && n < kTileN)
         ptx::cp_async_4(dst + swz128(n, k >> 1) + 4u * (k & 1), src[j],
                         ((okm >> j) & 1u) ? 4u : 0u);
-    }
-  }
-}
-
-// Epilogue of one converter thread: accumulator columns [col0, col0 + kCols)
-// of real row 2 ci + part (part 0 holds the real parts of complex row ci,
-// part 1 the imaginary parts).  Lane pairs swap halves with two shuffles per
-// four columns so that each thread holds complete complex values: part 0
-// writes columns 4q, 4q + 1 and part 1 columns 4q + 2, 4q + 3 of every group
-// of four.  With kFlagCPairs the two values go out as one 16-byte access (a
-// lane pair fills a 32-byte sector); with kFlagCCol16 one column offset is
-// looked up per 16 columns.  C <- alpha*acc (+ beta*C, or + C when
-// accumulating).
-template <int kCols>
-__device__ __forceinline__ void store_tile(const GemmArgs& g, float2* __restrict__ Cp,
-                                           int64_t row, bool row_ok, int64_t n0, int col0,
-                                           int part, const float (&master)[kCols],
-                                           int64_t n_end = INT64_MAX) {
-  const uint32_t flags = g.flags;
-  const bool accumulate = flags & kFlagAccumulate;
-  const bool beta_zero = flags & kFlagBetaZero;
-  const bool pairs = flags & kFlagCPairs;
-  const bool col16 = flags & kFlagCCol16;
-  const float ar = (float)g.alpha[0], ai = (float)g.alpha[1];
-  const float br = (float)g.beta[0], bi = (float)g.beta[1];
-  const int64_t N = min(g.N, n_end);  // columns of this tile: [n0, N)
-  const int64_t* __restrict__ csC = g.csC;
-  const int64_t uC_n = g.uC_n;
-  const int64_t rowC = row_ok ? offs(g.rsC, g.uC_m, row) : 0;
-  float2* __restrict__ Cr = Cp + rowC;
-  int64_t blk = 0;  // offset of the current 16-column block (kFlagCCol16)
-#pragma unroll
-  for (int q = 0; q < kCols / 4; ++q) {
-    const float s0 = part ? master[4 * q] : master[4 * q + 2];
-    const float s1 = part ? master[4 * q + 1] : master[4 * q + 3];
-    const float r0 = __shfl_xor_sync(0xffffffffu, s0, 1);
-    const float r1 = __shfl_xor_sync(0xffffffffu, s1, 1);
-    const float re0 = part ? r0 : master[4 * q], im0 = part ? master[4 * q + 2] : r0;
-    const float re1 = part ? r1 : master[4 * q + 1], im1 = part ? master[4 * q + 3] : r1;
-    const int c = col0 + 4 * q + 2 * part;
-    const int64_t n = n0 + c;
-    if (col16 && (q & 3) == 0) {
-      const int64_t nb = n0 + col0 + 16 * (q >> 2);
-      blk = (row_ok && nb < N) ? offs(csC, uC_n, nb) : 0;
-    }
-    if (!row_ok || n >= N) continue;
-    const int64_t on = col16 ? blk + (c - col0 - 16 * (q >> 2)) : offs(csC, uC_n, n);
-    const bool second = n + 1 < N;
-    const float t0r = ar * re0 - ai * im0, t0i = ar * im0 + ai * re0;
-    const float t1r = ar * re1 - ai * im1, t1i = ar * im1 + ai * re1;
-    if (pairs && second) {
-      float4* p4 = reinterpret_cast<float4*>(Cr + on);
-      if (accumulate) {
-        const float4 o = *p4;
-        *p4 = make_float4(o.x + t0r, o.y + t0i, o.z + t1r, o.w + t1i);
-      } else if (beta_zero) {
-        *p4 = make_float4(t0r, t0i, t1r, t1i);
-      } else {
-        const float4 o = *p4;
-        *p4 = make_float4(t0r + (br * o.x - bi * o.y), t0i + (br * o.y + bi * o.x),
-                          t1r + (br * o.z - bi * o.w), t1i + (br * o.w + bi * o.z));
-      }
-    } else {
-      float2* p0 = Cr + on;
-      float2* p1 = second ? Cr + (col16 ? on + 1 : offs(csC, uC_n, n + 1)) : p0;
-      if (accumulate) {
-        const float2 o = *p0;
-        *p0 = make_float2(o.x + t0r, o.y + t0i);
-        if (second) {
-          const float2 o1 = *p1;
-          *p1 = make_float2(o1.x + t1r, o1.y + t1i);
-        }
-      } else if (beta_zero) {
-        *p0 = make_float2(t0r, t0i);
-        if (second) *p1 = make_float2(t1r, t1i);
-      } else {
-        const float2 o = *p0;
-        *p0 = make_float2(t0r + (br * o.x - bi * o.y), t0i + (br * o.y + bi * o.x));
-        if (second) {
-          const float2 o1 = *p1;
-          *p1 = make_float2(t1r + (br * o1.x - bi * o1.y), t1i + (br * o1.y + bi * o1.x));
-        }
-      }
-    }
-  }
-}
-
-// Real epilogue: accumulator columns [col0, col0 + kCols) of real row `row`
-// (one TMEM lane per row, no pairing).  For real problems kFlagCPairs means
-// four consecutive columns contiguous and 16-byte aligned: one 16-byte store
-// per four values.  kFlagCCol16 as in store_tile.
-template <int kCols>
-__device__ __forceinline__ void store_tile_real(const GemmArgs& g, float* __restrict__ Cp,
-                                                int64_t row, bool row_ok, int64_t n0, int col0,
-                                                const float (&master)[kCols]) {
-  if (!row_ok) return;
-  const uint32_t flags = g.flags;
-  const bool accumulate = flags & kFlagAccumulate;
-  const bool beta_zero = flags & kFlagBetaZero;
-  const bool quads = flags & kFlagCPairs;
-  const bool col16 = flags & kFlagCCol16;
-  const float ar = (float)g.alpha[0], br = (float)g.beta[0];
-  const int64_t N = g.N;
-  const int64_t* __restrict__ csC = g.csC;
-  const int64_t uC_n = g.uC_n;
-  float* __restrict__ Cr = Cp + offs(g.rsC, g.uC_m, row);
-  int64_t blk = 0;
-#pragma unroll
-  for (int q = 0; q < kCols / 4; ++q) {
-    const int c = col0 + 4 * q;
-    const int64_t n = n0 + c;
-    if (col16 && (q & 3) == 0) {
-      const int64_t nb = n0 + col0 + 16 * (q >> 2);
-      blk = nb < N ? offs(csC, uC_n, nb) : 0;
-    }
-    if (n >= N) continue;
-    const int64_t on = col16 ? blk + (c - col0 - 16 * (q >> 2)) : offs(csC, uC_n, n);
-    float t[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) t[i] = ar * master[4 * q + i];
-    if (quads && n + 3 < N) {
-      float4* p4 = reinterpret_cast<float4*>(Cr + on);
-      if (accumulate) {
-        const float4 o = *p4;
-        *p4 = make_float4(o.x + t[0], o.y + t[1], o.z + t[2], o.w + t[3]);
-      } else if (beta_zero) {
-        *p4 = make_float4(t[0], t[1], t[2], t[3]);
-      } else {
-        const float4 o = *p4;
-        *p4 = make_float4(t[0] + br * o.x, t[1] + br * o.y, t[2] + br * o.z, t[3] + br * o.w);
-      }
-    } else {
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        if (n + i >= N) break;
-        float* p = Cr + (col16 ? on + i : (i == 0 ? on : offs(csC, uC_n, n + i)));
-        if (accumulate) *p += t[i];
-        else if (beta_zero) *p = t[i];
-        else *p = t[i] + br * *p;
-      }
     }
   }
 }
@@ -2111,343 +1927,6 @@ tc1m_contract(const GemmArgs args, const __grid_constant__ TmaMaps maps, int* er
   }
 }
 
-// ------------------------------------------------------ operand pieces ---
-// CTA pairs over operands split into bf16 pieces beforehand.
-//
-// A pre-pass (split_pieces) writes, for every complex row m of A, the two 1M
-// rows [re, -im, ...] and [im, re, ...] and, for every column n of B, the row
-// [re, im, ...] of its complex k (K fastest, real k = 2k + part), each value
-// split into P bf16 pieces exactly as tc1m_contract's converters split them
-// (split_bf16, conjugation first): P arrays per operand, rows `pitch`
-// elements apart.  The pair kernel then runs without converters: TMA loads
-// all pieces of a stage (3-D boxes: 64 real k x rows x P) into 128-byte
-// swizzled K-major shared memory, and one thread of the even CTA issues
-// tcgen05.mma.cta_group::2 with both operands read from shared memory.
-// Per accumulator its MMAs run in tc1m_contract's order (main product into
-// the chunk accumulators, a chunk every 16 MMAs of K = 16; corrections x0y1,
-// x1y0 [, x1y1, x0y2, x2y0] per K = 16 step into their own accumulator), so
-// the two forms give the same result bit for bit.
-//
-// The split happens once per operand element instead of once per tile that
-// reads it; the price is the pieces in device memory: 2 x 2 x 2P bytes per
-// complex element of A (the 1M rows) and 2 x 2P per element of B, written
-// and read back once by TMA per tile.
-constexpr int kPcStepK = 64;                   // real k per stage: one 128-byte row per piece
-constexpr int kPcABytes = 128 * 128;           // one A piece of a stage: 128 real rows
-constexpr int kPcBBytes = (kTileN / 2) * 128;  // one B piece: this CTA's 64 columns
-constexpr int kPcFold = 4;                     // stages per main chunk (16 MMAs of K = 16)
-constexpr int kPcBarrierBytes = 256;
-template <int P>
-constexpr int pc_stage_bytes() {
-  return P * (kPcABytes + kPcBBytes);
-}
-// Stages in the ring: as many as 227 KB hold (72 KB each for three pieces).
-template <int P>
-constexpr int pc_stages() {
-  return P == 3 ? 3 : 4;
-}
-template <int P>
-constexpr int pc_smem_bytes() {
-  return 1024 + pc_stages<P>() * pc_stage_bytes<P>() + kPcBarrierBytes;
-}
-
-// Pieces of one operand for a block of 32 rows x 32 complex k (256 threads):
-// the block reads its tile along whichever direction has unit stride
-// (through the offset vectors otherwise) and writes 16 bytes per piece and
-// output row per thread (4 complex k).  Blocks [0, blocks_a) cover A,
-// the rest B.  Rows past M or N are not written (the tensor maps end
-// there); complex k in [K, K rounded up to 4) are written as zeros.
-template <int P>
-__global__ void __launch_bounds__(256)
-split_pieces(const GemmArgs g, uint16_t* __restrict__ pa, uint16_t* __restrict__ pb,
-             int64_t pitch, int64_t plane_a, int64_t plane_b, int64_t blocks_a, int64_t tiles_k) {
-  __shared__ float2 tile[32][33];
-  const bool is_a = blockIdx.x < blocks_a;
-  const int64_t bid = is_a ? blockIdx.x : blockIdx.x - blocks_a;
-  const int64_t r0 = (bid / tiles_k) * 32, k0 = (bid % tiles_k) * 32;
-  const int64_t R = is_a ? g.M : g.N, K = g.K;
-  const float2* __restrict__ src = static_cast<const float2*>(is_a ? g.A : g.B);
-  const int64_t* rs = is_a ? g.rsA : g.csB;
-  const int64_t* ks = is_a ? g.csA : g.rsB;
-  const int64_t ur = is_a ? g.uA_m : g.uB_n;
-  const int64_t uk = is_a ? g.uA_k : g.uB_k;
-  const bool row_fast = ur == 1 && uk != 1;
-  const int t = threadIdx.x;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int r = row_fast ? (t & 31) : (t >> 5) + 8 * i;
-    const int k = row_fast ? (t >> 5) + 8 * i : (t & 31);
-    float2 v = make_float2(0.f, 0.f);
-    if (r0 + r < R && k0 + k < K) v = src[offs(rs, ur, r0 + r) + offs(ks, uk, k0 + k)];
-    tile[r][k] = v;
-  }
-  __syncthreads();
-  const int r = t >> 3, kq = 4 * (t & 7);
-  if (r0 + r >= R || k0 + kq >= K) return;
-  const bool conj = g.flags & (is_a ? kFlagConjA : kFlagConjB);
-  float2 v[4];
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    v[j] = tile[r][kq + j];
-    if (conj) v[j].y = -v[j].y;
-  }
-  const int64_t col = 2 * (k0 + kq);
-  uint32_t w[3][4];
-  if (is_a) {
-#pragma unroll
-    for (int part = 0; part < 2; ++part) {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float x0 = part ? v[j].y : v[j].x;
-        const float x1 = part ? v[j].x : -v[j].y;
-        split_bf16<P>(x0, x1, w[0][j], w[1][j], w[2][j]);
-      }
-      uint16_t* row = pa + (2 * (r0 + r) + part) * pitch + col;
-#pragma unroll
-      for (int p = 0; p < P; ++p)
-        *reinterpret_cast<uint4*>(row + p * plane_a) = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
-    }
-  } else {
-#pragma unroll
-    for (int j = 0; j < 4; ++j) split_bf16<P>(v[j].x, v[j].y, w[0][j], w[1][j], w[2][j]);
-    uint16_t* row = pb + (r0 + r) * pitch + col;
-#pragma unroll
-    for (int p = 0; p < P; ++p)
-      *reinterpret_cast<uint4*>(row + p * plane_b) = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
-  }
-}
-
-// The pair kernel over pieces.  Warps: 0 TMEM allocation and (even CTA, one
-// lane) MMA issue; 1 TMA (one lane per CTA); 2 (odd CTA, one lane) relays
-// the arrival of its stage to the even CTA's MMA thread; 4-11 fold the chunk
-// accumulators and write C (two warpgroups of 64 columns each, one TMEM lane
-// per thread), as tc1m_contract's converters do.
-template <int Prec>
-__global__ void __launch_bounds__(kThreads1, 1)
-tc1m_pieces(const GemmArgs args, const __grid_constant__ TmaMaps maps, int* err_flag) {
-  constexpr int P = Prec == kPrecBF16x6 ? 3 : 2;
-  constexpr int S = pc_stages<P>();
-  constexpr int kStageB = pc_stage_bytes<P>();
-  constexpr uint32_t kIdescP = ptx::idesc_f32acc(1u /*BF16*/, 256u, kTileN);
-  static_assert(8 * (3 * S + 6) <= kPcBarrierBytes, "barrier area");
-  static_assert(kStageB % 1024 == 0 && kPcBBytes % 1024 == 0, "swizzle atoms");
-
-  extern __shared__ __align__(16) uint8_t smem_raw[];
-  const uint32_t base = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
-  uint8_t* const base_ptr = smem_raw + (base - ptx::smem_u32(smem_raw));
-  const uint32_t bars = base + S * kStageB;
-  auto full_bar = [&](int s) { return bars + 8u * s; };
-  auto peer_bar = [&](int s) { return bars + 8u * (S + s); };
-  auto empty_bar = [&](int s) { return bars + 8u * (2 * S + s); };
-  auto chunk_full = [&](int b) { return bars + 8u * (3 * S + b); };
-  auto chunk_empty = [&](int b) { return bars + 8u * (3 * S + 2 + b); };
-  const uint32_t acc_bar = bars + 8u * (3 * S + 4);
-  const uint32_t tmem_slot = acc_bar + 8u;
-  volatile uint32_t* tmem_slot_ptr =
-      reinterpret_cast<volatile uint32_t*>(base_ptr + (tmem_slot - base));
-
-  const int tid = threadIdx.x;
-  const int warp = tid >> 5, lane = tid & 31;
-  const uint32_t rank = ptx::cluster_ctarank();
-  if (warp == 0) {
-    ptx::tmem_alloc2(tmem_slot, kTmemCols);
-    ptx::tmem_relinquish2();
-  }
-  if (tid == 32) {
-    for (int s = 0; s < S; ++s) {
-      ptx::mbar_init(full_bar(s), 1);
-      ptx::mbar_init(peer_bar(s), 1);
-      ptx::mbar_init(empty_bar(s), 1);
-    }
-    for (int b = 0; b < 2; ++b) {
-      ptx::mbar_init(chunk_full(b), 1);
-      ptx::mbar_init(chunk_empty(b), 2 * (kConverters1 / 32));
-    }
-    ptx::mbar_init(acc_bar, 1);
-    ptx::fence_mbar_init();
-  }
-  if (tid == 64) {
-    ptx::tma_prefetch_desc(&maps.a);
-    ptx::tma_prefetch_desc(&maps.b);
-  }
-  ptx::tc_fence_before();
-  ptx::cluster_sync();
-  ptx::tc_fence_after();
-  const uint32_t tmem = *tmem_slot_ptr;
-
-  // Tiles as in tc1m_contract's pair form: groups of 8 pair tiles along M
-  // sweep N; split-K rows over blockIdx.y.
-  const int64_t M = args.M, N = args.N;
-  const int64_t kb = static_cast<int64_t>(blockIdx.y) * args.k_per_split;
-  const int64_t K = min(args.K, kb + args.k_per_split);
-  constexpr int kRowsTile = 2 * kTileMc;
-  const int64_t tiles_m = (M + kRowsTile - 1) / kRowsTile;
-  const int64_t tiles_n = (N + kTileN - 1) / kTileN;
-  constexpr int64_t G = 8;
-  const int64_t t = blockIdx.x >> 1;
-  const int64_t group = t / (G * tiles_n);
-  const int64_t first_m = group * G;
-  const int64_t gsize = min(G, tiles_m - first_m);
-  const int64_t tm = first_m + (t % (G * tiles_n)) % gsize;
-  const int64_t tn = (t % (G * tiles_n)) / gsize;
-  const int64_t m0 = tm * kRowsTile + rank * kTileMc, n0 = tn * kTileN;
-  // Stages of 64 real k over this CTA row's real K range [2 kb, 2 K).
-  const int64_t ksteps = (2 * (K - kb) + kPcStepK - 1) / kPcStepK;
-
-  if (warp == 0) {
-    // ---------------------------------------------------------- MMA issue ---
-    if (lane == 0 && rank == 0) {
-      const uint64_t desc0 = ptx::smem_desc_sw128(base);
-      const uint32_t d_corr = tmem + kCorrCol;
-      for (int64_t s = 0; s < ksteps; ++s) {
-        const int st = static_cast<int>(s % S);
-        const uint32_t ph = static_cast<uint32_t>((s / S) & 1);
-        const int64_t c = s / kPcFold;
-        const int buf = static_cast<int>(c & 1);
-        const bool chunk_start = (s % kPcFold) == 0;
-        if (chunk_start && c >= 2 &&
-            !ptx::mbar_wait(chunk_empty(buf), static_cast<uint32_t>(((c - 2) >> 1) & 1))) {
-          record_error(err_flag, kErrChunkWait);
-          break;
-        }
-        if (!ptx::mbar_wait(full_bar(st), ph) || !ptx::mbar_wait(peer_bar(st), ph)) {
-          record_error(err_flag, kErrFullWait);
-          break;
-        }
-        ptx::tc_fence_after();
-        const uint32_t d_main = tmem + (buf ? kChunkCol1 : kChunkCol0);
-        const uint64_t ds = desc0 + static_cast<uint64_t>((st * kStageB) >> 4);
-        // K = 16 steps of this stage inside the CTA row's K range: a split
-        // may end half way through a stage (its K a multiple of 16 complex);
-        // the rest of the box belongs to the next split.  Past the end of K
-        // the box is zero-filled.
-        const int64_t rem = 2 * (K - kb) - kPcStepK * s;
-        const int nkk = rem >= kPcStepK ? 4 : static_cast<int>((rem + 15) / 16);
-        // Piece p, K = 16 step kk: A at +p x 16 KB, B after the A pieces at
-        // +p x 8 KB, each +32 bytes per step inside the 128-byte rows.
-        auto da = [&](int p, int kk) {
-          return ds + static_cast<uint64_t>((p * kPcABytes + 32 * kk) >> 4);
-        };
-        auto db = [&](int p, int kk) {
-          return ds + static_cast<uint64_t>((P * kPcABytes + p * kPcBBytes + 32 * kk) >> 4);
-        };
-#pragma unroll
-        for (int kk = 0; kk < 4; ++kk)
-          if (kk < nkk)
-            ptx::mma_f16_ss2(d_main, da(0, kk), db(0, kk), kIdescP,
-                             (chunk_start && kk == 0) ? 0u : 1u);
-#pragma unroll
-        for (int kk = 0; kk < 4; ++kk) {
-          if (kk >= nkk) break;
-          ptx::mma_f16_ss2(d_corr, da(0, kk), db(1, kk), kIdescP, (s == 0 && kk == 0) ? 0u : 1u);
-          ptx::mma_f16_ss2(d_corr, da(1, kk), db(0, kk), kIdescP, 1u);
-          if (P == 3) {
-            ptx::mma_f16_ss2(d_corr, da(1, kk), db(1, kk), kIdescP, 1u);
-            ptx::mma_f16_ss2(d_corr, da(0, kk), db(2, kk), kIdescP, 1u);
-            ptx::mma_f16_ss2(d_corr, da(2, kk), db(0, kk), kIdescP, 1u);
-          }
-        }
-        ptx::mma_commit2(empty_bar(st));
-        if ((s % kPcFold) == kPcFold - 1 || s == ksteps - 1) ptx::mma_commit2(chunk_full(buf));
-      }
-      // Signal the epilogue (also after an abort), then make sure no MMA is
-      // still writing TMEM before it is freed.
-      ptx::mma_commit2(acc_bar);
-      if (!ptx::mbar_wait(acc_bar, 0)) record_error(err_flag, kErrAccWait);
-    }
-    __syncwarp();
-  } else if (warp == 1) {
-    // ---------------------------------------------------------------- TMA ---
-    if (lane == 0) {
-      const int a_row = static_cast<int>(2 * m0);                   // 1M rows of this CTA
-      const int b_row = static_cast<int>(n0 + rank * (kTileN / 2));  // its B columns
-      for (int64_t s = 0; s < ksteps; ++s) {
-        const int st = static_cast<int>(s % S);
-        const uint32_t ph = static_cast<uint32_t>((s / S) & 1);
-        if (!ptx::mbar_wait(empty_bar(st), ph ^ 1u)) {
-          record_error(err_flag, kErrRawWait);
-          break;
-        }
-        const uint32_t dst = base + st * kStageB;
-        const int k0 = static_cast<int>(2 * kb + kPcStepK * s);
-        ptx::mbar_arrive_expect_tx(full_bar(st), static_cast<uint32_t>(kStageB));
-        ptx::tma_load_3d(dst, &maps.a, k0, a_row, 0, full_bar(st));
-        ptx::tma_load_3d(dst + P * kPcABytes, &maps.b, k0, b_row, 0, full_bar(st));
-      }
-    }
-    __syncwarp();
-  } else if (warp == 2) {
-    // -------------------------------------------------------------- relay ---
-    if (lane == 0 && rank == 1) {
-      for (int64_t s = 0; s < ksteps; ++s) {
-        const int st = static_cast<int>(s % S);
-        if (!ptx::mbar_wait(full_bar(st), static_cast<uint32_t>((s / S) & 1))) {
-          record_error(err_flag, kErrFullWait);
-          break;
-        }
-        ptx::mbar_arrive_cluster(ptx::mapa(peer_bar(st), 0));
-      }
-    }
-    __syncwarp();
-  } else if (tid >= kConvBase) {
-    // ------------------------------------------------- fold and epilogue ---
-    const int pt = tid - kConvBase;
-    const int wg = pt >> 7;
-    const int q = (pt >> 5) & 3;
-    const int rho = 32 * q + lane;
-    const int ci = rho >> 1;
-    const int part = rho & 1;
-    const uint32_t lane_base = static_cast<uint32_t>(32 * q) << 16;
-    const bool row_ok = (m0 + ci) < M;
-    float master[kMC1];
-#pragma unroll
-    for (int j = 0; j < kMC1; ++j) master[j] = 0.f;
-    auto fold_from = [&](uint32_t col) {
-#pragma unroll
-      for (int cc = 0; cc < kMC1 / 32; ++cc) {
-        uint32_t r[32];
-        ptx::tmem_ld32_sync(tmem + lane_base + col + kMC1 * wg + 32u * cc, r);
-#pragma unroll
-        for (int j = 0; j < 32; ++j) master[32 * cc + j] += __uint_as_float(r[j]);
-      }
-    };
-    bool ok = true;
-    const int64_t nchunks = (ksteps + kPcFold - 1) / kPcFold;
-    for (int64_t c = 0; c + 1 < nchunks; ++c) {
-      const int buf = static_cast<int>(c & 1);
-      if (!ptx::mbar_wait(chunk_full(buf), static_cast<uint32_t>((c >> 1) & 1))) {
-        record_error(err_flag, kErrChunkWait);
-        ok = false;
-        break;
-      }
-      ptx::tc_fence_after();
-      fold_from(buf ? kChunkCol1 : kChunkCol0);
-      ptx::tc_fence_before();
-      __syncwarp();
-      if (lane == 0) ptx::mbar_arrive_cluster(ptx::mapa(chunk_empty(buf), 0));
-    }
-    if (!ptx::mbar_wait(acc_bar, 0)) {
-      record_error(err_flag, kErrAccWait);
-      ok = false;
-    }
-    ptx::tc_fence_after();
-    if (ok) {
-      fold_from(((nchunks - 1) & 1) ? kChunkCol1 : kChunkCol0);
-      fold_from(kCorrCol);
-      float2* __restrict__ Cp =
-          static_cast<float2*>(args.C) + static_cast<int64_t>(blockIdx.y) * args.c_split_stride;
-      store_tile<kMC1>(args, Cp, m0 + ci, row_ok, n0, wg * kMC1, part, master);
-    }
-  }
-
-  ptx::tc_fence_before();
-  ptx::cluster_sync();
-  if (warp == 0) {
-    ptx::tc_fence_after();
-    ptx::tmem_dealloc2(tmem, kTmemCols);
-  }
-}
-
 // ------------------------------------------------------------------ host ---
 using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
                                    const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
@@ -2562,85 +2041,6 @@ cudaError_t launch_pair_prec(int method, int amode, int bmode, const GemmArgs& a
     default:
       return launch_pair<kPrecTF32x3>(amode, bmode, args, maps, stream, err_flag, tiles);
   }
-}
-
-// Operand pieces: row pitch in bf16 elements (real K rounded up to 16 bytes).
-int64_t pieces_pitch(int64_t K) { return (2 * K + 7) / 8 * 8; }
-
-// 3-D map over P piece arrays (`plane` elements apart) of `rows` rows of
-// `kreal` bf16 (`pitch` apart), loaded as boxes of 64 k x box_rows x P with
-// the 128-byte swizzle.
-bool make_map_pieces(CUtensorMap* map, const void* base, int64_t kreal, int64_t rows,
-                     int64_t pitch, int64_t plane, int pieces, uint32_t box_rows) {
-  EncodeTiledFn fn = encode_fn();
-  if (!fn || reinterpret_cast<uintptr_t>(base) % 16 != 0) return false;
-  if (kreal <= 0 || rows <= 0 || kreal >= (int64_t(1) << 31) || rows >= (int64_t(1) << 31))
-    return false;
-  cuuint64_t dims[3] = {static_cast<cuuint64_t>(kreal), static_cast<cuuint64_t>(rows),
-                        static_cast<cuuint64_t>(pieces)};
-  cuuint64_t strides[2] = {static_cast<cuuint64_t>(pitch * 2),
-                           static_cast<cuuint64_t>(plane * 2)};
-  cuuint32_t box[3] = {static_cast<cuuint32_t>(kPcStepK), box_rows, static_cast<cuuint32_t>(pieces)};
-  cuuint32_t estr[3] = {1, 1, 1};
-  return fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT16, 3, const_cast<void*>(base), dims, strides, box,
-            estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
-// The pieces of A and B not in `ready` (one launch, counted in *kernels;
-// into ws, A's first), then the pair kernel over them: tiles.x = 2 x pair
-// tiles, tiles.y = splits.
-template <int Prec>
-cudaError_t launch_pieces_prec(const GemmArgs& g, void* ws, const PiecesReady* ready, dim3 tiles,
-                               cudaStream_t stream, int* err_flag, int* kernels,
-                               cudaEvent_t* main_ev) {
-  constexpr int P = Prec == kPrecBF16x6 ? 3 : 2;
-  const int64_t pitch = pieces_pitch(g.K);
-  const bool ra = ready && ready->a, rb = ready && ready->b;
-  const int64_t plane_a = ra ? ready->a_plane : 2 * g.M * pitch;
-  const int64_t plane_b = rb ? ready->b_plane : g.N * pitch;
-  uint16_t* const w = static_cast<uint16_t*>(ws);
-  uint16_t* pa = ra ? static_cast<uint16_t*>(const_cast<void*>(ready->a)) : w;
-  uint16_t* pb = rb ? static_cast<uint16_t*>(const_cast<void*>(ready->b)) : w + (ra ? 0 : P * plane_a);
-  TmaMaps maps;
-  if (!make_map_pieces(&maps.a, pa, 2 * g.K, 2 * g.M, pitch, plane_a, P, 128) ||
-      !make_map_pieces(&maps.b, pb, 2 * g.K, g.N, pitch, plane_b, P, kTileN / 2))
-    return cudaErrorInvalidConfiguration;
-  const int64_t tiles_k = (g.K + 31) / 32;
-  const int64_t blocks_a = ra ? 0 : (g.M + 31) / 32 * tiles_k;
-  const int64_t blocks_b = rb ? 0 : (g.N + 31) / 32 * tiles_k;
-  if (blocks_a + blocks_b >= (int64_t(1) << 31)) return cudaErrorInvalidConfiguration;
-  cudaError_t e;
-  if (blocks_a + blocks_b > 0) {
-    split_pieces<P><<<static_cast<unsigned>(blocks_a + blocks_b), 256, 0, stream>>>(
-        g, pa, pb, pitch, plane_a, plane_b, blocks_a, tiles_k);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    ++*kernels;
-  }
-  constexpr int kSmem = pc_smem_bytes<P>();
-  static_assert(kSmem <= 227 * 1024, "shared memory budget");
-  static bool attr_set = false;
-  if (!attr_set) {
-    e = cudaFuncSetAttribute(tc1m_pieces<Prec>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
-    if (e != cudaSuccess) return e;
-    attr_set = true;
-  }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = tiles;
-  cfg.blockDim = dim3(kThreads1);
-  cfg.dynamicSmemBytes = kSmem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  if (main_ev) cudaEventRecord(main_ev[0], stream);
-  e = cudaLaunchKernelEx(&cfg, tc1m_pieces<Prec>, g, maps, err_flag);
-  if (main_ev) cudaEventRecord(main_ev[1], stream);
-  return e;
 }
 
 template <int AMode, int Prec, bool kReal>
@@ -2760,9 +2160,10 @@ bool common_block_stride16(const std::vector<int64_t>& rows, const std::vector<i
 // Epilogue store flags of a problem (kFlagCPairs, kFlagCCol16) from C's row
 // and column offsets: the uniform strides where the arguments carry them (a
 // uniform bundle, the dense split-K workspace), else the plan's vectors.
-uint32_t c_store_flags(const GemmArgs& g, const HostPlan& plan) {
-  auto col = [&](int64_t n) { return g.uC_n >= 0 ? n * g.uC_n : plan.csC[n]; };
-  auto row = [&](int64_t m) { return g.uC_m >= 0 ? m * g.uC_m : plan.rsC[m]; };
+uint32_t c_store_flags(const GemmArgs& g, const std::vector<int64_t>& rsC,
+                       const std::vector<int64_t>& csC) {
+  auto col = [&](int64_t n) { return g.uC_n >= 0 ? n * g.uC_n : csC[n]; };
+  auto row = [&](int64_t m) { return g.uC_m >= 0 ? m * g.uC_m : rsC[m]; };
   uint32_t f = 0;
   bool col16 = true;
   if (g.uC_n >= 0) {
@@ -2817,9 +2218,10 @@ bool make_map_f32(CUtensorMap* map, const void* base, int64_t inner, int64_t out
 
 // Real epilogue flags: kFlagCCol16 as for complex; kFlagCPairs for four
 // consecutive columns contiguous with 16-byte aligned starts.
-uint32_t c_store_flags_real(const GemmArgs& g, const HostPlan& plan) {
-  auto col = [&](int64_t n) { return g.uC_n >= 0 ? n * g.uC_n : plan.csC[n]; };
-  auto row = [&](int64_t m) { return g.uC_m >= 0 ? m * g.uC_m : plan.rsC[m]; };
+uint32_t c_store_flags_real(const GemmArgs& g, const std::vector<int64_t>& rsC,
+                            const std::vector<int64_t>& csC) {
+  auto col = [&](int64_t n) { return g.uC_n >= 0 ? n * g.uC_n : csC[n]; };
+  auto row = [&](int64_t m) { return g.uC_m >= 0 ? m * g.uC_m : rsC[m]; };
   uint32_t f = 0;
   bool col16 = true;
   if (g.uC_n >= 0) {
@@ -2861,7 +2263,7 @@ bool tc_prepare_real(const GemmArgs& g, const HostPlan& plan, int splits, int* a
   if (g.M >= (int64_t(1) << 31) / 128 || g.N >= (int64_t(1) << 31) / kTileN) return false;
   *out = g;
   out->flags = (g.flags & ~(kFlagCPairs | kFlagCCol16 | kFlagConjA | kFlagConjB)) |
-               c_store_flags_real(g, plan);
+               c_store_flags_real(g, plan.rsC, plan.csC);
   std::memset(static_cast<void*>(maps), 0, sizeof(*maps));
   *amode = kGatherMK;
   if (plan.uA_m == 1 && plan.uA_k >= 0 &&
@@ -2955,7 +2357,7 @@ bool tc_prepare(const GemmArgs& g, const HostPlan& plan, int splits, TcProblem* 
   if (tile_n == 0) tile_n = tc_default_tile_n(g.N);
   if (tile_n != 16 && tile_n != 32 && tile_n != 64 && tile_n != 128) return false;
   p->g = g;
-  p->g.flags = (g.flags & ~(kFlagCPairs | kFlagCCol16)) | c_store_flags(g, plan);
+  p->g.flags = (g.flags & ~(kFlagCPairs | kFlagCCol16)) | c_store_flags(g, plan.rsC, plan.csC);
   p->tile_n = tile_n;
   p->fold_shift = 2;  // kFold = 4 stages per main chunk
   p->skinny = 0;
@@ -3094,34 +2496,58 @@ size_t tc_pack_bytes(int dtype, const HostPlan& plan) {
   return b;
 }
 
-size_t tc_pieces_bytes(int dtype, int method, int64_t M, int64_t N, int64_t K,
-                       const PiecesReady* ready) {
-  if (dtype != T1M_COMPLEX64 || M <= kTileMc || N <= 0 || K <= 0) return 0;
-  if (method != T1M_METHOD_TC_BF16X3 && method != T1M_METHOD_TC_BF16X6 && method != kMethodTcAuto)
-    return 0;
-  const size_t pieces = method == T1M_METHOD_TC_BF16X3 ? 2 : 3;
-  const int64_t rows = (ready && ready->a ? 0 : 2 * M) + (ready && ready->b ? 0 : N);
-  return pieces * static_cast<size_t>(rows) * static_cast<size_t>(pieces_pitch(K)) * 2u;
+// Real rows of an operand's pieces and real k of a product.
+static int64_t pieces_rows(int dtype, bool operand_a, int64_t rows) {
+  return operand_a && dtype == T1M_COMPLEX64 ? 2 * rows : rows;
+}
+static int64_t pieces_kreal(int dtype, int64_t K) { return dtype == T1M_COMPLEX64 ? 2 * K : K; }
+
+int64_t tc_pieces_groups(int dtype, bool operand_a, int64_t rows) {
+  return piece_groups(pieces_rows(dtype, operand_a, rows));
 }
 
-int64_t tc_pieces_pitch(int64_t K) { return pieces_pitch(K); }
+size_t tc_pieces_array_bytes(int dtype, int pieces, int64_t groups, int64_t K) {
+  return pieces <= 0 ? 0 : piece_bytes(pieces, 8 * groups, pieces_kreal(dtype, K));
+}
 
-cudaError_t tc_split_operand(int pieces, bool operand_a, const GemmArgs& g, void* out,
-                             int64_t plane, cudaStream_t s) {
-  const int64_t pitch = pieces_pitch(g.K);
-  const int64_t tiles_k = (g.K + 31) / 32;
-  const int64_t blocks = ((operand_a ? g.M : g.N) + 31) / 32 * tiles_k;
-  if (blocks <= 0) return cudaSuccess;
-  if (blocks >= (int64_t(1) << 31)) return cudaErrorInvalidConfiguration;
-  uint16_t* o = static_cast<uint16_t*>(out);
-  const unsigned grid = static_cast<unsigned>(blocks);
-  // B alone: no A blocks (blocks_a = 0), B's arrays at o.
-  const int64_t ba = operand_a ? blocks : 0;
-  if (pieces == 2)
-    split_pieces<2><<<grid, 256, 0, s>>>(g, o, o, pitch, plane, plane, ba, tiles_k);
-  else
-    split_pieces<3><<<grid, 256, 0, s>>>(g, o, o, pitch, plane, plane, ba, tiles_k);
-  return cudaGetLastError();
+size_t tc_pieces_bytes(int dtype, int pieces, int64_t M, int64_t N, int64_t K,
+                       const PiecesReady* ready) {
+  if (pieces <= 0 || M <= 0 || N <= 0 || K <= 0) return 0;
+  const int64_t kr = pieces_kreal(dtype, K);
+  return (ready && ready->a ? 0 : piece_bytes(pieces, pieces_rows(dtype, true, M), kr)) +
+         (ready && ready->b ? 0 : piece_bytes(pieces, N, kr));
+}
+
+// The split pass of one operand of g.
+static PieceSplit piece_split_args(int dtype, bool operand_a, bool swapped, const GemmArgs& g,
+                                   const HostPlan& plan, void* out, int64_t groups) {
+  PieceSplit s{};
+  s.src = operand_a ? g.A : g.B;
+  s.ro = operand_a ? g.rsA : g.csB;
+  s.ko = operand_a ? g.csA : g.rsB;
+  s.ur = operand_a ? g.uA_m : g.uB_n;
+  s.uk = operand_a ? g.uA_k : g.uB_k;
+  s.R = operand_a ? g.M : g.N;
+  s.K = g.K;
+  s.out = static_cast<uint8_t*>(out);
+  s.rg = groups;
+  // The 1M rows belong to the product's first operand.
+  s.expand = operand_a != swapped && dtype == T1M_COMPLEX64 ? 1 : 0;
+  s.conj = (g.flags & (operand_a ? kFlagConjA : kFlagConjB)) ? 1 : 0;
+  // Read along the source's unit-stride mode: a row mode, the first K mode
+  // (or none), or a later K mode whose k step is whole stages.
+  const int64_t step = pack_step(plan.modes_k, !operand_a, operand_a ? plan.modes_m : plan.modes_n);
+  const int64_t stage = dtype == T1M_COMPLEX64 ? 16 : 32;
+  s.step = step;
+  s.mode = step == 0 ? kSplitRows : step > 0 && step % stage == 0 ? kSplitStep : kSplitK;
+  return s;
+}
+
+cudaError_t tc_split_operand(int dtype, int pieces, bool operand_a, const GemmArgs& g,
+                             const HostPlan& plan, void* out, int64_t groups, cudaStream_t s) {
+  const PieceSplit op = piece_split_args(dtype, operand_a, false, g, plan, out, groups);
+  const bool real = dtype == T1M_FLOAT32;
+  return launch_piece_split(pieces, real, &op, 1, nullptr, piece_split_blocks(real, op), s);
 }
 
 size_t tc_panel_bytes(int dtype, int64_t M, int64_t N, int64_t K) {
@@ -3133,29 +2559,121 @@ size_t tc_panel_bytes(int dtype, int64_t M, int64_t N, int64_t K) {
 }
 
 // Method of the pieces form for a product, 0 where it does not run: the
-// bf16 methods (the automatic method as BF16x6) with two or more 64-row M
-// tiles; any operand layout for T1M_TILE_PIECES (the split pass reads through
-// the scatter vectors), for T1M_TILE_AUTO where both operands load by TMA
-// (where CTA pairs would otherwise run).
-static int pieces_method(int method, int form, const TcProblem& p) {
-  if (p.tiles_m < 2) return 0;
+// bf16 methods (the automatic method as BF16x6).  T1M_TILE_PIECES takes it
+// for two or more 64-row M tiles; T1M_TILE_AUTO, unless both operands load
+// by TMA (`tma`), where the output is large enough that writing the pieces
+// and reading them back costs less than gathering and splitting per tile:
+// abcd,dbea->ec (96 x 64, K = 36864) takes 86 us over pieces, 70 packed and
+// split in the kernel; abcd,ebfd->aecf (1024^3) 56 against 77.
+static int pieces_method(int method, int dtype, int form, int64_t M, int64_t N, bool tma) {
+  if (M <= (dtype == T1M_COMPLEX64 ? kTileMc : 2 * kTileMc)) return 0;
   const int pm = method == kMethodTcAuto ? T1M_METHOD_TC_BF16X6 : method;
   if (pm != T1M_METHOD_TC_BF16X3 && pm != T1M_METHOD_TC_BF16X6) return 0;
   if (form == T1M_TILE_PIECES) return pm;
   if (form != T1M_TILE_AUTO) return 0;
+  // 2 M N / (M + N) >= 128: enough products per split element.
+  return tma || M * N >= 64 * (M + N) ? pm : 0;
+}
+
+// Both operands a uniform view with a unit-stride direction that TMA loads.
+static bool plain_tma(const TcProblem& p) {
   const bool a_block = (p.block_maps & 1) || p.amode == kAMK16;
   const bool b_block = (p.block_maps & 2) != 0;
-  const bool tma_a = !a_block && (p.amode == kAMK || p.amode == kAKM);
-  const bool tma_b = !b_block && (p.bmode == kBNK || p.bmode == kBKN);
-  return tma_a && tma_b ? pm : 0;
+  return !a_block && (p.amode == kAMK || p.amode == kAKM) && !b_block &&
+         (p.bmode == kBNK || p.bmode == kBKN);
+}
+
+static int pieces_of(int method) {
+  return method == T1M_METHOD_TC_BF16X3 ? 2 : method == T1M_METHOD_TC_BF16X6 ? 3 : 0;
 }
 
 int tc_pieces_count(int method, int dtype, const GemmArgs& g, const HostPlan& plan, int form) {
-  if (dtype != T1M_COMPLEX64 || !tc_supported(method, dtype, plan)) return 0;
-  TcProblem p;
-  if (!tc_prepare(g, plan, 1, &p)) return 0;
-  const int pm = pieces_method(method, form, p);
-  return pm == T1M_METHOD_TC_BF16X3 ? 2 : pm == T1M_METHOD_TC_BF16X6 ? 3 : 0;
+  if (!tc_supported(method, dtype, plan)) return 0;
+  bool tma = false;
+  if (dtype == T1M_COMPLEX64) {
+    TcProblem p;
+    tma = tc_prepare(g, plan, 1, &p) && plain_tma(p);
+  }
+  return pieces_of(pieces_method(method, dtype, form, g.M, g.N, tma));
+}
+
+// Whether the product runs with its operands exchanged: the kernel's rows
+// (the lanes of a warp) should run along C's unit stride, so a warp writes
+// whole lines; and of equally good orders the complex one that expands the
+// smaller operand into 1M rows.  Operands that are already split keep theirs.
+static bool swap_pieces(int dtype, const GemmArgs& g, const HostPlan& plan,
+                        const PiecesReady* ready) {
+  if (ready && (ready->a || ready->b)) return false;
+  auto unit = [](int64_t u, const std::vector<int64_t>& v, int64_t n) {
+    return n > 1 && (u >= 0 ? u : v[1] - v[0]) == 1;
+  };
+  const bool rows = unit(g.uC_m, plan.rsC, g.M), cols = unit(g.uC_n, plan.csC, g.N);
+  if (rows != cols) return cols;
+  return dtype == T1M_COMPLEX64 && g.N < g.M;
+}
+
+// The product of g over pieces (C, its offsets and epilogue forms), with the
+// operands exchanged or not.
+static void pieces_problem(int dtype, const GemmArgs& g, const HostPlan& plan, bool swap,
+                           PieceProblem* p) {
+  p->g = g;
+  p->swapped = swap ? 1 : 0;
+  if (swap) {
+    std::swap(p->g.M, p->g.N);
+    std::swap(p->g.rsC, p->g.csC);
+    std::swap(p->g.uC_m, p->g.uC_n);
+  }
+  p->g.flags &= ~(kFlagCPairs | kFlagCCol16);
+  const std::vector<int64_t>&r = swap ? plan.csC : plan.rsC, &c = swap ? plan.rsC : plan.csC;
+  p->g.flags |= dtype == T1M_FLOAT32 ? c_store_flags_real(p->g, r, c) : c_store_flags(p->g, r, c);
+}
+
+// The product over pieces: the operands not in `ready` split into `ws` (one
+// launch for two uniform views, else one per operand), then the pair kernel.
+static cudaError_t launch_pieces(int method, int dtype, const GemmArgs& g, const HostPlan& plan,
+                                 int splits, void* ws, const PiecesReady* ready,
+                                 cudaStream_t stream, int* err_flag, int* kernels,
+                                 cudaEvent_t* main_ev) {
+  const bool real = dtype == T1M_FLOAT32;
+  const int P = pieces_of(method);
+  const bool ra = ready && ready->a, rb = ready && ready->b;
+  PieceProblem p{};
+  const bool swap = swap_pieces(dtype, g, plan, ready);
+  pieces_problem(dtype, g, plan, swap, &p);
+  p.rg_a = ra ? ready->a_groups : tc_pieces_groups(dtype, true, p.g.M);
+  p.rg_b = rb ? ready->b_groups : tc_pieces_groups(dtype, false, p.g.N);
+  uint8_t* const w = static_cast<uint8_t*>(ws);
+  const size_t abytes = ra ? 0 : piece_bytes(P, pieces_rows(dtype, true, p.g.M), pieces_kreal(dtype, g.K));
+  uint8_t* const pa = ra ? static_cast<uint8_t*>(const_cast<void*>(ready->a)) : w;
+  uint8_t* const pb = rb ? static_cast<uint8_t*>(const_cast<void*>(ready->b)) : w + abytes;
+  p.a = pa;
+  p.b = pb;
+  PieceSplit ops[2];
+  int n = 0;
+  if (!ra) ops[n++] = piece_split_args(dtype, !swap, swap, g, plan, pa, p.rg_a);
+  if (!rb) ops[n++] = piece_split_args(dtype, swap, swap, g, plan, pb, p.rg_b);
+  const bool uniform = g.uA_m >= 0 && g.uA_k >= 0 && g.uB_k >= 0 && g.uB_n >= 0;
+  cudaError_t e;
+  if (n == 2 && uniform) {
+    ops[1].block_begin = piece_split_blocks(real, ops[0]);
+    e = launch_piece_split(P, real, ops, 2, nullptr,
+                           ops[1].block_begin + piece_split_blocks(real, ops[1]), stream);
+    if (e != cudaSuccess) return e;
+    ++*kernels;
+  } else {
+    for (int i = 0; i < n; ++i) {
+      e = launch_piece_split(P, real, &ops[i], 1, nullptr, piece_split_blocks(real, ops[i]), stream);
+      if (e != cudaSuccess) return e;
+      ++*kernels;
+    }
+  }
+  const int tn = piece_tile_n(real, p.g.M, p.g.N, g.K, splits);
+  piece_set_tiles(real, &p, tn, splits);
+  if (main_ev) cudaEventRecord(main_ev[0], stream);
+  e = launch_piece_products(P, real, tn > 128, &p, nullptr, 1, piece_tiles(p), stream, err_flag);
+  if (main_ev) cudaEventRecord(main_ev[1], stream);
+  if (e == cudaSuccess) ++*kernels;
+  return e;
 }
 
 cudaError_t launch_tc(int method, int dtype, const GemmArgs& args, const HostPlan& plan,
@@ -3275,6 +2793,11 @@ cudaError_t launch_tc(int method, int dtype, const GemmArgs& args, const HostPla
   };
   GemmArgs packed_args = args;
   const HostPlan* packed_plan = &plan;
+  // Whether the panel workspace holds the product's pieces.
+  auto pieces_ws_ok = [&](int pm) {
+    const size_t bytes = tc_pieces_bytes(dtype, pieces_of(pm), args.M, args.N, args.K, ready);
+    return bytes == 0 || (panel && panel_bytes >= bytes);
+  };
   if (real) {
     // Real float32: the one-tile kernel with uniform-view TMA, gathers or panels.
     int am = kGatherMK, bm = kGatherNK;
@@ -3282,6 +2805,17 @@ cudaError_t launch_tc(int method, int dtype, const GemmArgs& args, const HostPla
     GemmArgs gr;
     if (!tc_prepare_real(args, plan, splits, &am, &bm, &maps, &gr))
       return cudaErrorInvalidConfiguration;
+    if (const int pm = pieces_method(method, dtype, form, args.M, args.N,
+                                     am != kGatherMK && bm != kGatherNK)) {
+      if (pieces_ws_ok(pm)) {
+        if (used_method) *used_method = pm;
+        set_path(one_tile_a(am), bm == kGatherNK ? T1M_PATH_B_PANELS : one_tile_b(bm), false,
+                 am == kGatherMK, false);
+        if (path) *path |= T1M_PATH_PAIR | T1M_PATH_PIECES;
+        return launch_pieces(pm, dtype, gr, plan, splits, panel, ready, stream, err_flag, kernels,
+                             main_ev);
+      }
+    }
     const bool pa = am == kGatherMK && a_big;
     const bool pb = bm == kGatherNK && b_big && !panels_ok;
     if (pa || pb) {
@@ -3309,26 +2843,20 @@ cudaError_t launch_tc(int method, int dtype, const GemmArgs& args, const HostPla
   }
   TcProblem p;
   if (!tc_prepare(args, plan, splits, &p)) return cudaErrorInvalidConfiguration;
-  if (const int pm = pieces_method(method, form, p)) {
+  if (const int pm = pieces_method(method, dtype, form, args.M, args.N, plain_tma(p))) {
     // Operand pieces: split once (the operands not in `ready`) into the
     // panel workspace, then CTA pairs with both MMA operands in shared
     // memory.  Without the workspace the product takes the forms below.
-    const size_t need = tc_pieces_bytes(dtype, pm, args.M, args.N, args.K, ready);
-    if (need == 0 || (panel && panel_bytes >= need)) {
+    if (pieces_ws_ok(pm)) {
       if (used_method) *used_method = pm;
-      const int64_t pair_m = (p.g.M + 2 * kTileMc - 1) / (2 * kTileMc);
-      const dim3 pgrid(static_cast<unsigned>(2 * pair_m * p.tiles_n),
-                       static_cast<unsigned>(splits));
-      const cudaError_t e =
-          pm == T1M_METHOD_TC_BF16X3
-              ? launch_pieces_prec<kPrecBF16x3>(p.g, panel, ready, pgrid, stream, err_flag, kernels,
-                                                main_ev)
-              : launch_pieces_prec<kPrecBF16x6>(p.g, panel, ready, pgrid, stream, err_flag, kernels,
-                                                main_ev);
-      if (e == cudaSuccess) ++*kernels;
-      set_path(p.amode, p.bmode, false, false, false);
-      if (path && e == cudaSuccess) *path |= T1M_PATH_PAIR | T1M_PATH_PIECES;
-      return e;
+      // An operand without a TMA view counts as repacked: its split pass
+      // gathers it into a dense copy that the product loads in bulk.
+      const bool a_tma = !(p.block_maps & 1) && (p.amode == kAMK || p.amode == kAKM);
+      const bool b_tma = !(p.block_maps & 2) && (p.bmode == kBNK || p.bmode == kBKN);
+      set_path(a_tma ? p.amode : kAKM, b_tma ? p.bmode : T1M_PATH_B_PANELS, false, !a_tma, false);
+      if (path) *path |= T1M_PATH_PAIR | T1M_PATH_PIECES;
+      return launch_pieces(pm, dtype, p.g, plan, splits, panel, ready, stream, err_flag, kernels,
+                           main_ev);
     }
   }
   {
