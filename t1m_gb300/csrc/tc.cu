@@ -2514,8 +2514,13 @@ size_t tc_pieces_bytes(int dtype, int pieces, int64_t M, int64_t N, int64_t K,
                        const PiecesReady* ready) {
   if (pieces <= 0 || M <= 0 || N <= 0 || K <= 0) return 0;
   const int64_t kr = pieces_kreal(dtype, K);
-  return (ready && ready->a ? 0 : piece_bytes(pieces, pieces_rows(dtype, true, M), kr)) +
-         (ready && ready->b ? 0 : piece_bytes(pieces, N, kr));
+  // Either operand may become the product's first, with the 1M rows
+  // (swap_pieces); operands that are already split keep their order.
+  if (!ready || (!ready->a && !ready->b))
+    return piece_bytes(pieces, pieces_rows(dtype, true, std::max(M, N)), kr) +
+           piece_bytes(pieces, std::min(M, N), kr);
+  return (ready->a ? 0 : piece_bytes(pieces, pieces_rows(dtype, true, M), kr)) +
+         (ready->b ? 0 : piece_bytes(pieces, N, kr));
 }
 
 // The split pass of one operand of g.

@@ -68,3 +68,21 @@ def test_piece_edges(ctx, torch_cuda, case, dt, layout, beta):
     pair, rp = _run(ctx, torch_cuda, labels, ts, layout, "pair", beta)
     if rp.method == rep.method and rp.split_k == rep.split_k and rp.fetch["pair"]:
         np.testing.assert_array_equal(got, pair)
+
+
+@pytest.mark.parametrize("mn", [(150, 1900), (1900, 150)])
+@pytest.mark.parametrize("layout", ["row", "col"])
+def test_pieces_workspace_of_exchanged_operands(built_lib, torch_cuda, layout, mn):
+    """The first product of a context (no larger workspace left from an earlier
+    one), far from square: the pieces of whichever operand takes the 1M rows
+    fit the workspace."""
+    import t1m_gb300 as t1m
+    ctx = t1m.Context()
+    rng = np.random.default_rng(78)
+    ext = dict(m=mn[0], n=mn[1], k=300)
+    ts = [_tensor(rng, x, ext, np.complex64) for x in ("mk", "kn", "mn")]
+    got, rep = _run(ctx, torch_cuda, "mk,kn->mn", ts, layout, "auto", 0.25)
+    ctx.close()
+    assert rep.fetch["pieces"]
+    ref = 0.5 * ts[0].astype(np.complex128) @ ts[1].astype(np.complex128) + 0.25 * ts[2]
+    assert np.abs(got - ref).max() <= 1e-6 * np.abs(ref).max()
