@@ -1267,11 +1267,28 @@ extern "C" int t1m_contract_vjp(t1m_context* ctx, int dtype, const t1m_tensor* d
 // persistent launch, otherwise items run in dependency levels.  Optionally
 // the whole batch is captured once in a CUDA graph.  The reference has no
 // batching; its counterpart is a loop of t1m::contract calls.
+#include "pieces.h"
 #include "tc.h"
 
 namespace {
 
-enum Family : int { kFamTC = 0, kFamSimt = 1, kFamSimtSkinny = 2, kFamReduce = 3 };
+enum Family : int {
+  kFamTC = 0,
+  kFamSimt = 1,
+  kFamSimtSkinny = 2,
+  kFamReduce = 3,
+  // Tensor-core items over operand pieces: the split passes of a batch of
+  // items, one operand read along a later K mode, the batch's products.
+  kFamPieceSplit = 4,
+  kFamPieceStep = 5,
+  kFamPieces = 6
+};
+
+// Workspace of a grouped launch's operand pieces.  Items run in batches whose
+// pieces fit it, each batch split and multiplied before the next overwrites
+// them: at half the L2 (129 MB) the pieces are mostly read, and overwritten,
+// before they reach HBM.
+constexpr size_t kGroupPieceBytes = size_t(64) << 20;
 
 // Split-K inside a grouped launch: every tile covers at most kGroupKCap
 // complex (or real) K, so one long-K item (a skinny output over a big
@@ -1282,7 +1299,8 @@ constexpr int64_t kGroupKCap = 1024;
 constexpr size_t kGroupWorkBytes = size_t(2) << 30;
 constexpr size_t kGroupItemWorkBytes = size_t(256) << 20;
 
-int group_splits(int dtype, int fam, const HostPlan& hp, size_t es, int64_t* k_per_split) {
+int group_splits(int dtype, int fam, const HostPlan& hp, size_t es, int64_t* k_per_split,
+                 int64_t k_cap = kGroupKCap) {
   int bm = 0, bn = 0, bk = 0;
   if (fam == kFamTC) {
     tc_tile(dtype, &bm, &bn, &bk);
@@ -1295,7 +1313,7 @@ int group_splits(int dtype, int fam, const HostPlan& hp, size_t es, int64_t* k_p
   // plain tiles accumulate sequentially and cover at most its K limit (the
   // skinny kernel's lanes each sum a 1/32 share, the tensor-core limit is
   // above the cap).
-  int64_t cap = kGroupKCap;
+  int64_t cap = std::min(k_cap, kGroupKCap);
   if (fam == kFamSimt) {
     const int64_t lim = accuracy_k_limit(T1M_METHOD_PLAIN, dtype);
     if (lim > 0) cap = std::min(cap, lim);
@@ -1544,6 +1562,10 @@ struct t1m_group {
   void* simt_dev = nullptr;     // SimtProblem arrays, per (level, family)
   void* reduce_dev = nullptr;   // SplitReduce arrays, per level
   void* work = nullptr;         // split-K partials of all split items
+  void* pieces = nullptr;       // operand pieces of one batch of items
+  void* piece_dev = nullptr;    // PieceSplit array, then PieceProblem array
+  int64_t piece_probs = 0;      // byte offset of the PieceProblem array
+  std::vector<PieceSplit> steps;  // kFamPieceStep operands
   struct Launch {
     int family;
     int64_t offset;   // first descriptor in tc_dev / simt_dev
@@ -1586,6 +1608,17 @@ int enqueue_group(t1m_group* g, cudaStream_t s) {
           e = launch_splitk_reduce_group(g->dtype,
                                          static_cast<const SplitReduce*>(g->reduce_dev) + l.offset,
                                          l.count, l.tiles, s);
+        else if (l.family == kFamPieceSplit)
+          e = launch_piece_split(3, false, nullptr, l.count,
+                                 static_cast<const PieceSplit*>(g->piece_dev) + l.offset, l.tiles, s);
+        else if (l.family == kFamPieceStep)
+          e = launch_piece_split(3, false, &g->steps[size_t(l.offset)], 1, nullptr, l.tiles, s);
+        else if (l.family == kFamPieces)
+          e = launch_piece_products(
+              3, false, false, nullptr,
+              reinterpret_cast<const PieceProblem*>(static_cast<const char*>(g->piece_dev) +
+                                                    g->piece_probs) + l.offset,
+              l.count, l.tiles, s, ctx->d_err);
         else if (l.family == kFamSimtSkinny)
           e = launch_skinny_group(g->dtype, l.nmax,
                                   static_cast<const SimtProblem*>(g->simt_dev) + l.offset, l.count,
@@ -1620,6 +1653,8 @@ extern "C" int t1m_group_destroy(t1m_group* g) {
   if (g->reduce_dev) cudaFree(g->reduce_dev);
   if (g->work) cudaFree(g->work);
   if (g->done) cudaFree(g->done);
+  if (g->pieces) cudaFree(g->pieces);
+  if (g->piece_dev) cudaFree(g->piece_dev);
   delete g;
   return T1M_OK;
 }
@@ -1827,6 +1862,12 @@ extern "C" int t1m_group_create(t1m_context* ctx, int dtype, int n, const t1m_gr
       if (width[i] != kWidthSimt) width[i] = static_cast<int>(fw);
   }
 
+  // Tensor-core items of family launches run over operand pieces (BF16x6)
+  // where the automatic method or BF16x6 is set and workspaces are not capped.
+  const bool over_pieces = dtype == T1M_COMPLEX64 && !one_launch && ctx->opt_work_limit < 0 &&
+                           (ctx->method == T1M_METHOD_AUTO ||
+                            ctx->method == T1M_METHOD_TC_BF16X6);
+
   // Autotuning of family launches: per shape class, time the candidate
   // families once on a representative item (into a scratch output) and keep
   // the fastest.
@@ -1864,6 +1905,19 @@ extern "C" int t1m_group_create(t1m_context* ctx, int dtype, int n, const t1m_gr
         cudaFree(scratch);
         return fail(ctx, T1M_ERR_ALLOC, "autotune descriptor");
       }
+      // Pieces of the tensor-core candidate, as it is launched below: into the
+      // scratch partials, whose layout may order the operands differently.
+      void* probe_pieces = nullptr;
+      if (over_pieces) {
+        int64_t kps = 0;
+        const int sp = group_splits(dtype, kFamTC, hp, es, &kps);
+        PieceItem pi;
+        tc_piece_item(split_args(args[i], scratch, kps), hp, sp, &pi);
+        if (cudaMalloc(&probe_pieces, pi.bytes[0] + pi.bytes[1]) != cudaSuccess) {
+          cudaGetLastError();
+          probe_pieces = nullptr;
+        }
+      }
       float best = 1e30f;
       int best_f = family[i];
       for (int f : cands) {
@@ -1875,7 +1929,18 @@ extern "C" int t1m_group_create(t1m_context* ctx, int dtype, int n, const t1m_gr
         for (int rep = 0; rep < 3 && ok; ++rep) {
           cudaEventRecord(ctx->ev[4], ctx->stream);
           cudaError_t le;
-          if (f == kFamTC) {
+          if (f == kFamTC && probe_pieces) {
+            PieceItem pi;
+            tc_piece_item(probe, hp, nsp, &pi);
+            piece_item_place(&pi, probe_pieces);
+            le = cudaSuccess;
+            for (int o = 0; o < 2 && le == cudaSuccess; ++o)
+              le = launch_piece_split(3, false, &pi.op[o], 1, nullptr,
+                                      piece_split_blocks(false, pi.op[o]), ctx->stream);
+            if (le == cudaSuccess)
+              le = launch_piece_products(3, false, false, &pi.p, nullptr, 1, piece_tiles(pi.p),
+                                         ctx->stream, ctx->d_err);
+          } else if (f == kFamTC) {
             TcProblem tp;
             ok = tc_prepare(probe, hp, nsp, &tp);
             tp.tile_begin = 0;
@@ -1916,6 +1981,7 @@ extern "C" int t1m_group_create(t1m_context* ctx, int dtype, int n, const t1m_gr
       }
       cudaFree(pd);
       cudaFree(scratch);
+      if (probe_pieces) cudaFree(probe_pieces);
       if (int st = check_device_error(ctx)) return st;
       family[i] = best_f;
       g_tune.choice[key] = best_f;
@@ -1929,10 +1995,21 @@ extern "C" int t1m_group_create(t1m_context* ctx, int dtype, int n, const t1m_gr
   std::vector<int> splits(n, 1);
   std::vector<int64_t> kps(n, 0), work_off(n, -1);
   size_t work_bytes = 0;
+  // Tensor-core items over pieces of a level with few tiles (a chain's steps)
+  // split further, to occupy the 76 pairs: at K = 512, one 64 x 64 item took
+  // 72 us as one tile.  At least 64 complex k each.
+  std::vector<double> level_k(n ? *std::max_element(level.begin(), level.end()) + 1 : 1, 0.0);
+  for (int i = 0; i < n; ++i)
+    if (family[i] == kFamTC)
+      level_k[level[i]] += double((plans[i].M + 127) / 128) * double((plans[i].N + 127) / 128) *
+                           double(plans[i].K);
   for (int i = 0; i < n; ++i) {
     const HostPlan& hp = plans[i];
     if (hp.M == 0 || hp.N == 0 || hp.K == 0) continue;
-    splits[i] = group_splits(dtype, family[i], hp, es, &kps[i]);
+    const int64_t cap = over_pieces && family[i] == kFamTC
+                            ? std::max<int64_t>(64, static_cast<int64_t>(level_k[level[i]] / 76))
+                            : kGroupKCap;
+    splits[i] = group_splits(dtype, family[i], hp, es, &kps[i], cap);
     if (splits[i] > 1) {
       work_off[i] = static_cast<int64_t>(work_bytes);
       work_bytes += (size_t(splits[i]) * size_t(hp.M) * size_t(hp.N) * es + 255) & ~size_t(255);
@@ -2029,7 +2106,52 @@ extern "C" int t1m_group_create(t1m_context* ctx, int dtype, int n, const t1m_gr
     max_level = -1;  // no level launches
   }
   g->levels.assign(max_level + 1, {});
+  std::vector<PieceSplit> psplits;
+  std::vector<PieceProblem> pprobs;
+  size_t piece_work = 0;
   for (int lv = 0; lv <= max_level; ++lv) {
+    if (over_pieces) {
+      std::vector<int> ids;
+      for (int i = 0; i < n; ++i)
+        if (level[i] == lv && family[i] == kFamTC && plans[i].M > 0 && plans[i].N > 0 &&
+            plans[i].K > 0) ids.push_back(i);
+      for (size_t at = 0; at < ids.size();) {
+        t1m_group::Launch S{kFamPieceSplit, int64_t(psplits.size()), 0, 0};
+        t1m_group::Launch P{kFamPieces, int64_t(pprobs.size()), 0, 0};
+        size_t used = 0;
+        for (; at < ids.size(); ++at) {
+          PieceItem it;
+          tc_piece_item(main_args[ids[at]], plans[ids[at]], splits[ids[at]], &it);
+          const size_t need = it.bytes[0] + it.bytes[1];
+          if (used > 0 && used + need > kGroupPieceBytes) break;
+          for (int o = 0; o < 2; ++o) {
+            PieceSplit& op = it.op[o];
+            op.out = reinterpret_cast<uint8_t*>(used);  // offset until the workspace exists
+            used += it.bytes[o];
+            const int64_t blocks = piece_split_blocks(false, op);
+            if (op.mode == kSplitStep) {
+              t1m_group::Launch T{kFamPieceStep, int64_t(g->steps.size()), 1, blocks};
+              g->steps.push_back(op);
+              g->levels[lv].push_back(T);
+            } else {
+              op.block_begin = S.tiles;
+              S.tiles += blocks;
+              ++S.count;
+              psplits.push_back(op);
+            }
+          }
+          it.p.a = it.op[0].out;
+          it.p.b = it.op[1].out;
+          it.p.tile_begin = P.tiles;
+          P.tiles += piece_tiles(it.p);
+          ++P.count;
+          pprobs.push_back(it.p);
+        }
+        piece_work = std::max(piece_work, used);
+        if (S.count > 0) g->levels[lv].push_back(S);
+        g->levels[lv].push_back(P);
+      }
+    }
     for (int fam : {kFamTC, kFamSimt, kFamSimtSkinny}) {
       t1m_group::Launch L{fam, fam == kFamTC ? int64_t(tcs.size()) : int64_t(simts.size()), 0, 0};
       if (fam == kFamSimtSkinny) {
@@ -2042,6 +2164,7 @@ extern "C" int t1m_group_create(t1m_context* ctx, int dtype, int n, const t1m_gr
       for (int i = 0; i < n; ++i) {
         if (level[i] != lv || family[i] != fam) continue;
         const HostPlan& hp = plans[i];
+        if (fam == kFamTC && over_pieces && hp.M > 0 && hp.N > 0 && hp.K > 0) continue;
         if (fam == kFamTC) {
           TcProblem tp;
           if (!tc_prepare(main_args[i], hp, splits[i], &tp))
@@ -2095,6 +2218,28 @@ extern "C" int t1m_group_create(t1m_context* ctx, int dtype, int n, const t1m_gr
       e = cudaMalloc(&g->done, sizeof(int) * size_t(int64_t(tcs.size()) + g->fix_count));
     if (e == cudaSuccess)
       e = cudaMemset(g->done, 0, sizeof(int) * size_t(int64_t(tcs.size()) + g->fix_count));
+    if (e != cudaSuccess) return fail(ctx, T1M_ERR_ALLOC, "group descriptors");
+  }
+  if (!pprobs.empty()) {
+    e = cudaMalloc(&g->pieces, piece_work);
+    if (e != cudaSuccess) return fail(ctx, T1M_ERR_ALLOC, "group operand pieces");
+    uint8_t* const base = static_cast<uint8_t*>(g->pieces);
+    auto place = [&](const uint8_t* off) { return base + reinterpret_cast<size_t>(off); };
+    for (PieceSplit& x : psplits) x.out = place(x.out);
+    for (PieceSplit& x : g->steps) x.out = place(x.out);
+    for (PieceProblem& x : pprobs) {
+      x.a = place(x.a);
+      x.b = place(x.b);
+    }
+    g->piece_probs = int64_t((psplits.size() * sizeof(PieceSplit) + 15) / 16 * 16);
+    const size_t pbytes = pprobs.size() * sizeof(PieceProblem);
+    e = cudaMalloc(&g->piece_dev, size_t(g->piece_probs) + pbytes);
+    if (e == cudaSuccess && !psplits.empty())
+      e = cudaMemcpy(g->piece_dev, psplits.data(), psplits.size() * sizeof(PieceSplit),
+                     cudaMemcpyHostToDevice);
+    if (e == cudaSuccess)
+      e = cudaMemcpy(static_cast<char*>(g->piece_dev) + g->piece_probs, pprobs.data(), pbytes,
+                     cudaMemcpyHostToDevice);
     if (e != cudaSuccess) return fail(ctx, T1M_ERR_ALLOC, "group descriptors");
   }
   if (!reds.empty()) {

@@ -184,6 +184,11 @@ cudaError_t launch_simt_group(int dtype, bool skinny, const SimtProblem* dev, in
 // columns, bound by reading A once.  Rows per CTA: one warp per row (16 / nmax
 // rows per warp, 8 warps) when A has unit K stride, else one thread per row.
 constexpr int kSkinnyMaxN = 16;
+// Lanes along k: A with unit K stride, or too few rows to occupy a block's
+// threads with one row each.
+__host__ __device__ constexpr bool skinny_k_lanes(int64_t u_k, int64_t rows) {
+  return u_k == 1 || rows <= 64;
+}
 __host__ __device__ constexpr int skinny_rows(bool k_unit, int nmax) {
   return k_unit ? 8 * (16 / nmax) : 256;
 }

@@ -877,6 +877,26 @@ int piece_tile_n(bool real, int64_t M, int64_t N, int64_t K, int splits) {
   return best;
 }
 
+int piece_tile_n_batch(int64_t N) {
+  int best = 128;
+  double best_cost = 1e300;
+  for (int w = 128; w >= 32; w -= 32) {
+    const double cost = double((N + w - 1) / w) * std::max(60.0, 0.55 * w);
+    if (cost < best_cost) {
+      best_cost = cost;
+      best = w;
+    }
+  }
+  return best;
+}
+
+void piece_item_place(PieceItem* it, void* ws) {
+  it->op[0].out = static_cast<uint8_t*>(ws);
+  it->op[1].out = it->op[0].out + it->bytes[0];
+  it->p.a = it->op[0].out;
+  it->p.b = it->op[1].out;
+}
+
 void piece_set_tiles(bool real, PieceProblem* p, int tile_n, int splits) {
   const int64_t rows = real ? 256 : 128;
   p->tile_n = tile_n;

@@ -66,13 +66,27 @@ struct PieceProblem {
   int32_t pad;
 };
 
+// One product of a grouped launch (complex64, BF16x6): the product and the
+// split passes of its operands, without their workspace (piece_item_place).
+struct PieceItem {
+  PieceProblem p;
+  PieceSplit op[2];        // the product's first operand (1M rows), its second
+  size_t bytes[2];         // their pieces
+};
+void tc_piece_item(const GemmArgs& g, const HostPlan& plan, int splits, PieceItem* it);
+// Put the item's pieces at ws (bytes[0] + bytes[1] bytes).
+void piece_item_place(PieceItem* it, void* ws);
+
 // Blocks of the split pass of one operand.
 int64_t piece_split_blocks(bool real, const PieceSplit& s);
 // Split `n` operands in one launch (none of them kSplitStep when n > 1 or
 // dev is given): `ops` by value (n <= 2) or the device array `dev`.
 cudaError_t launch_piece_split(int pieces, bool real, const PieceSplit* ops, int n,
                                const PieceSplit* dev, int64_t blocks, cudaStream_t stream);
-// Tile width of a product and its tile counts (from g and splits).
+// Tile width of a product alone on the GPU, of one in a batch that fills it
+// (up to 128 columns: their epilogue overlaps the next tile), and its tile
+// counts (from g and splits).
+int piece_tile_n_batch(int64_t N);
 int piece_tile_n(bool real, int64_t M, int64_t N, int64_t K, int splits);
 void piece_set_tiles(bool real, PieceProblem* p, int tile_n, int splits);
 inline int64_t piece_tiles(const PieceProblem& p) {

@@ -251,8 +251,11 @@ cudaError_t launch_group(const SimtProblem* dev, int nprob, int64_t total_tiles,
 // their unit-stride direction:
 //   K unit stride: one warp per row (16 / NMAX rows per warp), lanes over k
 //     (256-byte coalesced reads), lane partial sums reduced across the warp;
+//   few rows (skinny_k_lanes): the same through the chunk's K offsets, staged
+//     in shared memory (one thread per row left the other threads of the
+//     block idle: a 32768-long dot product took 129 us);
 //   otherwise: one thread per row, k in order (coalesced across threads where
-//     M is unit stride), the chunk's K offsets staged in shared memory.
+//     M is unit stride).
 // Tiles are numbered split-major per problem; a split writes its partial
 // product to its workspace slice exactly like the other kernels.
 __device__ __forceinline__ float shfl_xor(float v, int m) { return __shfl_xor_sync(0xffffffffu, v, m); }
@@ -276,9 +279,12 @@ __device__ __forceinline__ void skinny_store(const GemmArgs& g, T* C, int64_t m,
     *p = add(ab, mul(scal<T>(g.beta), *p));
 }
 
-template <class T, int NMAX, bool KUNIT>
+// kKLanes: lanes over k, one warp per row; else one thread per row.
+// kKUnit (with kKLanes): A has unit K stride, else its K offsets are looked up.
+template <class T, int NMAX, bool kKLanes, bool kKUnit>
 __device__ __forceinline__ void skinny_body(const GemmArgs& g, int64_t tile, T (*Bs)[2048 / NMAX],
                                             int64_t* ks) {
+  constexpr bool KUNIT = kKLanes;
   constexpr int KB = 2048 / NMAX;            // k per shared-memory chunk
   constexpr int RW = KUNIT ? 16 / NMAX : 1;  // rows per warp (K unit) / per thread
   constexpr int BMr = skinny_rows(KUNIT, NMAX);
@@ -320,7 +326,7 @@ __device__ __forceinline__ void skinny_body(const GemmArgs& g, int64_t tile, T (
         v = conj_if(B[offs(g.rsB, g.uB_k, k0 + kk) + offs(g.csB, g.uB_n, n)], conjB);
       Bs[n][kk] = v;
     }
-    if (!KUNIT)
+    if (!kKUnit)
       for (int kk = tid; kk < kn; kk += kThreads) ks[kk] = offs(g.csA, g.uA_k, k0 + kk);
     __syncthreads();
     // kU k-steps of every row are loaded before any of them is used, so
@@ -335,7 +341,9 @@ __device__ __forceinline__ void skinny_body(const GemmArgs& g, int64_t tile, T (
 #pragma unroll
           for (int r = 0; r < RW; ++r) {
             const int kk = kk0 + 32 * u;
-            a[u][r] = (rowok[r] && kk < kn) ? conj_if(A[rowoff[r] + k0 + kk], conjA) : zero<T>();
+            a[u][r] = (rowok[r] && kk < kn)
+                          ? conj_if(A[rowoff[r] + (kKUnit ? k0 + kk : ks[kk])], conjA)
+                          : zero<T>();
           }
 #pragma unroll
         for (int u = 0; u < kU; ++u) {
@@ -546,9 +554,11 @@ skinny_contract(const SimtProblem* group, int nprob) {
     }
   }
   if (ga.uA_k == 1)
-    skinny_body<T, NMAX, true>(ga, tile, Bs, ks);
+    skinny_body<T, NMAX, true, true>(ga, tile, Bs, ks);
+  else if (skinny_k_lanes(ga.uA_k, ga.M))
+    skinny_body<T, NMAX, true, false>(ga, tile, Bs, ks);
   else
-    skinny_body<T, NMAX, false>(ga, tile, Bs, ks);
+    skinny_body<T, NMAX, false, false>(ga, tile, Bs, ks);
 }
 
 template <class T, int NMAX>
@@ -600,7 +610,7 @@ bool skinny_async_ok(const GemmArgs& g, const std::vector<int64_t>& rsA, size_t 
 }
 
 int64_t skinny_tiles(const GemmArgs& g, int splits, int nmax) {
-  const int64_t rows = skinny_rows(g.uA_k == 1, nmax);
+  const int64_t rows = skinny_rows(skinny_k_lanes(g.uA_k, g.M), nmax);
   return int64_t(splits) * ((g.M + rows - 1) / rows);
 }
 

@@ -2633,6 +2633,22 @@ static void pieces_problem(int dtype, const GemmArgs& g, const HostPlan& plan, b
   p->g.flags |= dtype == T1M_FLOAT32 ? c_store_flags_real(p->g, r, c) : c_store_flags(p->g, r, c);
 }
 
+void tc_piece_item(const GemmArgs& g, const HostPlan& plan, int splits, PieceItem* it) {
+  constexpr int dtype = T1M_COMPLEX64, P = 3;
+  *it = PieceItem{};
+  const bool swap = swap_pieces(dtype, g, plan, nullptr);
+  pieces_problem(dtype, g, plan, swap, &it->p);
+  PieceProblem& p = it->p;
+  p.rg_a = tc_pieces_groups(dtype, true, p.g.M);
+  p.rg_b = tc_pieces_groups(dtype, false, p.g.N);
+  it->op[0] = piece_split_args(dtype, !swap, swap, g, plan, nullptr, p.rg_a);
+  it->op[1] = piece_split_args(dtype, swap, swap, g, plan, nullptr, p.rg_b);
+  const int64_t kr = pieces_kreal(dtype, g.K);
+  it->bytes[0] = piece_bytes(P, pieces_rows(dtype, true, p.g.M), kr);
+  it->bytes[1] = piece_bytes(P, p.g.N, kr);
+  piece_set_tiles(false, &p, piece_tile_n_batch(p.g.N), splits);
+}
+
 // The product over pieces: the operands not in `ready` split into `ws` (one
 // launch for two uniform views, else one per operand), then the pair kernel.
 static cudaError_t launch_pieces(int method, int dtype, const GemmArgs& g, const HostPlan& plan,
