@@ -1934,9 +1934,10 @@ extern "C" int t1m_group_create(t1m_context* ctx, int dtype, int n, const t1m_gr
             tc_piece_item(probe, hp, nsp, &pi);
             piece_item_place(&pi, probe_pieces);
             le = cudaSuccess;
-            for (int o = 0; o < 2 && le == cudaSuccess; ++o)
-              le = launch_piece_split(3, false, &pi.op[o], 1, nullptr,
-                                      piece_split_blocks(false, pi.op[o]), ctx->stream);
+            for (int o = 0; o < 2 && le == cudaSuccess; ++o) {
+              const int64_t blocks = piece_split_blocks(false, pi.op[o]);
+              le = launch_piece_split(3, false, &pi.op[o], 1, nullptr, blocks, ctx->stream);
+            }
             if (le == cudaSuccess)
               le = launch_piece_products(3, false, false, &pi.p, nullptr, 1, piece_tiles(pi.p),
                                          ctx->stream, ctx->d_err);
@@ -1954,7 +1955,7 @@ extern "C" int t1m_group_create(t1m_context* ctx, int dtype, int n, const t1m_gr
             if (skinny_async_ok(sp.g, hp.rsA, es, nmax)) sp.g.flags |= kFlagSkinnyAsync;
             cudaMemcpy(pd, &sp, sizeof(sp), cudaMemcpyHostToDevice);
             le = launch_skinny_group(dtype, nmax, static_cast<SimtProblem*>(pd), 1,
-                                     skinny_tiles(probe, nsp, nmax), ctx->stream);
+                                     skinny_tiles(sp.g, nsp, nmax), ctx->stream);
           } else {
             SimtProblem sp{probe, 0};
             cudaMemcpy(pd, &sp, sizeof(sp), cudaMemcpyHostToDevice);
@@ -1995,20 +1996,25 @@ extern "C" int t1m_group_create(t1m_context* ctx, int dtype, int n, const t1m_gr
   std::vector<int> splits(n, 1);
   std::vector<int64_t> kps(n, 0), work_off(n, -1);
   size_t work_bytes = 0;
-  // Tensor-core items over pieces of a level with few tiles (a chain's steps)
-  // split further, to occupy the 76 pairs: at K = 512, one 64 x 64 item took
-  // 72 us as one tile.  At least 64 complex k each.
-  std::vector<double> level_k(n ? *std::max_element(level.begin(), level.end()) + 1 : 1, 0.0);
-  for (int i = 0; i < n; ++i)
+  // Items of a level with few tiles (a chain's steps) split further, to
+  // occupy the 76 pairs (over pieces, at least 64 complex k each) or the SMs
+  // (skinny, at least 128): as one tile, a 64 x 64 x 512 step took 72 us.
+  std::vector<double> level_tc(n ? *std::max_element(level.begin(), level.end()) + 1 : 1, 0.0);
+  std::vector<double> level_skinny(level_tc.size(), 0.0);
+  for (int i = 0; i < n; ++i) {
+    const HostPlan& hp = plans[i];
     if (family[i] == kFamTC)
-      level_k[level[i]] += double((plans[i].M + 127) / 128) * double((plans[i].N + 127) / 128) *
-                           double(plans[i].K);
+      level_tc[level[i]] += double((hp.M + 127) / 128) * double((hp.N + 127) / 128) * double(hp.K);
+    if (family[i] == kFamSimtSkinny) level_skinny[level[i]] += double((hp.M + 31) / 32) * double(hp.K);
+  }
   for (int i = 0; i < n; ++i) {
     const HostPlan& hp = plans[i];
     if (hp.M == 0 || hp.N == 0 || hp.K == 0) continue;
-    const int64_t cap = over_pieces && family[i] == kFamTC
-                            ? std::max<int64_t>(64, static_cast<int64_t>(level_k[level[i]] / 76))
-                            : kGroupKCap;
+    int64_t cap = kGroupKCap;
+    if (over_pieces && family[i] == kFamTC)
+      cap = std::max<int64_t>(64, static_cast<int64_t>(level_tc[level[i]] / 76));
+    else if (family[i] == kFamSimtSkinny)
+      cap = std::max<int64_t>(128, static_cast<int64_t>(level_skinny[level[i]] / ctx->num_sms));
     splits[i] = group_splits(dtype, family[i], hp, es, &kps[i], cap);
     if (splits[i] > 1) {
       work_off[i] = static_cast<int64_t>(work_bytes);
@@ -2182,7 +2188,7 @@ extern "C" int t1m_group_create(t1m_context* ctx, int dtype, int n, const t1m_gr
         } else if (fam == kFamSimtSkinny) {
           SimtProblem sp{main_args[i], L.tiles};
           if (skinny_async_ok(sp.g, hp.rsA, es, L.nmax)) sp.g.flags |= kFlagSkinnyAsync;
-          L.tiles += skinny_tiles(main_args[i], splits[i], L.nmax);
+          L.tiles += skinny_tiles(sp.g, splits[i], L.nmax);
           simts.push_back(sp);
         } else {
           int bm, bn;

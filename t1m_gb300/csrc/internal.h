@@ -195,6 +195,9 @@ __host__ __device__ constexpr int skinny_rows(bool k_unit, int nmax) {
 // kFlagSkinnyAsync for an item of a skinny launch of column bound nmax
 // (rs: the plan's A row offsets; uniform stride uA_m where >= 0).
 bool skinny_async_ok(const GemmArgs& g, const std::vector<int64_t>& rsA, size_t elem, int nmax);
+// Rows per block of the asynchronous form: several 32-row tiles share one
+// staged B chunk where there are enough of them.
+__host__ __device__ constexpr int skinny_async_rows(int64_t rows) { return rows >= 256 ? 128 : 32; }
 // Tiles of one skinny problem: splits x ceil(M / rows).
 int64_t skinny_tiles(const GemmArgs& g, int splits, int nmax);
 cudaError_t launch_skinny_group(int dtype, int nmax, const SimtProblem* dev, int nprob,

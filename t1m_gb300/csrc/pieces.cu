@@ -79,19 +79,21 @@ __device__ __forceinline__ void split_row_chunk(const PieceSplit& o, int64_t ks,
     if (!o.expand) {
       put_chunk<P>(o.out, chunk_at<P>(o.rg, ks, r, c), stride, v);
     } else {
-      float x[8];
+      // The second 1M row's pairs [im, re] are the first's [re, -im] with the
+      // halves exchanged and -im negated: the split is symmetric in the sign.
+      uint32_t w[3][4];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        x[2 * j] = v[2 * j];
-        x[2 * j + 1] = -v[2 * j + 1];
-      }
-      put_chunk<P>(o.out, chunk_at<P>(o.rg, ks, 2 * r, c), stride, x);
+      for (int j = 0; j < 4; ++j)
+        split_bf16<P>(v[2 * j], -v[2 * j + 1], w[0][j], w[1][j], w[2][j]);
+      uint8_t* const at = o.out + chunk_at<P>(o.rg, ks, 2 * r, c);
+      uint8_t* const at1 = o.out + chunk_at<P>(o.rg, ks, 2 * r + 1, c);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        x[2 * j] = v[2 * j + 1];
-        x[2 * j + 1] = v[2 * j];
+      for (int p = 0; p < P; ++p) {
+        *reinterpret_cast<uint4*>(at + p * stride) = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) w[p][j] = __byte_perm(w[p][j], 0u, 0x1032) ^ 0x8000u;
+        *reinterpret_cast<uint4*>(at1 + p * stride) = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
       }
-      put_chunk<P>(o.out, chunk_at<P>(o.rg, ks, 2 * r + 1, c), stride, x);
     }
   }
 }
@@ -112,19 +114,17 @@ split_pieces(const SplitPair pair, const PieceSplit* dev, int n) {
   __shared__ T tile[kSplitRowsPer][KB + 1];
   __shared__ PieceSplit so;
   if (dev) {
-    int lo = 0, hi = n - 1;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (dev[mid].block_begin <= blockIdx.x) lo = mid; else hi = mid - 1;
-    }
-    if (threadIdx.x == 0) so = dev[lo];
+    const int lo = block_find(n, blockIdx.x, [&](int i) { return dev[i].block_begin; });
+    block_copy(&so, dev + lo);
     __syncthreads();
   }
   const PieceSplit& o =
       dev ? so : (pair.n > 1 && blockIdx.x >= pair.op[1].block_begin ? pair.op[1] : pair.op[0]);
-  const int64_t bid = blockIdx.x - o.block_begin;
-  const int64_t kblocks = (o.K + KB - 1) / KB;
-  const int64_t r0 = (bid / kblocks) * kSplitRowsPer, k0 = (bid % kblocks) * KB;
+  // Block counts of a launch fit 32 bits (launch_piece_split).
+  const int bid = static_cast<int>(blockIdx.x - o.block_begin);
+  const int kblocks = static_cast<int>((o.K + KB - 1) / KB);
+  const int rb = bid / kblocks;
+  const int64_t r0 = int64_t(rb) * kSplitRowsPer, k0 = int64_t(bid - rb * kblocks) * KB;
   const T* __restrict__ src = static_cast<const T*>(o.src);
   const int t = threadIdx.x;
   constexpr int kPer = kSplitRowsPer * KB / 256;
@@ -229,14 +229,36 @@ split_pieces_step(const PieceSplit o) {
 
 // ---------------------------------------------------------------- product ---
 
-constexpr int kPcThreads = 640;        // warp 0 MMA, 1 loads, 2 relay, 4-19 epilogue
+constexpr int kPcThreads = 640;        // warp 0 MMA, 1 loads, 2 relay, 3 tiles, 4-19 epilogue
 constexpr int kPcEpiBase = 128;
 constexpr int kPcEpiWarps = 16;
 constexpr uint32_t kPcTmemCols = 512;
-constexpr int kPcBarriers = 256;
+constexpr int kPcBarriers = 512;
 constexpr int kPcARows = 128;          // real rows of A per CTA
 constexpr int kPcABytes = kPcARows * 64;
 constexpr int kPcFold = 8;             // stages per main chunk: 16 MMAs of K = 16
+
+// One tile as the roles of a CTA see it, written to shared memory by the
+// scheduling warp up to kPcWorks tiles ahead: finding a tile's problem and
+// its fields takes about 1000 clocks of dependent loads and divisions, which
+// each role used to pay per tile (K = 128: 12.9k clocks a tile for 6.9k of
+// MMAs).
+constexpr int kPcWorks = 4;
+struct PcWork {
+  const uint8_t* a;     // this CTA's rows and columns in the first stage, piece 0
+  const uint8_t* b;
+  int64_t pa, pb;       // bytes from piece to piece
+  void* C;              // of the tile's split
+  const int64_t *rsC, *csC;
+  int64_t uC_m, uC_n;
+  int64_t row0, M, n0, N;
+  float alpha[2], beta[2];
+  uint32_t flags;
+  uint32_t abytes, bbytes;  // per piece and stage (row groups that exist)
+  int32_t steps;        // K = 16 MMA steps; 0: no more tiles
+  int32_t tn;
+  int32_t swapped;
+};
 
 // kWide: tiles of 160 to 256 columns, one chunk and one correction
 // accumulator of 256 columns; otherwise up to 128 columns and two of each.
@@ -248,26 +270,24 @@ struct PcShape {
   static constexpr int kBBytes = kMaxN / 2 * 64;            // one piece of this CTA's columns
   static constexpr int kStage = P * (kPcABytes + kBBytes);  // 48 / 36 KB for three pieces
   static constexpr int kStages = kWide ? (P == 3 ? 4 : 6) : (P == 3 ? 6 : 8);
-  static constexpr int kSmem = 1024 + kStages * kStage + kPcBarriers;
+  static constexpr int kUnits = kMaxN / 16 / (kPcEpiWarps / 4);  // 16-column units per thread
+  static constexpr int kCols = 16 * kUnits;                      // columns per warpgroup
+  static constexpr int kSmem = 1024 + kStages * kStage + kPcBarriers +
+                               kPcWorks * static_cast<int>(sizeof(PcWork)) +
+                               kPcEpiWarps * kCols * 8;
   static_assert(kSmem <= 227 * 1024, "shared memory budget");
-  static_assert(8 * (2 * kStages + 4 * kBufs + 2) <= kPcBarriers, "barrier area");
+  static_assert(8 * (2 * kStages + 4 * kBufs + 2 * kPcWorks + 2) <= kPcBarriers, "barrier area");
   __device__ static constexpr uint32_t chunk_col(int b) { return 128u * b; }
   __device__ static constexpr uint32_t corr_col(int b) { return 256u + 128u * b; }
 };
 
-struct PcTile {
-  const PieceProblem* p;
-  int64_t tm, n0, kb, steps;  // steps: K = 16 MMA steps of this tile
-  int64_t split;
-  int tn;
-};
-
-// Tiles of a problem are numbered split-major; within a split, groups of 8
-// pair tiles along M sweep N, so pairs running together share both operands
-// in L2.
-template <bool kReal>
-__device__ __forceinline__ PcTile pc_locate(const PieceProblem* single, const PieceProblem* group,
-                                            int nprob, int64_t t, int& hint) {
+// Tile t of the launch for CTA `rank` of its pair.  Tiles of a problem are
+// numbered split-major; within a split, groups of 8 pair tiles along M sweep
+// N, so pairs running together share both operands in L2.
+template <int P, bool kReal>
+__device__ __forceinline__ void pc_fill(PcWork& w, const PieceProblem* single,
+                                        const PieceProblem* group, int nprob, int64_t t,
+                                        uint32_t rank, int& hint) {
   const PieceProblem* p = single;
   if (group) {
     int lo = hint;
@@ -275,9 +295,10 @@ __device__ __forceinline__ PcTile pc_locate(const PieceProblem* single, const Pi
     hint = lo;
     p = group + lo;
   }
+  const GemmArgs& g = p->g;
   // Tile counts of a launch fit 32 bits (launch_piece_products).
   const int lt = static_cast<int>(t - p->tile_begin);
-  const int tiles_m = p->tiles_m, tiles_n = p->tiles_n;
+  const int tiles_m = p->tiles_m, tiles_n = p->tiles_n, tn = p->tile_n;
   const int per_split = tiles_m * tiles_n;
   const int split = p->splits > 1 ? lt / per_split : 0, r = lt - split * per_split;
   constexpr int G = 8;
@@ -285,18 +306,40 @@ __device__ __forceinline__ PcTile pc_locate(const PieceProblem* single, const Pi
   const int first_m = grp * G;
   const int gsize = min(G, tiles_m - first_m);
   const int col = in / gsize;
-  PcTile x;
-  x.p = p;
-  x.split = split;
-  x.tm = first_m + in - col * gsize;
-  x.tn = p->tile_n;
-  x.n0 = int64_t(col) * x.tn;
+  const int64_t tm = first_m + in - col * gsize;
+  const int64_t n0 = int64_t(col) * tn;
   constexpr int64_t f = kReal ? 1 : 2;
-  const int64_t kb = int64_t(split) * p->g.k_per_split;
-  const int64_t ke = min(p->g.K, kb + p->g.k_per_split);
-  x.kb = f * kb;
-  x.steps = (f * (ke - kb) + 15) / 16;
-  return x;
+  const int64_t kb = int64_t(split) * g.k_per_split;
+  const int64_t ke = min(g.K, kb + g.k_per_split);
+  const int64_t ks0 = f * kb / kPieceStageK;
+  // Row groups of this CTA's rows and columns that exist (the rest of a
+  // stage keeps old bytes: rows and columns nobody writes to C).
+  const int64_t ga = (2 * tm + rank) * (kPcARows / 8), gb = (n0 + rank * (tn / 2)) / 8;
+  const int64_t na = min(int64_t(kPcARows / 8), p->rg_a - ga);
+  const int64_t nb = min(int64_t(tn / 16), p->rg_b - gb);
+  w.a = p->a + (ks0 * P * p->rg_a + ga) * kPieceAtom;
+  w.b = p->b + (ks0 * P * p->rg_b + gb) * kPieceAtom;
+  w.pa = p->rg_a * kPieceAtom;
+  w.pb = p->rg_b * kPieceAtom;
+  w.abytes = na > 0 ? static_cast<uint32_t>(na) * kPieceAtom : 0u;
+  w.bbytes = nb > 0 ? static_cast<uint32_t>(nb) * kPieceAtom : 0u;
+  w.C = static_cast<uint8_t*>(g.C) + split * g.c_split_stride * (kReal ? 4 : 8);
+  w.rsC = g.rsC;
+  w.csC = g.csC;
+  w.uC_m = g.uC_m;
+  w.uC_n = g.uC_n;
+  w.row0 = (2 * tm + rank) * (kReal ? kPcARows : kPcARows / 2);
+  w.M = g.M;
+  w.n0 = n0;
+  w.N = g.N;
+  w.alpha[0] = static_cast<float>(g.alpha[0]);
+  w.alpha[1] = static_cast<float>(g.alpha[1]);
+  w.beta[0] = static_cast<float>(g.beta[0]);
+  w.beta[1] = static_cast<float>(g.beta[1]);
+  w.flags = g.flags;
+  w.steps = static_cast<int>((f * (ke - kb) + 15) / 16);
+  w.tn = tn;
+  w.swapped = p->swapped;
 }
 
 // C <- alpha * acc (+ beta * C, or + C when accumulating) for the 16 columns
@@ -304,14 +347,15 @@ __device__ __forceinline__ PcTile pc_locate(const PieceProblem* single, const Pi
 // 0) and imaginary row.  As store_tile, but old values are read together
 // before any is written, so accumulating products wait once per group
 // instead of once per access.
-__device__ __forceinline__ void pc_store16(const GemmArgs& g, float2* __restrict__ Cr, bool row_ok,
-                                           int64_t n0, int part, const float* acc) {
-  const uint32_t flags = g.flags;
+// `cols`: the 16 columns' offsets, in shared memory.
+__device__ __forceinline__ void pc_store16(const PcWork& w, const int64_t* cols,
+                                           float2* __restrict__ Cr, bool row_ok, int64_t n0,
+                                           int part, const float* acc) {
+  const uint32_t flags = w.flags;
   const bool accumulate = flags & kFlagAccumulate, read = accumulate || !(flags & kFlagBetaZero);
   const bool col16 = flags & kFlagCCol16;
-  const float ar = (float)g.alpha[0], ai = (float)g.alpha[1];
-  const float br = (float)g.beta[0], bi = (float)g.beta[1];
-  const int64_t N = g.N;
+  const float ar = w.alpha[0], ai = w.alpha[1], br = w.beta[0], bi = w.beta[1];
+  const int64_t N = w.N;
   if (n0 >= N) return;  // uniform over the warp
   float2 v[8];
 #pragma unroll
@@ -332,7 +376,7 @@ __device__ __forceinline__ void pc_store16(const GemmArgs& g, float2* __restrict
   };
   // Value 2 q + e belongs to column n0 + 4 q + 2 part + e.
   if ((flags & kFlagCPairs) && col16 && n0 + 16 <= N) {
-    float4* p = reinterpret_cast<float4*>(Cr + offs(g.csC, g.uC_n, n0) + 2 * part);
+    float4* p = reinterpret_cast<float4*>(Cr + cols[0] + 2 * part);
     if (read) {
       float4 o[4];
 #pragma unroll
@@ -353,9 +397,9 @@ __device__ __forceinline__ void pc_store16(const GemmArgs& g, float2* __restrict
       bool in[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const int64_t n = n0 + 8 * h + 4 * (i >> 1) + 2 * part + (i & 1);
-        in[i] = n < N;
-        p[i] = Cr + (in[i] ? offs(g.csC, g.uC_n, n) : 0);
+        const int c = 8 * h + 4 * (i >> 1) + 2 * part + (i & 1);
+        in[i] = n0 + c < N;
+        p[i] = Cr + cols[c];
       }
       if (read) {
         float2 o[4];
@@ -372,16 +416,17 @@ __device__ __forceinline__ void pc_store16(const GemmArgs& g, float2* __restrict
 }
 
 // The real form: columns [n0, n0 + 16) of one real row per lane.
-__device__ __forceinline__ void pc_store16_real(const GemmArgs& g, float* __restrict__ Cr,
-                                                int64_t n0, const float* acc) {
-  const uint32_t flags = g.flags;
+__device__ __forceinline__ void pc_store16_real(const PcWork& w, const int64_t* cols,
+                                                float* __restrict__ Cr, int64_t n0,
+                                                const float* acc) {
+  const uint32_t flags = w.flags;
   const bool accumulate = flags & kFlagAccumulate, read = accumulate || !(flags & kFlagBetaZero);
-  const float ar = (float)g.alpha[0], br = (float)g.beta[0];
-  const int64_t N = g.N;
+  const float ar = w.alpha[0], br = w.beta[0];
+  const int64_t N = w.N;
   if (n0 >= N) return;
   auto combine = [&](float t, float o) { return accumulate ? o + t : t + br * o; };
   if ((flags & kFlagCPairs) && (flags & kFlagCCol16) && n0 + 16 <= N) {
-    float4* p = reinterpret_cast<float4*>(Cr + offs(g.csC, g.uC_n, n0));
+    float4* p = reinterpret_cast<float4*>(Cr + cols[0]);
     float4 o[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) o[q] = read ? p[q] : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -401,9 +446,8 @@ __device__ __forceinline__ void pc_store16_real(const GemmArgs& g, float* __rest
       bool in[8];
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        const int64_t n = n0 + 8 * h + i;
-        in[i] = n < N;
-        p[i] = Cr + (in[i] ? offs(g.csC, g.uC_n, n) : 0);
+        in[i] = n0 + 8 * h + i < N;
+        p[i] = Cr + cols[8 * h + i];
       }
       float o[8];
 #pragma unroll
@@ -421,8 +465,8 @@ __device__ __forceinline__ void pc_store16_real(const GemmArgs& g, float* __rest
 // SMs.  Warp 0 (even CTA, one lane) issues every MMA; warp 1 (one lane per
 // CTA) loads the CTA's 128 rows of A and half of the tile's columns of B;
 // warp 2 (odd CTA, one lane) relays the arrival of its stage to the MMA
-// thread; warps 4-19 fold chunks and write C (one TMEM lane per thread, the
-// four warpgroups taking the tile's 16-column units in turn).
+// thread; warp 3 (one lane per CTA) finds the tiles; warps 4-19 fold chunks and write C (one TMEM lane per thread, the
+// four warpgroups each a quarter of the columns).
 //
 // Overlap.  Loads run ahead over tile borders.  With tiles of up to 128
 // columns both chunk and correction accumulators are doubled, so a tile's
@@ -442,7 +486,7 @@ tc1m_pieces(const __grid_constant__ PieceProblem single, const PieceProblem* gro
             int64_t total_tiles, int* err_flag) {
   using Sh = PcShape<P, kWide>;
   constexpr int S = Sh::kStages, kBufs = Sh::kBufs;
-  constexpr int kUnits = Sh::kMaxN / 16 / (kPcEpiWarps / 4);  // 16-column units per thread
+  constexpr int kUnits = Sh::kUnits, kCols = Sh::kCols;
 
   extern __shared__ __align__(16) uint8_t smem_raw[];
   const uint32_t base = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -454,10 +498,14 @@ tc1m_pieces(const __grid_constant__ PieceProblem single, const PieceProblem* gro
   auto chunk_empty = [&](int b) { return bars + 8u * (2 * S + kBufs + b); };
   auto corr_full = [&](int b) { return bars + 8u * (2 * S + 2 * kBufs + b); };
   auto corr_empty = [&](int b) { return bars + 8u * (2 * S + 3 * kBufs + b); };
-  const uint32_t end_bar = bars + 8u * (2 * S + 4 * kBufs);
+  auto work_full = [&](int e) { return bars + 8u * (2 * S + 4 * kBufs + e); };
+  auto work_empty = [&](int e) { return bars + 8u * (2 * S + 4 * kBufs + kPcWorks + e); };
+  const uint32_t end_bar = bars + 8u * (2 * S + 4 * kBufs + 2 * kPcWorks);
   const uint32_t tmem_slot = end_bar + 8u;
   volatile uint32_t* tmem_slot_ptr =
       reinterpret_cast<volatile uint32_t*>(base_ptr + (tmem_slot - base));
+  PcWork* const works = reinterpret_cast<PcWork*>(base_ptr + S * Sh::kStage + kPcBarriers);
+  int64_t* const col_offsets = reinterpret_cast<int64_t*>(works + kPcWorks);
 
   const int tid = threadIdx.x;
   // Broadcast from lane 0, so the compiler knows the roles are warp-uniform.
@@ -480,6 +528,12 @@ tc1m_pieces(const __grid_constant__ PieceProblem single, const PieceProblem* gro
       ptx::mbar_init(corr_full(b), 1);
       ptx::mbar_init(corr_empty(b), 2 * kPcEpiWarps);
     }
+    // Readers of a tile: loads, epilogue warps, and the MMA warp (even CTA) or
+    // the relay (odd CTA).
+    for (int e = 0; e < kPcWorks; ++e) {
+      ptx::mbar_init(work_full(e), 1);
+      ptx::mbar_init(work_empty(e), 2 + kPcEpiWarps);
+    }
     ptx::mbar_init(end_bar, 1);
     ptx::fence_mbar_init();
   }
@@ -491,8 +545,50 @@ tc1m_pieces(const __grid_constant__ PieceProblem single, const PieceProblem* gro
   // Everything above may overlap the end of the split pass; the descriptors,
   // pieces and C below may have been written by earlier kernels.
   ptx::grid_dependency_wait();
-  const int64_t first = blockIdx.x >> 1, stride = gridDim.x >> 1;
-  if (warp == 0) {
+  // The next tile of this role: its entry, or null when there are no more
+  // (or a wait ran out, which is recorded).
+  struct Cursor {
+    int e = 0;
+    uint32_t phase = 0;
+  };
+  auto take = [&](const Cursor& c) -> const PcWork* {
+    if (!ptx::mbar_wait(work_full(c.e), c.phase)) {
+      record_error(err_flag, kErrWorkWait);
+      return nullptr;
+    }
+    const PcWork* w = works + c.e;
+    return w->steps > 0 ? w : nullptr;
+  };
+  // Hand the entry back (one arrival per role) and go on to the next.
+  auto advance = [&](Cursor& c) {
+    if (++c.e == kPcWorks) {
+      c.e = 0;
+      c.phase ^= 1u;
+    }
+  };
+  if (warp == 3) {
+    // --------------------------------------------------------- scheduling ---
+    if (lane == 0) {
+      const int64_t first = blockIdx.x >> 1, stride = gridDim.x >> 1;
+      int hint = 0;
+      Cursor c;
+      for (int64_t t = first;; t += stride) {
+        if (!ptx::mbar_wait(work_empty(c.e), c.phase ^ 1u)) {
+          record_error(err_flag, kErrWorkWait);
+          break;
+        }
+        PcWork& w = works[c.e];
+        if (t < total_tiles)
+          pc_fill<P, kReal>(w, &single, group, nprob, t, rank, hint);
+        else
+          w.steps = 0;
+        ptx::mbar_arrive(work_full(c.e));
+        advance(c);
+        if (t >= total_tiles) break;
+      }
+    }
+    __syncwarp();
+  } else if (warp == 0) {
     // ---------------------------------------------------------- MMA issue ---
     // The whole warp runs this loop and one elected lane issues: with
     // warp-uniform control flow the descriptors stay in uniform registers.
@@ -502,16 +598,9 @@ tc1m_pieces(const __grid_constant__ PieceProblem single, const PieceProblem* gro
     if (rank == 0) {
       const uint64_t desc0 = ptx::smem_desc_sw64(base);
       const bool issue = ptx::elect_one();
-      int slot = 0, tile_cnt = 0, chunk = 0, hint = 0;
+      int slot = 0, tile_cnt = 0, chunk = 0;
       uint32_t phase = 0;
       bool ok = true;
-      int x_tn = 0, x_steps = 0, x_swap = 0;
-      auto look = [&](int64_t t) {
-        const PcTile x = pc_locate<kReal>(&single, group, nprob, t, hint);
-        x_tn = __shfl_sync(0xffffffffu, x.tn, 0);
-        x_steps = __shfl_sync(0xffffffffu, static_cast<int>(x.steps), 0);
-        x_swap = __shfl_sync(0xffffffffu, x.p->swapped, 0);
-      };
       // Products of one ring slot.  Piece p, K = 16 step kk: A at +p x 8 KB,
       // B after the A pieces, +32 bytes per step inside the 64-byte rows.
       auto mains = [&](int st, int nkk, uint32_t d, uint32_t idesc, bool first_of_chunk) {
@@ -550,11 +639,16 @@ tc1m_pieces(const __grid_constant__ PieceProblem single, const PieceProblem* gro
           ptx::mma_commit2(empty_bar(st));
         }
       };
-      if (first < total_tiles) look(first);
-      for (int64_t t = first; t < total_tiles && ok; t += stride) {
-        const int steps = x_steps;
-        const bool swapped = x_swap != 0;
-        const uint32_t idesc = ptx::idesc_f32acc(1u /*BF16*/, 256u, static_cast<uint32_t>(x_tn));
+      Cursor cur;
+      while (ok) {
+        const PcWork* w = take(cur);
+        if (!w) break;
+        const int steps = __shfl_sync(0xffffffffu, w->steps, 0);
+        const int tn = __shfl_sync(0xffffffffu, w->tn, 0);
+        const bool swapped = __shfl_sync(0xffffffffu, w->swapped, 0) != 0;
+        if (issue) ptx::mbar_arrive(work_empty(cur.e));
+        advance(cur);
+        const uint32_t idesc = ptx::idesc_f32acc(1u /*BF16*/, 256u, static_cast<uint32_t>(tn));
         const int ns = (steps + 1) / 2;
         const int cb = tile_cnt % kBufs;
         const uint32_t d_corr = tmem + Sh::corr_col(cb);
@@ -601,8 +695,6 @@ tc1m_pieces(const __grid_constant__ PieceProblem single, const PieceProblem* gro
           }
           corrections(slot, nkk, d_corr, idesc, s == 0, swapped);
           if (two) corrections(slot2, nkk2, d_corr, idesc, false, swapped);
-          // The next tile is looked up while this tile's MMAs run.
-          if (s == 0 && t + stride < total_tiles) look(t + stride);
           slot = two ? slot2 : slot;
           phase = two ? phase2 : phase;
           s += two ? 2 : 1;
@@ -623,40 +715,38 @@ tc1m_pieces(const __grid_constant__ PieceProblem single, const PieceProblem* gro
   } else if (warp == 1) {
     // -------------------------------------------------------------- loads ---
     if (lane == 0) {
-      int64_t it = 0;
-      int hint = 0;
+      int slot = 0;
+      uint32_t phase = 0;
+      Cursor cur;
       bool ok = true;
-      for (int64_t t = first; t < total_tiles && ok; t += stride) {
-        const PcTile x = pc_locate<kReal>(&single, group, nprob, t, hint);
-        const PieceProblem* p = x.p;
-        // Row groups of this CTA's rows and columns that exist (the rest of
-        // the stage keeps old bytes: rows and columns nobody writes to C).
-        const int64_t ga = (2 * x.tm + rank) * (kPcARows / 8);
-        const int64_t gb = (x.n0 + rank * (x.tn / 2)) / 8;
-        const int64_t na = min(int64_t(kPcARows / 8), p->rg_a - ga);
-        const int64_t nb = min(int64_t(x.tn / 16), p->rg_b - gb);
-        const uint32_t abytes = na > 0 ? static_cast<uint32_t>(na) * kPieceAtom : 0u;
-        const uint32_t bbytes = nb > 0 ? static_cast<uint32_t>(nb) * kPieceAtom : 0u;
-        const int64_t ks0 = x.kb / kPieceStageK, ns = (x.steps + 1) / 2;
-        const uint8_t* a = p->a + (ks0 * P * p->rg_a + ga) * kPieceAtom;
-        const uint8_t* b = p->b + (ks0 * P * p->rg_b + gb) * kPieceAtom;
-        const int64_t pa = p->rg_a * kPieceAtom, pb = p->rg_b * kPieceAtom;
-        for (int64_t s = 0; s < ns; ++s, ++it) {
-          const int st = static_cast<int>(it % S);
-          if (!ptx::mbar_wait(empty_bar(st), static_cast<uint32_t>((it / S) & 1) ^ 1u)) {
+      while (ok) {
+        const PcWork* w = take(cur);
+        if (!w) break;
+        const uint8_t *a = w->a, *b = w->b;
+        const int64_t pa = w->pa, pb = w->pb;
+        const uint32_t abytes = w->abytes, bbytes = w->bbytes;
+        const int ns = (w->steps + 1) / 2;
+        ptx::mbar_arrive(work_empty(cur.e));
+        advance(cur);
+        for (int s = 0; s < ns; ++s) {
+          if (!ptx::mbar_wait(empty_bar(slot), phase ^ 1u)) {
             record_error(err_flag, kErrRawWait);
             ok = false;
             break;
           }
-          const uint32_t dst = base + st * Sh::kStage;
-          ptx::mbar_arrive_expect_tx(full_bar(st), P * (abytes + bbytes));
+          const uint32_t dst = base + slot * Sh::kStage;
+          ptx::mbar_arrive_expect_tx(full_bar(slot), P * (abytes + bbytes));
 #pragma unroll
           for (int q = 0; q < P; ++q) {
-            if (abytes) ptx::bulk_load(dst + q * kPcABytes, a, abytes, full_bar(st));
+            if (abytes) ptx::bulk_load(dst + q * kPcABytes, a, abytes, full_bar(slot));
             if (bbytes)
-              ptx::bulk_load(dst + P * kPcABytes + q * Sh::kBBytes, b, bbytes, full_bar(st));
+              ptx::bulk_load(dst + P * kPcABytes + q * Sh::kBBytes, b, bbytes, full_bar(slot));
             a += pa;
             b += pb;
+          }
+          if (++slot == S) {
+            slot = 0;
+            phase ^= 1u;
           }
         }
       }
@@ -665,20 +755,27 @@ tc1m_pieces(const __grid_constant__ PieceProblem single, const PieceProblem* gro
   } else if (warp == 2) {
     // -------------------------------------------------------------- relay ---
     if (lane == 0 && rank == 1) {
-      int64_t it = 0;
-      int hint = 0;
+      int slot = 0;
+      uint32_t phase = 0;
+      Cursor cur;
       bool ok = true;
-      for (int64_t t = first; t < total_tiles && ok; t += stride) {
-        const PcTile x = pc_locate<kReal>(&single, group, nprob, t, hint);
-        const int64_t ns = (x.steps + 1) / 2;
-        for (int64_t s = 0; s < ns; ++s, ++it) {
-          const int st = static_cast<int>(it % S);
-          if (!ptx::mbar_wait(full_bar(st), static_cast<uint32_t>((it / S) & 1))) {
+      while (ok) {
+        const PcWork* w = take(cur);
+        if (!w) break;
+        const int ns = (w->steps + 1) / 2;
+        ptx::mbar_arrive(work_empty(cur.e));
+        advance(cur);
+        for (int s = 0; s < ns; ++s) {
+          if (!ptx::mbar_wait(full_bar(slot), phase)) {
             record_error(err_flag, kErrFullWait);
             ok = false;
             break;
           }
-          ptx::mbar_arrive_cluster(ptx::mapa(full_bar(st), 0));
+          ptx::mbar_arrive_cluster(ptx::mapa(full_bar(slot), 0));
+          if (++slot == S) {
+            slot = 0;
+            phase ^= 1u;
+          }
         }
       }
     }
@@ -690,20 +787,36 @@ tc1m_pieces(const __grid_constant__ PieceProblem single, const PieceProblem* gro
     const int q = (pt >> 5) & 3;
     const int rho = 32 * q + lane;  // real row of this CTA's 128 = TMEM lane
     const uint32_t lane_base = static_cast<uint32_t>(32 * q) << 16;
-    int64_t chunk = 0, tile_cnt = 0;
-    int hint = 0;
-    for (int64_t t = first; t < total_tiles; t += stride, ++tile_cnt) {
-      const PcTile x = pc_locate<kReal>(&single, group, nprob, t, hint);
+    int64_t* const cols = col_offsets + (warp - 4) * kCols;
+    int chunk = 0, tile_cnt = 0;
+    Cursor cur;
+    while (true) {
+      const PcWork* w = take(cur);
+      if (!w) break;
+      const int tn = w->tn;
+      // C's offsets of this lane's row and of the warpgroup's columns, while
+      // the tile's products run.
+      const int64_t row = w->row0 + (kReal ? rho : rho >> 1);
+      const bool row_ok = row < w->M;
+      const int64_t row_off = row_ok ? offs(w->rsC, w->uC_m, row) : 0;
+#pragma unroll
+      for (int j = 0; j < kCols / 32; ++j) {
+        const int64_t n = w->n0 + kCols * wg + 32 * j + lane;
+        cols[32 * j + lane] = n < w->N ? offs(w->csC, w->uC_n, n) : 0;
+      }
+      __syncwarp();
       float master[kUnits][16];
 #pragma unroll
       for (int u = 0; u < kUnits; ++u)
 #pragma unroll
         for (int j = 0; j < 16; ++j) master[u][j] = 0.f;
-      auto unit_col = [&](int u) { return 16 * (wg + 4 * u); };
+      // Unit u holds columns [unit_col(u), + 16) of the tile: each warpgroup
+      // takes kCols adjacent columns.
+      auto unit_col = [&](int u) { return kCols * wg + 16 * u; };
       auto fold = [&](uint32_t col) {
 #pragma unroll
         for (int u = 0; u < kUnits; ++u) {
-          if (unit_col(u) < x.tn) {
+          if (unit_col(u) < tn) {
             uint32_t r[16];
             ptx::tmem_ld16_sync(tmem + lane_base + col + unit_col(u), r);
 #pragma unroll
@@ -716,9 +829,9 @@ tc1m_pieces(const __grid_constant__ PieceProblem single, const PieceProblem* gro
         __syncwarp();
         if (lane == 0) ptx::mbar_arrive_cluster(ptx::mapa(bar, 0));
       };
-      const int64_t nchunks = (x.steps + 2 * kPcFold - 1) / (2 * kPcFold);
+      const int nchunks = (w->steps + 2 * kPcFold - 1) / (2 * kPcFold);
       bool ok = true;
-      for (int64_t c = 0; c < nchunks; ++c, ++chunk) {
+      for (int c = 0; c < nchunks; ++c, ++chunk) {
         const int buf = static_cast<int>(chunk % kBufs);
         if (!ptx::mbar_wait(chunk_full(buf), static_cast<uint32_t>((chunk / kBufs) & 1))) {
           record_error(err_flag, kErrChunkWait);
@@ -738,25 +851,25 @@ tc1m_pieces(const __grid_constant__ PieceProblem single, const PieceProblem* gro
       ptx::tc_fence_after();
       fold(Sh::corr_col(cb));
       release(corr_empty(cb));
-      const GemmArgs& g = x.p->g;
       if constexpr (kReal) {
-        const int64_t row = (2 * x.tm + rank) * kPcARows + rho;
-        if (row < g.M) {
-          float* Cr = static_cast<float*>(g.C) + x.split * g.c_split_stride +
-                      offs(g.rsC, g.uC_m, row);
+        if (row_ok) {
+          float* Cr = static_cast<float*>(w->C) + row_off;
 #pragma unroll
           for (int u = 0; u < kUnits; ++u)
-            if (unit_col(u) < x.tn) pc_store16_real(g, Cr, x.n0 + unit_col(u), master[u]);
+            if (unit_col(u) < tn)
+              pc_store16_real(*w, cols + 16 * u, Cr, w->n0 + unit_col(u), master[u]);
         }
       } else {
-        const int64_t row = (2 * x.tm + rank) * (kPcARows / 2) + (rho >> 1);
-        const bool row_ok = row < g.M;
-        float2* Cr = static_cast<float2*>(g.C) + x.split * g.c_split_stride +
-                     (row_ok ? offs(g.rsC, g.uC_m, row) : 0);
+        float2* Cr = static_cast<float2*>(w->C) + row_off;
 #pragma unroll
         for (int u = 0; u < kUnits; ++u)
-          if (unit_col(u) < x.tn) pc_store16(g, Cr, row_ok, x.n0 + unit_col(u), rho & 1, master[u]);
+          if (unit_col(u) < tn)
+            pc_store16(*w, cols + 16 * u, Cr, row_ok, w->n0 + unit_col(u), rho & 1, master[u]);
       }
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive(work_empty(cur.e));
+      advance(cur);
+      ++tile_cnt;
     }
   }
 

@@ -401,9 +401,9 @@ __device__ __forceinline__ void skinny_body(const GemmArgs& g, int64_t tile, T (
 // (at most kSkinnyAsyncMaxK) is staged once, after the first A stages are
 // issued.  Warp w reduces rows 4w..4w+3, lanes over k as in skinny_body.
 // Five stages of 16 KB with two CTAs per SM keep up to 128 KB of A in flight
-// per SM; the sweep's second steps (59.8 GB of A per batch) read at 2.8 TB/s,
-// about as with three stages: the per-tile B staging and the short K chunks
-// (at most kSkinnyAsyncMaxK per tile) bound them.
+// per SM.  A block runs up to four 32-row tiles over one staged B chunk, their
+// copies in one continuous ring: with one tile per block (256 KB of A) its
+// start and the B staging took a third of its time.
 constexpr int kSkStages = 5;
 constexpr int kSkKS = 64;  // k per stage
 constexpr size_t kSkAsyncSmem =
@@ -436,13 +436,17 @@ __device__ __forceinline__ void skinny_async_body(const GemmArgs& g, int64_t til
   T (*Bs)[kSkinnyAsyncMaxK] =
       reinterpret_cast<T (*)[kSkinnyAsyncMaxK]>(dsmem + size_t(kSkStages) * 32 * kSkKS * 8);
   const int64_t M = g.M, N = g.N, K = g.K;
-  const int64_t tiles_m = (M + 31) / 32;
+  const int rows_per = skinny_async_rows(M);
+  const int64_t tiles_m = (M + rows_per - 1) / rows_per;
   const int64_t split = tile / tiles_m;
-  const int64_t m0 = (tile - split * tiles_m) * 32;
+  const int64_t m0 = (tile - split * tiles_m) * rows_per;
   const int64_t kb = split * g.k_per_split;
   const int64_t ke = min(K, kb + g.k_per_split);
   const int kn = static_cast<int>(ke - kb);
   const int nst = (kn + kSkKS - 1) / kSkKS;
+  // Stages of all the block's 32-row tiles, one after the other.
+  const int ntile = static_cast<int>((min(M - m0, static_cast<int64_t>(rows_per)) + 31) / 32);
+  const int total = nst * ntile;
   T* __restrict__ C = static_cast<T*>(g.C) + split * g.c_split_stride;
   const T* __restrict__ A = static_cast<const T*>(g.A);
   const T* __restrict__ B = static_cast<const T*>(g.B);
@@ -451,53 +455,63 @@ __device__ __forceinline__ void skinny_async_body(const GemmArgs& g, int64_t til
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
   // Copies of this thread: 16-byte chunk c = tid + 256 i of a stage, row
-  // c / 32, elements 2 (c % 32) and 2 (c % 32) + 1.
+  // c / 32, elements 2 (c % 32) and 2 (c % 32) + 1.  (is, it): the stage and
+  // tile issued next.
   int64_t rowoff[4];
   bool rok[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int r = (tid >> 5) + 8 * i;
-    rok[i] = m0 + r < M;
-    rowoff[i] = rok[i] ? offs(g.rsA, g.uA_m, m0 + r) : 0;
-  }
-  const int kk2 = 2 * (tid & 31);
-  auto issue = [&](int s) {
-    const int slot = s % kSkStages;
-    const int64_t k0 = kb + int64_t(s) * kSkKS;
+  int is = 0, it = 0, islot = 0;
+  auto rows_of = [&](int rt) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const int r = (tid >> 5) + 8 * i;
-      const int64_t k = k0 + kk2;
-      const bool in = rok[i] && k < ke;
-      const uint32_t bytes = in ? static_cast<uint32_t>(min(static_cast<int64_t>(2), ke - k) * 8) : 0u;
-      const T* src = in ? A + rowoff[i] + k : A;
-      cp_async_16(static_cast<uint32_t>(__cvta_generic_to_shared(&ring[slot][r][kk2])), src, bytes);
+      const int64_t m = m0 + 32 * rt + (tid >> 5) + 8 * i;
+      rok[i] = m < M;
+      rowoff[i] = rok[i] ? offs(g.rsA, g.uA_m, m) : 0;
+    }
+  };
+  rows_of(0);
+  const int kk2 = 2 * (tid & 31);
+  auto issue = [&]() {
+    if (it < ntile) {
+      const int64_t k = kb + int64_t(is) * kSkKS + kk2;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int r = (tid >> 5) + 8 * i;
+        const bool in = rok[i] && k < ke;
+        const uint32_t bytes =
+            in ? static_cast<uint32_t>(min(static_cast<int64_t>(2), ke - k) * 8) : 0u;
+        const T* src = in ? A + rowoff[i] + k : A;
+        cp_async_16(static_cast<uint32_t>(__cvta_generic_to_shared(&ring[islot][r][kk2])), src,
+                    bytes);
+      }
+      if (++islot == kSkStages) islot = 0;
+      if (++is == nst) {
+        is = 0;
+        if (++it < ntile) rows_of(it);
+      }
     }
     cp_async_commit();
   };
 #pragma unroll
-  for (int s = 0; s < kSkStages - 1; ++s) {
-    if (s < nst) issue(s);
-    else cp_async_commit();
-  }
+  for (int s = 0; s < kSkStages - 1; ++s) issue();
   // B chunk, zero-padded to NMAX columns and to whole stages, while the
   // first A stages are in flight (visible at the first stage's barrier).
-  for (int e = tid; e < NMAX * nst * kSkKS; e += kThreads) {
-    const int n = e / (nst * kSkKS), kk = e % (nst * kSkKS);
-    T v = zero<T>();
-    if (n < N && kk < kn)
-      v = conj_if(B[offs(g.rsB, g.uB_k, kb + kk) + offs(g.csB, g.uB_n, n)], conjB);
-    Bs[n][kk] = v;
+  for (int kk = tid; kk < nst * kSkKS; kk += kThreads) {
+    const int64_t ob = kk < kn ? offs(g.rsB, g.uB_k, kb + kk) : 0;
+#pragma unroll
+    for (int n = 0; n < NMAX; ++n)
+      Bs[n][kk] = n < N && kk < kn ? conj_if(B[ob + offs(g.csB, g.uB_n, n)], conjB) : zero<T>();
   }
   T acc[RW][NMAX];
 #pragma unroll
   for (int r = 0; r < RW; ++r)
 #pragma unroll
     for (int n = 0; n < NMAX; ++n) acc[r][n] = zero<T>();
-  for (int s = 0; s < nst; ++s) {
+  int st = 0, slot = 0;
+  int64_t mt = m0;  // first row of the current tile
+  for (int s = 0; s < total; ++s) {
     cp_async_wait<kSkStages - 2>();
     __syncthreads();  // stage s visible to all; the slot refilled below is free
-    const int slot = s % kSkStages;
+    issue();
 #pragma unroll
     for (int u = 0; u < kSkKS / 32; ++u) {
       const int kk = lane + 32 * u;
@@ -505,28 +519,40 @@ __device__ __forceinline__ void skinny_async_body(const GemmArgs& g, int64_t til
       for (int r = 0; r < RW; ++r) {
         const T a = conj_if(ring[slot][warp * RW + r][kk], conjA);
 #pragma unroll
-        for (int n = 0; n < NMAX; ++n) mac(acc[r][n], a, Bs[n][s * kSkKS + kk]);
+        for (int n = 0; n < NMAX; ++n) mac(acc[r][n], a, Bs[n][st * kSkKS + kk]);
       }
     }
-    if (s + kSkStages - 1 < nst) issue(s + kSkStages - 1);
-    else cp_async_commit();
+    if (++slot == kSkStages) slot = 0;
+    if (++st < nst) continue;
+    // The tile's last stage: the 16 sums (4 rows x 4 columns) of every lane
+    // added across the warp.  Each step exchanges half of the values a lane
+    // still holds (16 exchanges instead of 80), lane l ending with value
+    // (l >> 1) & 15, which it writes.
+    st = 0;
+    T v[RW * NMAX];
+#pragma unroll
+    for (int r = 0; r < RW; ++r)
+#pragma unroll
+      for (int n = 0; n < NMAX; ++n) {
+        v[r * NMAX + n] = acc[r][n];
+        acc[r][n] = zero<T>();
+      }
+#pragma unroll
+    for (int h = RW * NMAX / 2, d = 16; h >= 1; h >>= 1, d >>= 1) {
+      const bool up = lane & d;
+#pragma unroll
+      for (int i = 0; i < h; ++i) {
+        const T keep = up ? v[i + h] : v[i];
+        v[i] = add(keep, shfl_xor(up ? v[i] : v[i + h], d));
+      }
+    }
+    v[0] = add(v[0], shfl_xor(v[0], 1));
+    const int val = (lane >> 1) & 15, n = val % NMAX;
+    const int64_t m = mt + warp * RW + val / NMAX;
+    if (!(lane & 1) && m < M && n < N) skinny_store(g, C, m, n, v[0]);
+    mt += 32;
   }
   cp_async_wait<0>();
-#pragma unroll
-  for (int r = 0; r < RW; ++r) {
-#pragma unroll
-    for (int n = 0; n < NMAX; ++n) {
-      T v = acc[r][n];
-#pragma unroll
-      for (int d = 16; d >= 1; d >>= 1) v = add(v, shfl_xor(v, d));
-      acc[r][n] = v;
-    }
-    const int64_t m = m0 + warp * RW + r;
-    if (lane == 0 && m < M)
-#pragma unroll
-      for (int n = 0; n < NMAX; ++n)
-        if (n < N) skinny_store(g, C, m, n, acc[r][n]);
-  }
 }
 
 template <class T, int NMAX>
@@ -539,13 +565,9 @@ skinny_contract(const SimtProblem* group, int nprob) {
   T (*Bs)[2048 / NMAX] = reinterpret_cast<T (*)[2048 / NMAX]>(skinny_dsmem);
   int64_t* ks = reinterpret_cast<int64_t*>(skinny_dsmem + size_t(NMAX) * (2048 / NMAX) * sizeof(T));
   int64_t tile = blockIdx.x;
-  int lo = 0, hi = nprob - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (group[mid].tile_begin <= tile) lo = mid; else hi = mid - 1;
-  }
+  const int lo = block_find(nprob, tile, [&](int i) { return group[i].tile_begin; });
   tile -= group[lo].tile_begin;
-  if (threadIdx.x == 0) ga = group[lo].g;
+  block_copy(&ga, &group[lo].g);
   __syncthreads();
   if constexpr (NMAX == 4 && sizeof(T) == 8) {
     if (ga.flags & kFlagSkinnyAsync) {
@@ -610,7 +632,8 @@ bool skinny_async_ok(const GemmArgs& g, const std::vector<int64_t>& rsA, size_t 
 }
 
 int64_t skinny_tiles(const GemmArgs& g, int splits, int nmax) {
-  const int64_t rows = skinny_rows(skinny_k_lanes(g.uA_k, g.M), nmax);
+  const int64_t rows = g.flags & kFlagSkinnyAsync ? skinny_async_rows(g.M)
+                                                  : skinny_rows(skinny_k_lanes(g.uA_k, g.M), nmax);
   return int64_t(splits) * ((g.M + rows - 1) / rows);
 }
 

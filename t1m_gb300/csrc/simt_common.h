@@ -6,6 +6,8 @@
 
 #include <cstdint>
 
+#include "device_common.h"
+
 namespace t1m {
 namespace gb300 {
 namespace {
@@ -73,10 +75,6 @@ __device__ __forceinline__ float add(float a, float b) { return a + b; }
 __device__ __forceinline__ double add(double a, double b) { return a + b; }
 __device__ __forceinline__ float2 add(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ double2 add(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
-
-__device__ __forceinline__ int64_t offs(const int64_t* v, int64_t u, int64_t i) {
-  return u >= 0 ? i * u : __ldg(v + i);
-}
 
 // Global -> shared copy of one element (4, 8 or 16 bytes) that does not pass
 // through registers; src_bytes 0 writes zeros (operands past the tile edge).

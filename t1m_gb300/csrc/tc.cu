@@ -2550,9 +2550,10 @@ static PieceSplit piece_split_args(int dtype, bool operand_a, bool swapped, cons
 
 cudaError_t tc_split_operand(int dtype, int pieces, bool operand_a, const GemmArgs& g,
                              const HostPlan& plan, void* out, int64_t groups, cudaStream_t s) {
-  const PieceSplit op = piece_split_args(dtype, operand_a, false, g, plan, out, groups);
+  PieceSplit op = piece_split_args(dtype, operand_a, false, g, plan, out, groups);
   const bool real = dtype == T1M_FLOAT32;
-  return launch_piece_split(pieces, real, &op, 1, nullptr, piece_split_blocks(real, op), s);
+  const int64_t blocks = piece_split_blocks(real, op);
+  return launch_piece_split(pieces, real, &op, 1, nullptr, blocks, s);
 }
 
 size_t tc_panel_bytes(int dtype, int64_t M, int64_t N, int64_t K) {
@@ -2677,13 +2678,14 @@ static cudaError_t launch_pieces(int method, int dtype, const GemmArgs& g, const
   cudaError_t e;
   if (n == 2 && uniform) {
     ops[1].block_begin = piece_split_blocks(real, ops[0]);
-    e = launch_piece_split(P, real, ops, 2, nullptr,
-                           ops[1].block_begin + piece_split_blocks(real, ops[1]), stream);
+    const int64_t blocks = ops[1].block_begin + piece_split_blocks(real, ops[1]);
+    e = launch_piece_split(P, real, ops, 2, nullptr, blocks, stream);
     if (e != cudaSuccess) return e;
     ++*kernels;
   } else {
     for (int i = 0; i < n; ++i) {
-      e = launch_piece_split(P, real, &ops[i], 1, nullptr, piece_split_blocks(real, ops[i]), stream);
+      const int64_t blocks = piece_split_blocks(real, ops[i]);
+      e = launch_piece_split(P, real, &ops[i], 1, nullptr, blocks, stream);
       if (e != cudaSuccess) return e;
       ++*kernels;
     }

@@ -6,6 +6,7 @@
 
 #include <cstdint>
 
+#include "device_common.h"
 #include "internal.h"
 #include "ptx.h"
 
@@ -20,12 +21,9 @@ enum : int {
   kErrChunkWait = 4,
   kErrRawWait = 5,
   kErrAccEmptyWait = 6,
-  kErrDepWait = 7
+  kErrDepWait = 7,
+  kErrWorkWait = 8
 };
-
-__device__ __forceinline__ int64_t offs(const int64_t* v, int64_t u, int64_t i) {
-  return u >= 0 ? i * u : __ldg(v + i);
-}
 
 __device__ __forceinline__ void record_error(int* flag, int code) {
   if (flag) atomicCAS(flag, 0, code);
