@@ -279,6 +279,21 @@ def _data_ptr(data: Any) -> tuple[int, np.dtype]:
                     f"(element type {getattr(data, 'dtype', None)})")
 
 
+_INT64_ARRAYS: dict[int, type] = {}
+
+
+def _int64_array(n: int) -> type:
+    """The ctypes array type of max(1, n) int64 (built once per length)."""
+    t = _INT64_ARRAYS.get(n)
+    if t is None:
+        t = _INT64_ARRAYS[n] = C.c_int64 * max(1, n)
+    return t
+
+
+_FLOAT1, _FLOAT2 = C.c_float * 1, C.c_float * 2
+_DOUBLE1, _DOUBLE2 = C.c_double * 1, C.c_double * 2
+
+
 @dataclass
 class tensor:
     """Non-owning tensor view, like the reference's t1m::tensor (t1m.h:31-66).
@@ -300,11 +315,12 @@ class tensor:
     def _c(self, keep: list, ptr: int | None = None) -> _Tensor:
         if ptr is None:
             ptr = _data_ptr(self.data)[0]
-        ext = (C.c_int64 * max(1, len(self.dims)))(*[int(d) for d in self.dims])
+        n = len(self.dims)
+        ext = _int64_array(n)(*map(int, self.dims))
         keep.append(ext)
-        t = _Tensor(len(self.dims), int(self.layout), ext, None, ptr)
+        t = _Tensor(n, int(self.layout), ext, None, ptr)
         if self.strides is not None:
-            st = (C.c_int64 * max(1, len(self.strides)))(*[int(s) for s in self.strides])
+            st = _int64_array(len(self.strides))(*map(int, self.strides))
             keep.append(st)
             t.layout = STRIDED
             t.strides = st
@@ -320,12 +336,12 @@ class tensor:
 def _scalar_bytes(dtype: int, v) -> C.Array:
     v = complex(v)
     if dtype == FLOAT32:
-        return (C.c_float * 1)(v.real)
+        return _FLOAT1(v.real)
     if dtype == FLOAT64:
-        return (C.c_double * 1)(v.real)
+        return _DOUBLE1(v.real)
     if dtype == COMPLEX64:
-        return (C.c_float * 2)(v.real, v.imag)
-    return (C.c_double * 2)(v.real, v.imag)
+        return _FLOAT2(v.real, v.imag)
+    return _DOUBLE2(v.real, v.imag)
 
 
 def contract_raw(alpha, a: tensor, la: str, b: tensor, lb: str, beta, c: tensor, lc: str,

@@ -26,7 +26,12 @@ enum : int {
 };
 
 __device__ __forceinline__ void record_error(int* flag, int code) {
-  if (flag) atomicCAS(flag, 0, code);
+  // Host memory (t1m_context::d_err): a plain store, the first code seen wins.
+  volatile int* const f = flag;
+  if (f && *f == 0) {
+    *f = code;
+    __threadfence_system();
+  }
 }
 
 // Split-product precision of the one-tile-per-CTA kernel.
