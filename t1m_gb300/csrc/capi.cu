@@ -287,18 +287,20 @@ int choose_splits(const t1m_context* ctx, int method, int dtype, int64_t M, int6
   const int64_t tiles = ((M + bm - 1) / bm) * ((N + bn - 1) / bn);
   const int64_t ksteps = (K + bk - 1) / bk;
   int64_t s = 1;
-  if (method == T1M_METHOD_PLAIN && ctx->split_k == 0 &&
-      (dtype == T1M_FLOAT64 || dtype == T1M_COMPLEX128)) {
-    s = fp64_form(dtype, M, N, K, 0).splits;
+  const SmallForm small = method == T1M_METHOD_PLAIN && ctx->split_k == 0
+                              ? small_form(dtype, M, N, K, 0)
+                              : SmallForm{0, 1};
+  if (small.tile > 0) {
+    s = small.splits;
   } else if (ctx->split_k > 0) {
     s = ctx->split_k;
   } else {
     const int64_t target = int64_t(ctx->num_sms) * per_sm;
     if (tiles < target / 2 && ksteps >= 8)
       s = std::min<int64_t>((target + tiles - 1) / tiles, ksteps / 4);
-    const int64_t lim = promote ? accuracy_k_limit(method, dtype) : 0;
-    if (lim > 0) s = std::max<int64_t>(s, (K + lim - 1) / lim);
   }
+  const int64_t lim = promote && ctx->split_k == 0 ? accuracy_k_limit(method, dtype) : 0;
+  if (lim > 0) s = std::max<int64_t>(s, (K + lim - 1) / lim);
   s = std::max<int64_t>(1, std::min<int64_t>({s, ksteps, 4096}));
   while (s > 1 && size_t(s) * size_t(M) * size_t(N) * elem > kMaxWorkBytes) --s;
   const int64_t steps_per = (ksteps + s - 1) / s;
@@ -620,6 +622,9 @@ int run_pipelined(t1m_context* ctx, int method, int dtype, size_t es, const Host
   };
 
   int kernels = 0, used_method = method, splits = 1, nblock = 0;
+  // Plain blocks run on the whole product's tile form, for the same sums.
+  const uint32_t tile_flag =
+      method == T1M_METHOD_PLAIN ? small_tile_flag(small_form(dtype, hp.M, hp.N, hp.K, 1).tile) : 0;
   // Block (slab i, half h): the slab dimension shortened to the slab, the
   // halved dimension to the half, operands and C shifted accordingly
   // (uniform strides, so no scatter vector changes).
@@ -651,6 +656,7 @@ int run_pipelined(t1m_context* ctx, int method, int dtype, size_t es, const Host
     }
     gs.k_per_split = hp.K;
     gs.c_split_stride = 0;
+    gs.flags |= tile_flag;
     return gs;
   };
   // Operand pieces: where the blocks run as pieces, the resident operand is

@@ -151,17 +151,24 @@ cudaError_t launch_simt(int dtype, const GemmArgs& args, int splits, cudaStream_
 // Output tile sizes of the plain kernel for a dtype (for split decisions).
 void simt_tile(int dtype, int* bm, int* bn, int* bk);
 
-// fp64.cu: the plain kernel of float64 / complex128.  Tile (16 or 8 rows and
-// columns), split count and K per split (a multiple of 16) of a product; with
-// `forced` > 0 that split count.
-struct Fp64Form {
+// small_tile.cu: small output tiles (16 or 8 rows and columns), for float64 /
+// complex128 and for small float32 / complex64 products.  The tile (0: the
+// plain kernel of simt.cu) and split count of a product; with `forced` > 0
+// that split count.
+struct SmallForm {
   int tile;
   int splits;
-  int64_t k_per_split;
 };
+SmallForm small_form(int dtype, int64_t M, int64_t N, int64_t K, int64_t forced);
+// Flags that fix the tile of a plain product (blocks of one product that must
+// sum as the whole would); without them launch_simt asks small_form.
+constexpr uint32_t kFlagTilePlain = 256u, kFlagTile16 = 512u, kFlagTile8 = 1024u;
+inline uint32_t small_tile_flag(int tile) {
+  return tile == 16 ? kFlagTile16 : tile == 8 ? kFlagTile8 : kFlagTilePlain;
+}
+cudaError_t launch_small(int dtype, int tile, const GemmArgs& args, int splits,
+                         cudaStream_t stream);
 constexpr int kFp64Tile = 16;  // tile of grouped launches
-Fp64Form fp64_form(int dtype, int64_t M, int64_t N, int64_t K, int64_t forced);
-cudaError_t launch_fp64(int dtype, const GemmArgs& args, int splits, cudaStream_t stream);
 struct SimtProblem;
 cudaError_t launch_fp64_group(int dtype, const SimtProblem* dev, int nprob, int64_t total_tiles,
                               cudaStream_t stream);

@@ -260,8 +260,10 @@ extern "C" int t1m_contract_noalloc(void* stream_ptr, int method, int dtype, con
     const int64_t ksteps = (hp.K + bk - 1) / bk;
     int64_t s = 1;
     const int64_t target = int64_t(sms) * per_sm;
-    if (method == T1M_METHOD_PLAIN && (dtype == T1M_FLOAT64 || dtype == T1M_COMPLEX128))
-      s = fp64_form(dtype, hp.M, hp.N, hp.K, 0).splits;
+    const SmallForm small = method == T1M_METHOD_PLAIN ? small_form(dtype, hp.M, hp.N, hp.K, 0)
+                                                       : SmallForm{0, 1};
+    if (small.tile > 0)
+      s = small.splits;
     else if (tiles < target / 2 && ksteps >= 8)
       s = std::min<int64_t>((target + tiles - 1) / tiles, ksteps / 4);
     // The precision rule of the automatic method (accuracy_k_limit).

@@ -684,11 +684,13 @@ void simt_tile(int dtype, int* bm, int* bn, int* bk) {
 cudaError_t launch_simt(int dtype, const GemmArgs& args, int splits, cudaStream_t stream,
                         int* kernels) {
   *kernels = 1;
-  switch (dtype) {
-    case 0: return launch<float, 8, 8, 8>(args, splits, stream);
-    case 1: case 3: return launch_fp64(dtype, args, splits, stream);
-    case 2: return launch<float2, 4, 8, 8>(args, splits, stream);
-  }
+  const int tile = args.flags & kFlagTile16      ? 16
+                   : args.flags & kFlagTile8     ? 8
+                   : args.flags & kFlagTilePlain ? 0
+                                                 : small_form(dtype, args.M, args.N, args.K, splits).tile;
+  if (tile > 0) return launch_small(dtype, tile, args, splits, stream);
+  if (dtype == 0) return launch<float, 8, 8, 8>(args, splits, stream);
+  if (dtype == 2) return launch<float2, 4, 8, 8>(args, splits, stream);
   return cudaErrorInvalidValue;
 }
 

@@ -1,4 +1,4 @@
-// Element helpers of the SIMT kernels (simt.cu, fp64.cu): complex and real
+// Element helpers of the SIMT kernels (simt.cu, small_tile.cu): complex and real
 // arithmetic by element type, offset lookup and asynchronous element copies.
 #pragma once
 

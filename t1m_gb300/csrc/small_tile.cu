@@ -1,21 +1,23 @@
-// float64 / complex128 contraction in FP64 FMAs on small output tiles.
+// Contractions on small output tiles: the plain kernel of float64 /
+// complex128, and of float32 / complex64 products too small for simt.cu's.
 //
-// GB300 issues two FP64 FMAs per clock and SM (1.25 TFLOP/s nominal), so a
-// warp's FMA occupies its scheduler for 64 clocks and everything else of the
-// loop (shared-memory reads, copies, address arithmetic) hides behind it even
-// with one output per thread.  What bounds a product is how evenly its FMAs
-// spread over the 152 SMs and how many of them are padding.  Hence the small
-// tiles: a 128 x 64 tile of 256 threads (the FP32 kernel's shape) takes an SM
-// 16 us per 8 k of float64, whatever part of it lies inside the output.
+// FP64: GB300 issues two FP64 FMAs per clock and SM (1.25 TFLOP/s nominal),
+// so a warp's FMA occupies its scheduler for 64 clocks and everything else of
+// the loop (shared-memory reads, copies, address arithmetic) hides behind it
+// even with one output per thread.  What bounds a product is how evenly its
+// FMAs spread over the 152 SMs and how many of them are padding; a 128 x 64
+// tile of 256 threads (simt.cu's shape) takes an SM 16 us per 8 k of float64,
+// whatever part of it lies inside the output.
+// FP32: a small product is a chain of latencies (offsets, operands, sums,
+// C), to which a 64 x 128 tile adds the FMAs of its padding.
 //   16 x 16 outputs: two per thread;
 //   8 x 8 outputs:   one per thread, the two halves of the block taking
 //                    alternate k and added in a fixed order at the end, for
 //                    outputs with too few tiles to occupy every SM.
 // Steps past K are not computed, and a warp whose outputs all lie past the edge
 // computes nothing.
-// Measured (GB300): complex128 1024^3 8.23 -> 6.95 ms (1.24 TFLOP/s), float64
-// 9216 x 96 x 96 283 -> 195 us per synchronous call, 98% of the 2-FMA rate in
-// the first.
+// Measured (GB300): complex128 1024^3 8.23 -> 6.95 ms (1.24 TFLOP/s, 98% of
+// the two-FMA rate), float64 9216 x 96 x 96 281 -> 196 us a call.
 //
 // Tiles are gathered through the scatter vectors as in simt.cu (the plain
 // form; replaces the reference's include/t1m/t1m.h:432-557 in FP64), each
@@ -32,10 +34,15 @@ namespace t1m {
 namespace gb300 {
 namespace {
 
-constexpr int kThreads64 = 128;
-constexpr int kBK64 = 16;      // k per stage
-constexpr int kStages64 = 3;
+constexpr int kThreads = 128;
+constexpr int kBK = 16;      // k per stage
+constexpr int kStages = 3;
 
+__device__ __forceinline__ float flip(float v, uint64_t) { return v; }
+__device__ __forceinline__ float2 flip(float2 v, uint64_t sign) {
+  v.y = __uint_as_float(__float_as_uint(v.y) ^ static_cast<uint32_t>(sign >> 32));
+  return v;
+}
 // Conjugation by the sign bit: a floating negation of a value that is not an
 // FMA operand would go through the FP64 pipe (measured: half as many FP64
 // instructions again, complex128 1024^3 10.5 ms against 7.1).
@@ -46,10 +53,10 @@ __device__ __forceinline__ double2 flip(double2 v, uint64_t sign) {
 }
 
 template <class T, int kTile>
-struct Smem64 {
+struct SmallSmem {
   static constexpr int kPad = 32 / sizeof(T);
-  T a[kStages64][kBK64][kTile + kPad];
-  T b[kStages64][kBK64][kTile + kPad];
+  T a[kStages][kBK][kTile + kPad];
+  T b[kStages][kBK][kTile + kPad];
   T part[kTile * kTile];  // the second k slice's sums (8 x 8 form)
   int64_t row_a[kTile], col_b[kTile];
 };
@@ -58,10 +65,10 @@ struct Smem64 {
 // columns.  kNFast: consecutive threads along n (C unit stride along its
 // columns), else along m.
 template <class T, int kTile, bool kNFast>
-__device__ __forceinline__ void fp64_tile(const GemmArgs& args, int64_t tile, int64_t split,
-                                          Smem64<T, kTile>& sm) {
-  constexpr int kOut = kTile * kTile >= kThreads64 ? kTile * kTile / kThreads64 : 1;
-  constexpr int kSlices = kThreads64 * kOut / (kTile * kTile);  // k slices of the block
+__device__ __forceinline__ void small_tile(const GemmArgs& args, int64_t tile, int64_t split,
+                                          SmallSmem<T, kTile>& sm) {
+  constexpr int kOut = kTile * kTile >= kThreads ? kTile * kTile / kThreads : 1;
+  constexpr int kSlices = kThreads * kOut / (kTile * kTile);  // k slices of the block
   constexpr int kSlow = kTile / kOut;                           // step between a thread's outputs
   auto& As = sm.a;
   auto& Bs = sm.b;
@@ -95,23 +102,23 @@ __device__ __forceinline__ void fp64_tile(const GemmArgs& args, int64_t tile, in
 
   const bool a_kfast = args.uA_k == 1;
   const bool b_kfast = args.uB_k == 1 || args.uB_n != 1;
-  constexpr int kPer = kTile * kBK64 / kThreads64;
-  static_assert(kPer * kThreads64 == kTile * kBK64, "stage copies");
+  constexpr int kPer = kTile * kBK / kThreads;
+  static_assert(kPer * kThreads == kTile * kBK, "stage copies");
   auto issue = [&](int64_t k0, int buf) {
 #pragma unroll
     for (int p = 0; p < kPer; ++p) {
-      const int idx = tid + p * kThreads64;
-      const int m = a_kfast ? idx / kBK64 : idx % kTile;
-      const int k = a_kfast ? idx % kBK64 : idx / kTile;
+      const int idx = tid + p * kThreads;
+      const int m = a_kfast ? idx / kBK : idx % kTile;
+      const int k = a_kfast ? idx % kBK : idx / kTile;
       const bool in = m0 + m < M && k0 + k < K;
       cp_async_elem<sizeof(T)>(&As[buf][k][m],
                                in ? A + rowA[m] + offs(args.csA, args.uA_k, k0 + k) : A, in);
     }
 #pragma unroll
     for (int p = 0; p < kPer; ++p) {
-      const int idx = tid + p * kThreads64;
-      const int n = b_kfast ? idx / kBK64 : idx % kTile;
-      const int k = b_kfast ? idx % kBK64 : idx / kTile;
+      const int idx = tid + p * kThreads;
+      const int n = b_kfast ? idx / kBK : idx % kTile;
+      const int k = b_kfast ? idx % kBK : idx / kTile;
       const bool in = n0 + n < N && k0 + k < K;
       cp_async_elem<sizeof(T)>(&Bs[buf][k][n],
                                in ? B + offs(args.rsB, args.uB_k, k0 + k) + colB[n] : B, in);
@@ -134,20 +141,20 @@ __device__ __forceinline__ void fp64_tile(const GemmArgs& args, int64_t tile, in
 #pragma unroll
     for (int u = 0; u < kChains; ++u) part[j][u] = zero<T>();
 
-  const int64_t ksteps = K > kb ? (K - kb + kBK64 - 1) / kBK64 : 0;
+  const int64_t ksteps = K > kb ? (K - kb + kBK - 1) / kBK : 0;
 #pragma unroll
-  for (int st = 0; st < kStages64 - 1; ++st) {
-    if (st < ksteps) issue(kb + st * kBK64, st);
+  for (int st = 0; st < kStages - 1; ++st) {
+    if (st < ksteps) issue(kb + st * kBK, st);
     cp_async_commit_group();
   }
   for (int64_t st = 0; st < ksteps; ++st) {
-    const int buf = static_cast<int>(st % kStages64);
-    cp_async_wait_group<kStages64 - 2>();
+    const int buf = static_cast<int>(st % kStages);
+    cp_async_wait_group<kStages - 2>();
     __syncthreads();  // stage st has landed for every thread; stage st - 1 is consumed
-    const int64_t nxt = st + kStages64 - 1;
-    if (nxt < ksteps) issue(kb + nxt * kBK64, static_cast<int>(nxt % kStages64));
+    const int64_t nxt = st + kStages - 1;
+    if (nxt < ksteps) issue(kb + nxt * kBK, static_cast<int>(nxt % kStages));
     cp_async_commit_group();
-    const int kn = static_cast<int>(min(static_cast<int64_t>(kBK64), K - kb - st * kBK64));
+    const int kn = static_cast<int>(min(static_cast<int64_t>(kBK), K - kb - st * kBK));
     auto step = [&](int k, int u) {
       const T x = kNFast ? flip(Bs[buf][k][f], signB) : flip(As[buf][k][f], signA);
 #pragma unroll
@@ -158,9 +165,9 @@ __device__ __forceinline__ void fp64_tile(const GemmArgs& args, int64_t tile, in
         if (kNFast) mac(part[j][u], y, x); else mac(part[j][u], x, y);
       }
     };
-    if (kn == kBK64) {
+    if (kn == kBK) {
 #pragma unroll
-      for (int k = 0; k < kBK64; k += 4)
+      for (int k = 0; k < kBK; k += 4)
 #pragma unroll
         for (int u = 0; u < kChains; ++u) step(k + u * kSlices + slice, u);
     } else {
@@ -209,9 +216,9 @@ __device__ __forceinline__ void fp64_tile(const GemmArgs& args, int64_t tile, in
 // group[0..nprob) (sorted by tile_begin, split-major within a problem);
 // otherwise it is a tile of args0 and blockIdx.y its split.
 template <class T, int kTile, bool kGroup>
-__global__ void __launch_bounds__(kThreads64)
-fp64_contract(const GemmArgs args0, const SimtProblem* group, int nprob) {
-  __shared__ __align__(16) Smem64<T, kTile> sm;
+__global__ void __launch_bounds__(kThreads)
+small_contract(const GemmArgs args0, const SimtProblem* group, int nprob) {
+  __shared__ __align__(16) SmallSmem<T, kTile> sm;
   __shared__ GemmArgs group_args;
   int64_t tile = blockIdx.x, split = blockIdx.y;
   if constexpr (kGroup) {
@@ -229,9 +236,9 @@ fp64_contract(const GemmArgs args0, const SimtProblem* group, int nprob) {
   }
   const GemmArgs& args = kGroup ? group_args : args0;
   if (args.uC_n == 1 && args.uC_m != 1)
-    fp64_tile<T, kTile, true>(args, tile, split, sm);
+    small_tile<T, kTile, true>(args, tile, split, sm);
   else
-    fp64_tile<T, kTile, false>(args, tile, split, sm);
+    small_tile<T, kTile, false>(args, tile, split, sm);
 }
 
 template <class T>
@@ -241,47 +248,67 @@ cudaError_t launch(const GemmArgs& g, int tile, int splits, cudaStream_t stream)
   if (tiles > 0x7fffffffLL || splits < 1 || splits > 65535) return cudaErrorInvalidConfiguration;
   const dim3 grid(static_cast<unsigned>(tiles), static_cast<unsigned>(splits));
   if (tile == 16)
-    fp64_contract<T, 16, false><<<grid, kThreads64, 0, stream>>>(g, nullptr, 0);
+    small_contract<T, 16, false><<<grid, kThreads, 0, stream>>>(g, nullptr, 0);
   else
-    fp64_contract<T, 8, false><<<grid, kThreads64, 0, stream>>>(g, nullptr, 0);
+    small_contract<T, 8, false><<<grid, kThreads, 0, stream>>>(g, nullptr, 0);
   return cudaGetLastError();
 }
 
 }  // namespace
 
-Fp64Form fp64_form(int dtype, int64_t M, int64_t N, int64_t K, int64_t forced) {
-  // Clocks of the busiest SM: whole blocks per SM times a block's FMAs at two
-  // per clock (four per complex product), plus 2000 for the fill of the copy
-  // ring and the epilogue, plus, when split, 6000 for the reduction launch
-  // and 1 per 8 bytes x SM of partials written and read back.
+SmallForm small_form(int dtype, int64_t M, int64_t N, int64_t K, int64_t forced) {
+  const bool cplx = dtype == T1M_COMPLEX128 || dtype == T1M_COMPLEX64;
+  const bool wide = dtype == T1M_FLOAT64 || dtype == T1M_COMPLEX128;
+  const double es = (cplx ? 2 : 1) * (wide ? 8 : 4);
   constexpr double kSms = 152;
-  const double fma = dtype == T1M_COMPLEX128 ? 4 : 1, es = dtype == T1M_COMPLEX128 ? 16 : 8;
-  const int64_t ksteps = std::max<int64_t>(1, (K + kBK64 - 1) / kBK64);
-  Fp64Form best{16, 1, ksteps * kBK64};
+  const int64_t ksteps = std::max<int64_t>(1, (K + kBK - 1) / kBK);
+  SmallForm best{16, 1};
   double best_cost = 1e300;
-  for (int tile : {16, 8}) {
-    const double tiles = double((M + tile - 1) / tile) * double((N + tile - 1) / tile);
-    for (int64_t s = forced > 0 ? forced : 1; s <= (forced > 0 ? forced : 64); ++s) {
-      if (s > 1 && s > ksteps) break;
-      const int64_t per = (ksteps + s - 1) / s;
-      const int64_t used = (ksteps + per - 1) / per;
-      if (forced <= 0 && used != s) continue;  // the same partition as a smaller s
-      const double waves = double(static_cast<int64_t>((tiles * used + kSms - 1) / kSms));
-      double cost = waves * tile * tile * double(std::min(K, per * kBK64)) * fma / 2 + 2000;
-      if (used > 1) cost += 6000 + 2.0 * double(used) * double(M) * double(N) * es / (8 * kSms);
-      if (cost < best_cost) {
-        best_cost = cost;
-        best = {tile, static_cast<int>(used), per * kBK64};
-      }
+  // Clocks of the busiest SM: whole blocks per SM times a block's k steps,
+  // plus 2000 for the fill of the copy ring and the epilogue, plus, when
+  // split, 6000 for the reduction launch and 1 per 8 bytes x SM of partials
+  // written and read back.
+  auto consider = [&](int tile, double tiles, double per_k, double floor_k, int64_t s) {
+    const int64_t per = (ksteps + s - 1) / s;
+    const int64_t used = (ksteps + per - 1) / per;
+    if (forced <= 0 && used != s) return;  // the same partition as a smaller s
+    const double waves = double(static_cast<int64_t>((tiles * used + kSms - 1) / kSms));
+    const double k = double(std::min(K, per * kBK));
+    double cost = std::max(waves * per_k, floor_k) * k + 2000;
+    if (used > 1) cost += 6000 + 2.0 * double(used) * double(M) * double(N) * es / (8 * kSms);
+    if (cost < best_cost) {
+      best_cost = cost;
+      best = {tile, static_cast<int>(used)};
+    }
+  };
+  for (int64_t s = forced > 0 ? forced : 1; s <= (forced > 0 ? forced : 64); ++s) {
+    if (s > 1 && s > ksteps) break;
+    for (int tile : {16, 8}) {
+      const double tiles = double((M + tile - 1) / tile) * double((N + tile - 1) / tile);
+      // A block's clocks per k: its FMAs (FP64: two per clock, four per
+      // complex product) or the shared-memory reads of its four warps; a
+      // stage of 16 k takes at least its latency.
+      const double per_k = wide ? double(tile) * tile * (cplx ? 4 : 1) / 2 : (tile == 16 ? 18 : 9);
+      consider(tile, tiles, per_k, wide ? 0 : 20, s);
+    }
+    if (!wide) {
+      // simt.cu's tile: 8192 (complex, four FMAs) or 16384 products per k on
+      // 128 lanes, two blocks per SM.
+      const double tiles = cplx ? double((M + 63) / 64) * double((N + 127) / 128)
+                                : double((M + 127) / 128) * double((N + 127) / 128);
+      consider(0, tiles, cplx ? 256 : 128, cplx ? 256 : 128, s);
     }
   }
   return best;
 }
 
-cudaError_t launch_fp64(int dtype, const GemmArgs& g, int splits, cudaStream_t stream) {
-  const int tile = fp64_form(dtype, g.M, g.N, g.K, splits).tile;
-  return dtype == T1M_COMPLEX128 ? launch<double2>(g, tile, splits, stream)
-                                 : launch<double>(g, tile, splits, stream);
+cudaError_t launch_small(int dtype, int tile, const GemmArgs& g, int splits, cudaStream_t stream) {
+  switch (dtype) {
+    case T1M_FLOAT32: return launch<float>(g, tile, splits, stream);
+    case T1M_FLOAT64: return launch<double>(g, tile, splits, stream);
+    case T1M_COMPLEX64: return launch<float2>(g, tile, splits, stream);
+    default: return launch<double2>(g, tile, splits, stream);
+  }
 }
 
 cudaError_t launch_fp64_group(int dtype, const SimtProblem* dev, int nprob, int64_t total_tiles,
@@ -291,9 +318,9 @@ cudaError_t launch_fp64_group(int dtype, const SimtProblem* dev, int nprob, int6
   const GemmArgs none{};
   const unsigned grid = static_cast<unsigned>(total_tiles);
   if (dtype == T1M_COMPLEX128)
-    fp64_contract<double2, kFp64Tile, true><<<grid, kThreads64, 0, stream>>>(none, dev, nprob);
+    small_contract<double2, kFp64Tile, true><<<grid, kThreads, 0, stream>>>(none, dev, nprob);
   else
-    fp64_contract<double, kFp64Tile, true><<<grid, kThreads64, 0, stream>>>(none, dev, nprob);
+    small_contract<double, kFp64Tile, true><<<grid, kThreads, 0, stream>>>(none, dev, nprob);
   return cudaGetLastError();
 }
 

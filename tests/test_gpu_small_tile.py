@@ -1,8 +1,8 @@
-"""The plain kernel of float64 / complex128 (fp64.cu) at the edges of its
-16 x 16 and 8 x 8 tiles, its 16-k stages and its k slices, split and unsplit,
-against an extended-precision product.  Elementwise bound: a sum of K products
-in any order differs from the exact one by at most about (4 K + 8) u |A||B|
-(four real products per complex term), u = 2^-53.
+"""The small output tiles (small_tile.cu) of the plain method at the edges of
+the 16 x 16 and 8 x 8 tiles, the 16-k stages and the k slices, split and
+unsplit, against an extended-precision product.  Elementwise bound: a sum of K
+products in any order differs from the exact one by at most about (4 K + 8) u
+|A||B| (four real products per complex term), u = 2^-53 or 2^-24.
 """
 import numpy as np
 import pytest
@@ -15,9 +15,9 @@ SHAPES = [(1, 1, 1), (8, 8, 16), (9, 7, 17), (16, 16, 15), (17, 33, 47), (31, 5,
 
 @pytest.mark.parametrize("splits", [0, 3])
 @pytest.mark.parametrize("layout", ["row", "col"])
-@pytest.mark.parametrize("dt", [np.float64, np.complex128])
+@pytest.mark.parametrize("dt", [np.float64, np.complex128, np.float32, np.complex64])
 @pytest.mark.parametrize("shape", SHAPES, ids=lambda s: "x".join(map(str, s)))
-def test_fp64_edges(ctx, torch_cuda, shape, dt, layout, splits):
+def test_small_tile_edges(ctx, torch_cuda, shape, dt, layout, splits):
     import t1m_gb300 as t1m
     torch = torch_cuda
     M, N, K = shape
@@ -25,12 +25,13 @@ def test_fp64_edges(ctx, torch_cuda, shape, dt, layout, splits):
 
     def rand(*s):
         x = rng.uniform(-1, 1, s)
-        return x + 1j * rng.uniform(-1, 1, s) if dt == np.complex128 else x
+        return (x + 1j * rng.uniform(-1, 1, s) if conj else x).astype(dt)
+
+    conj = np.dtype(dt).kind == "c"
 
     A, B, C = rand(M, K), rand(K, N), rand(M, N)
     order = "C" if layout == "row" else "F"
     L = t1m.row_major if layout == "row" else t1m.col_major
-    conj = dt == np.complex128
     alpha, beta = (0.5 - 1j, 0.25) if conj else (0.5, 0.25)
     ga, gb, gc = (torch.from_numpy(np.ravel(x, order=order).copy()).cuda() for x in (A, B, C))
     ctx.set_method("plain")
@@ -46,5 +47,5 @@ def test_fp64_edges(ctx, torch_cuda, shape, dt, layout, splits):
     Aw = np.conj(A) if conj else A
     ref = wide(alpha) * (Aw.astype(wide) @ B.astype(wide)) + wide(beta) * C.astype(wide)
     got = gc.cpu().numpy().reshape((M, N), order=order)
-    bound = (4 * K + 8) * 2.0 ** -53 * (abs(alpha) * (abs(A) @ abs(B)) * 2 + abs(beta) * abs(C) * 2)
+    bound = (4 * K + 8) * np.finfo(dt).eps / 2 * (abs(alpha) * (abs(A) @ abs(B)) * 2 + abs(beta) * abs(C) * 2)
     assert np.all(np.abs(got - ref.astype(dt)) <= bound)
