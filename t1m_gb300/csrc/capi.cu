@@ -21,6 +21,7 @@
 #include <unordered_map>
 
 #include "internal.h"
+#include "stream.h"
 #include "t1m_capi.h"
 
 using namespace t1m::gb300;
@@ -197,7 +198,9 @@ std::string plan_key(int dtype, const t1m_tensor* a, const int64_t* sa, const ch
 }
 
 int upload_plan(t1m_context* ctx, const HostPlan& hp, DevicePlan* dp) {
-  const std::vector<int64_t>* vs[6] = {&hp.rsA, &hp.csA, &hp.rsB, &hp.csB, &hp.rsC, &hp.csC};
+  constexpr int kVectors = 8;
+  const std::vector<int64_t>* vs[kVectors] = {&hp.rsA, &hp.csA, &hp.rsB,       &hp.csB,
+                                              &hp.rsC, &hp.csC, &hp.stream_ka, &hp.stream_kb};
   size_t total = 0;
   for (auto* v : vs) total += (v->size() + 1) * sizeof(int64_t);
   void* block = nullptr;
@@ -205,9 +208,9 @@ int upload_plan(t1m_context* ctx, const HostPlan& hp, DevicePlan* dp) {
   if (e != cudaSuccess) return fail(ctx, T1M_ERR_ALLOC, std::string("plan allocation: ") + cudaGetErrorString(e));
   std::vector<int64_t> host;
   host.reserve(total / sizeof(int64_t));
-  const int64_t* ptrs[6];
+  const int64_t* ptrs[kVectors];
   size_t off = 0;
-  for (int i = 0; i < 6; ++i) {
+  for (int i = 0; i < kVectors; ++i) {
     ptrs[i] = static_cast<const int64_t*>(block) + off;
     host.insert(host.end(), vs[i]->begin(), vs[i]->end());
     host.push_back(0);
@@ -222,6 +225,8 @@ int upload_plan(t1m_context* ctx, const HostPlan& hp, DevicePlan* dp) {
   dp->bytes = total;
   dp->rsA = ptrs[0]; dp->csA = ptrs[1]; dp->rsB = ptrs[2];
   dp->csB = ptrs[3]; dp->rsC = ptrs[4]; dp->csC = ptrs[5];
+  dp->stream_ka = hp.stream_ka.empty() ? nullptr : ptrs[6];
+  dp->stream_kb = hp.stream_kb.empty() ? nullptr : ptrs[7];
   return T1M_OK;
 }
 
@@ -380,6 +385,16 @@ int launch_product(t1m_context* ctx, int method, int dtype, size_t es, const Hos
                                          ctx->method == T1M_METHOD_AUTO)
                          : 1;
     int form = ctx->tile_form;
+    // Small outputs over long bundles stream both operands once.
+    int64_t stream_kps = 0;
+    const int stream_s = allow_split && method == kMethodTcAuto && dtype == T1M_COMPLEX64 &&
+                                 ctx->split_k == 0 && form == T1M_TILE_AUTO && !ctx->autotune
+                             ? stream_splits(g.M, g.N, g.K, &stream_kps)
+                             : 0;
+    if (stream_s > 0) {
+      splits = stream_s;
+      kps = stream_kps;
+    }
     if (allow_split && ctx->autotune && ctx->split_k == 0 && ctx->tile_form == T1M_TILE_AUTO &&
         method != T1M_METHOD_PLAIN && method != T1M_METHOD_DMMA) {
       int tf = 0, ts = 0;
@@ -412,6 +427,16 @@ int launch_product(t1m_context* ctx, int method, int dtype, size_t es, const Hos
       e = launch_simt(dtype, gm, splits, s, &nk);
     } else if (method == T1M_METHOD_DMMA) {
       e = launch_dmma(dtype, gm, splits, s, &nk);
+    } else if (stream_s > 0) {
+      if (ctx->mev_armed) cudaEventRecord(ctx->mev[0], s);
+      e = launch_stream(gm, stream_layout(gm, hp), splits, s, ctx->d_err);
+      if (ctx->mev_armed) {
+        cudaEventRecord(ctx->mev[1], s);
+        ctx->mev_recorded = e == cudaSuccess;
+      }
+      nk = 1;
+      *used_method = T1M_METHOD_TC_BF16X6;
+      ctx->last_path = T1M_PATH_TC;  // both operands gathered
     } else {
       std::string err;
       int ran = method;
@@ -1059,6 +1084,8 @@ int t1m_contract(t1m_context* ctx, int dtype, const void* alpha, const t1m_tenso
     if (st != T1M_OK) return fail(ctx, st, err);
     st = upload_plan(ctx, fresh.host, &fresh.dev);
     if (st != T1M_OK) return st;
+    fresh.host.dev_stream_ka = fresh.dev.stream_ka;
+    fresh.host.dev_stream_kb = fresh.dev.stream_kb;
     ctx->plans.push_front(std::move(fresh));
     ctx->index[key] = ctx->plans.begin();
     entry = &*ctx->plans.begin();

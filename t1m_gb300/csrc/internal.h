@@ -50,6 +50,12 @@ struct HostPlan {
   int64_t uA_m = -1, uA_k = -1, uB_k = -1, uB_n = -1, uC_m = -1, uC_n = -1;
   // Number of elements each tensor spans in memory (1 + sum (e-1)*s).
   int64_t spanA = 0, spanB = 0, spanC = 0;
+  // K offsets of A and B in an order that interleaves A's and B's unit-stride
+  // K modes (4 x 8 or 8 x 4 elements first), where they are different modes of
+  // such extents: a run of 32 k is then whole 32-byte sectors of both
+  // (stream.cu).  Empty otherwise.  dev_*: their device copies.
+  std::vector<int64_t> stream_ka, stream_kb;
+  const int64_t *dev_stream_ka = nullptr, *dev_stream_kb = nullptr;
   // Derived once per plan (the context caches plans across calls): results
   // of the tensor-core path's layout checks over the scatter vectors, keyed
   // by check and length, and the plans with densely packed operands (index
@@ -84,7 +90,7 @@ struct DevicePlan {
   void* block = nullptr;
   size_t bytes = 0;
   const int64_t *rsA = nullptr, *csA = nullptr, *rsB = nullptr, *csB = nullptr,
-                *rsC = nullptr, *csC = nullptr;
+                *rsC = nullptr, *csC = nullptr, *stream_ka = nullptr, *stream_kb = nullptr;
 };
 
 // Kernel arguments of one contraction launch (plain or tensor-core).

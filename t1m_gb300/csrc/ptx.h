@@ -67,12 +67,6 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
   return true;
 }
 
-// Programmatic dependent launch: wait until the kernels this one depends on
-// have finished and their writes are visible (returns at once otherwise).
-__device__ __forceinline__ void grid_dependency_wait() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-
 // Per-warpgroup register budget (every warp of the warpgroup executes it).
 template <uint32_t kRegs>
 __device__ __forceinline__ void regs_dec() {
@@ -317,6 +311,15 @@ __device__ __forceinline__ void mma_f16_ts2(uint32_t d_tmem, uint32_t a_tmem, ui
       "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
       " tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n}" ::"r"(d_tmem),
       "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// One CTA: both operands from its shared memory.
+__device__ __forceinline__ void mma_f16_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
+                                           uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(d_tmem),
+      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 // Both operands from shared memory (descriptors): A's 128 rows of each CTA

@@ -33,6 +33,7 @@ __global__ void __launch_bounds__(kThreads, 2)
 simt_contract(const GemmArgs args0, const SimtProblem* group, int nprob) {
   constexpr int BM = 16 * TM;
   constexpr int BN = 16 * TN;
+  begin_dependent();
   int64_t tile = blockIdx.x;
   // The contraction of this CTA: a shared-memory copy of its descriptor for
   // grouped launches, the parameter space otherwise.
@@ -227,8 +228,8 @@ cudaError_t launch(const GemmArgs& args, int splits, cudaStream_t stream) {
   if (tiles > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
   if (splits < 1 || splits > 65535) return cudaErrorInvalidConfiguration;
   const dim3 grid(static_cast<unsigned>(tiles), static_cast<unsigned>(splits));
-  simt_contract<T, TM, TN, BK, false><<<grid, kThreads, 0, stream>>>(args, nullptr, 0);
-  return cudaGetLastError();
+  return launch_dependent(simt_contract<T, TM, TN, BK, false>, grid, dim3(kThreads), 0, stream, args,
+                          nullptr, 0);
 }
 
 template <class T, int TM, int TN, int BK>
@@ -237,9 +238,8 @@ cudaError_t launch_group(const SimtProblem* dev, int nprob, int64_t total_tiles,
   if (total_tiles <= 0) return cudaSuccess;
   if (total_tiles > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
   GemmArgs none{};
-  simt_contract<T, TM, TN, BK, true><<<static_cast<unsigned>(total_tiles), kThreads, 0, stream>>>(
-      none, dev, nprob);
-  return cudaGetLastError();
+  return launch_dependent(simt_contract<T, TM, TN, BK, true>, dim3(static_cast<unsigned>(total_tiles)),
+                          dim3(kThreads), 0, stream, none, dev, nprob);
 }
 
 // ------------------------------------------------------------- skinny ---
@@ -564,6 +564,7 @@ skinny_contract(const SimtProblem* group, int nprob) {
   extern __shared__ __align__(16) unsigned char skinny_dsmem[];
   T (*Bs)[2048 / NMAX] = reinterpret_cast<T (*)[2048 / NMAX]>(skinny_dsmem);
   int64_t* ks = reinterpret_cast<int64_t*>(skinny_dsmem + size_t(NMAX) * (2048 / NMAX) * sizeof(T));
+  begin_dependent();
   int64_t tile = blockIdx.x;
   const int lo = block_find(nprob, tile, [&](int i) { return group[i].tile_begin; });
   tile -= group[lo].tile_begin;
@@ -601,9 +602,8 @@ cudaError_t launch_skinny(const SimtProblem* dev, int nprob, int64_t total_tiles
       attr_set = true;
     }
   }
-  skinny_contract<T, NMAX><<<static_cast<unsigned>(total_tiles), kThreads, kDyn, stream>>>(
-      dev, nprob);
-  return cudaGetLastError();
+  return launch_dependent(skinny_contract<T, NMAX>, dim3(static_cast<unsigned>(total_tiles)),
+                          dim3(kThreads), kDyn, stream, dev, nprob);
 }
 
 template <int NMAX>

@@ -220,6 +220,7 @@ __global__ void __launch_bounds__(kThreads)
 small_contract(const GemmArgs args0, const SimtProblem* group, int nprob) {
   __shared__ __align__(16) SmallSmem<T, kTile> sm;
   __shared__ GemmArgs group_args;
+  begin_dependent();
   int64_t tile = blockIdx.x, split = blockIdx.y;
   if constexpr (kGroup) {
     int lo = 0, hi = nprob - 1;
@@ -247,11 +248,8 @@ cudaError_t launch(const GemmArgs& g, int tile, int splits, cudaStream_t stream)
   if (tiles == 0) return cudaSuccess;
   if (tiles > 0x7fffffffLL || splits < 1 || splits > 65535) return cudaErrorInvalidConfiguration;
   const dim3 grid(static_cast<unsigned>(tiles), static_cast<unsigned>(splits));
-  if (tile == 16)
-    small_contract<T, 16, false><<<grid, kThreads, 0, stream>>>(g, nullptr, 0);
-  else
-    small_contract<T, 8, false><<<grid, kThreads, 0, stream>>>(g, nullptr, 0);
-  return cudaGetLastError();
+  return launch_dependent(tile == 16 ? small_contract<T, 16, false> : small_contract<T, 8, false>,
+                          grid, dim3(kThreads), 0, stream, g, nullptr, 0);
 }
 
 }  // namespace
@@ -316,12 +314,12 @@ cudaError_t launch_fp64_group(int dtype, const SimtProblem* dev, int nprob, int6
   if (total_tiles <= 0) return cudaSuccess;
   if (total_tiles > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
   const GemmArgs none{};
-  const unsigned grid = static_cast<unsigned>(total_tiles);
-  if (dtype == T1M_COMPLEX128)
-    small_contract<double2, kFp64Tile, true><<<grid, kThreads, 0, stream>>>(none, dev, nprob);
-  else
-    small_contract<double, kFp64Tile, true><<<grid, kThreads, 0, stream>>>(none, dev, nprob);
-  return cudaGetLastError();
+  const dim3 grid(static_cast<unsigned>(total_tiles));
+  return dtype == T1M_COMPLEX128
+             ? launch_dependent(small_contract<double2, kFp64Tile, true>, grid, dim3(kThreads), 0,
+                                stream, none, dev, nprob)
+             : launch_dependent(small_contract<double, kFp64Tile, true>, grid, dim3(kThreads), 0,
+                                stream, none, dev, nprob);
 }
 
 }  // namespace gb300

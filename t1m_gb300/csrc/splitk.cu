@@ -14,15 +14,12 @@
 #include <algorithm>
 #include <cstdint>
 
+#include "device_common.h"
 #include "internal.h"
 
 namespace t1m {
 namespace gb300 {
 namespace {
-
-__device__ __forceinline__ int64_t offs(const int64_t* v, int64_t u, int64_t i) {
-  return u >= 0 ? i * u : __ldg(v + i);
-}
 
 template <class W> struct Wide;
 template <> struct Wide<float> {
@@ -84,6 +81,7 @@ template <class T>
 __global__ void __launch_bounds__(256)
 splitk_reduce(const T* __restrict__ work, int splits, int G, const GemmArgs out) {
   __shared__ double2 part[8][32];
+  begin_dependent();
   const int64_t MN = out.M * out.N;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = warp % G, sub = warp / G, per = 8 / G;
@@ -122,6 +120,7 @@ template <class T>
 __global__ void __launch_bounds__(256)
 splitk_reduce_group(const SplitReduce* __restrict__ probs, int n, int64_t total) {
   __shared__ double2 part[8][32];
+  begin_dependent();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t nchunks = (total + 31) / 32;
   for (int64_t c = blockIdx.x; c < nchunks; c += gridDim.x) {
@@ -163,8 +162,8 @@ template <class T>
 cudaError_t launch_group(const SplitReduce* dev, int n, int64_t total, cudaStream_t stream) {
   if (total <= 0 || n <= 0) return cudaSuccess;
   const int64_t blocks = std::min<int64_t>((total + 31) / 32, 152 * 8);
-  splitk_reduce_group<T><<<static_cast<unsigned>(blocks), 256, 0, stream>>>(dev, n, total);
-  return cudaGetLastError();
+  return launch_dependent(splitk_reduce_group<T>, dim3(static_cast<unsigned>(blocks)), dim3(256), 0,
+                          stream, dev, n, total);
 }
 
 template <class T>
@@ -174,9 +173,8 @@ cudaError_t launch(const void* work, int splits, const GemmArgs& out, cudaStream
   const int G = splits <= 2 ? 2 : splits <= 4 ? 4 : 8;
   const int64_t chunks = (mn + 31) / 32;
   const int64_t blocks = std::min<int64_t>((chunks + 8 / G - 1) / (8 / G), 152 * 8);
-  splitk_reduce<T><<<static_cast<unsigned>(blocks), 256, 0, stream>>>(
-      static_cast<const T*>(work), splits, G, out);
-  return cudaGetLastError();
+  return launch_dependent(splitk_reduce<T>, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, stream,
+                          static_cast<const T*>(work), splits, G, out);
 }
 
 }  // namespace

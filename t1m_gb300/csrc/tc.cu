@@ -67,6 +67,7 @@
 #include "internal.h"
 #include "pieces.h"
 #include "ptx.h"
+#include "stream.h"
 #include "t1m_capi.h"
 #include "tc.h"
 #include "tc_common.h"
@@ -2632,6 +2633,18 @@ static void pieces_problem(int dtype, const GemmArgs& g, const HostPlan& plan, b
   p->g.flags &= ~(kFlagCPairs | kFlagCCol16);
   const std::vector<int64_t>&r = swap ? plan.csC : plan.rsC, &c = swap ? plan.rsC : plan.csC;
   p->g.flags |= dtype == T1M_FLOAT32 ? c_store_flags_real(p->g, r, c) : c_store_flags(p->g, r, c);
+}
+
+StreamLayout stream_layout(const GemmArgs& g, const HostPlan& plan) {
+  StreamLayout l{};
+  l.a_rows = pack_step(plan.modes_k, false, plan.modes_m) == 0;
+  l.b_rows = pack_step(plan.modes_k, true, plan.modes_n) == 0;
+  l.a_k = plan.dev_stream_ka;
+  l.b_k = plan.dev_stream_kb;
+  PieceProblem p{};
+  pieces_problem(T1M_COMPLEX64, g, plan, g.N < g.M, &p);
+  l.store_flags = p.g.flags & (kFlagCPairs | kFlagCCol16);
+  return l;
 }
 
 void tc_piece_item(const GemmArgs& g, const HostPlan& plan, int splits, PieceItem* it) {
