@@ -174,10 +174,10 @@ inline uint32_t small_tile_flag(int tile) {
 }
 cudaError_t launch_small(int dtype, int tile, const GemmArgs& args, int splits,
                          cudaStream_t stream);
-constexpr int kFp64Tile = 16;  // tile of grouped launches
+constexpr int kSmallTile = 16;  // tile of grouped launches
 struct SimtProblem;
-cudaError_t launch_fp64_group(int dtype, const SimtProblem* dev, int nprob, int64_t total_tiles,
-                              cudaStream_t stream);
+cudaError_t launch_small_group(int dtype, const SimtProblem* dev, int nprob, int64_t total_tiles,
+                               cudaStream_t stream);
 
 // One contraction of a grouped plain launch (device array, sorted by
 // tile_begin).  Its tiles are numbered split-major: g.k_per_split and

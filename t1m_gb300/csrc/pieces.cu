@@ -114,8 +114,11 @@ split_pieces(const SplitPair pair, const PieceSplit* dev, int n) {
   constexpr int KB = split_k<kReal>();
   __shared__ T tile[kSplitRowsPer][KB + 1];
   __shared__ PieceSplit so;
+  // The kernels ahead have finished once a block is past its wait: then the
+  // next kernel may start (a second split reads and writes other memory).
+  const bool beside = !dev && pair.op[0].beside;
+  if (!beside) begin_dependent();
   release_dependents();
-  begin_dependent();
   if (dev) {
     const int lo = block_find(n, blockIdx.x, [&](int i) { return dev[i].block_begin; });
     block_copy(&so, dev + lo);
@@ -160,20 +163,23 @@ split_pieces(const SplitPair pair, const PieceSplit* dev, int n) {
   const int c = t & 3, r = (t >> 2) & 31, st = t >> 7;
   constexpr int kStageE = kReal ? 32 : 16;  // elements per stage
   const int64_t ks = k0 / kStageE + st;
-  if (r0 + r >= o.R || ks * kStageE >= o.K) return;
-  float v[8];
-  constexpr int kChunkE = kReal ? 8 : 4;
+  if (r0 + r < o.R && ks * kStageE < o.K) {
+    float v[8];
+    constexpr int kChunkE = kReal ? 8 : 4;
 #pragma unroll
-  for (int j = 0; j < kChunkE; ++j) {
-    const T x = tile[r][st * kStageE + c * kChunkE + j];
-    if constexpr (kReal) {
-      v[j] = x;
-    } else {
-      v[2 * j] = x.x;
-      v[2 * j + 1] = x.y;
+    for (int j = 0; j < kChunkE; ++j) {
+      const T x = tile[r][st * kStageE + c * kChunkE + j];
+      if constexpr (kReal) {
+        v[j] = x;
+      } else {
+        v[2 * j] = x.x;
+        v[2 * j + 1] = x.y;
+      }
     }
+    split_row_chunk<P, kReal>(o, ks, r0 + r, c, v);
   }
-  split_row_chunk<P, kReal>(o, ks, r0 + r, c, v);
+  // This kernel's end stands for the other split's too.
+  if (beside) begin_dependent();
 }
 
 // kSplitStep: the source is contiguous along k_hi (k = k_lo + step * k_hi).
@@ -188,8 +194,8 @@ split_pieces_step(const PieceSplit o) {
   // stores along k_hi nor the chunk reads conflict.
   constexpr int kRow = KL + 1, kPlane = R * kRow + 1;
   __shared__ T tile[KH * kPlane];
+  if (!o.beside) begin_dependent();
   release_dependents();
-  begin_dependent();
   const int64_t nhi = o.K / o.step, nlo = o.step / KL;
   const int64_t hblocks = (nhi + KH - 1) / KH;
   int64_t b = blockIdx.x;
@@ -211,12 +217,11 @@ split_pieces_step(const PieceSplit o) {
   }
   __syncthreads();
   const int c = lane & 3, r = lane >> 2;
-  if (r0 + r >= o.R) return;
   constexpr int kChunkE = kReal ? 8 : 4;
 #pragma unroll
   for (int i = 0; i < KH / 8; ++i) {
     const int h = warp + 8 * i;
-    if (h0 + h >= nhi) break;
+    if (h0 + h >= nhi || r0 + r >= o.R) break;
     const T* s = tile + h * kPlane + r * kRow + c * kChunkE;
     float v[8];
 #pragma unroll
@@ -230,6 +235,7 @@ split_pieces_step(const PieceSplit o) {
     }
     split_row_chunk<P, kReal>(o, (l0 + o.step * (h0 + h)) / KL, r0 + r, c, v);
   }
+  if (o.beside) begin_dependent();
 }
 
 // ---------------------------------------------------------------- product ---

@@ -46,7 +46,9 @@ struct PieceSplit {
   int32_t expand;          // complex A: the two 1M rows of every row
   int32_t conj;
   int32_t mode;
-  int32_t pad;
+  // Runs beside the split launched just before it, whose blocks let it start
+  // once everything ahead of both has finished: it waits at its end instead.
+  int32_t beside;
 };
 
 // One product over pieces.  g: C, its offsets and epilogue, M, N, K,

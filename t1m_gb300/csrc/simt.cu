@@ -665,7 +665,7 @@ cudaError_t launch_simt_group(int dtype, bool skinny, const SimtProblem* dev, in
     return cudaErrorInvalidValue;
   }
   switch (dtype) {
-    case 1: case 3: return launch_fp64_group(dtype, dev, nprob, total_tiles, stream);
+    case 1: case 3: return launch_small_group(dtype, dev, nprob, total_tiles, stream);
     case 0: return launch_group<float, 8, 8, 8>(dev, nprob, total_tiles, stream);
     case 2: return launch_group<float2, 4, 8, 8>(dev, nprob, total_tiles, stream);
   }
@@ -676,7 +676,7 @@ void simt_tile(int dtype, int* bm, int* bn, int* bk) {
   switch (dtype) {
     case 0: *bm = 128; *bn = 128; break;
     case 2: *bm = 64; *bn = 128; break;
-    default: *bm = *bn = kFp64Tile; *bk = 16; return;
+    default: *bm = *bn = kSmallTile; *bk = 16; return;
   }
   *bk = 8;
 }

@@ -36,7 +36,10 @@ namespace {
 
 constexpr int kThreads = 128;
 constexpr int kBK = 16;      // k per stage
-constexpr int kStages = 3;
+// Stages of the copy ring: a small block's time is the latency of its
+// copies, so as many as 48 KB of static shared memory hold.
+template <class T>
+constexpr int ring_stages() { return sizeof(T) == 16 ? 3 : 5; }
 
 __device__ __forceinline__ float flip(float v, uint64_t) { return v; }
 __device__ __forceinline__ float2 flip(float2 v, uint64_t sign) {
@@ -52,13 +55,19 @@ __device__ __forceinline__ double2 flip(double2 v, uint64_t sign) {
   return v;
 }
 
+// K offsets held in shared memory: looked up per stage, each stage waited for
+// its offsets before its copies could start (a 16 x 16 x 512 block: 52 us).
+constexpr int kOffsets = 512;
+
 template <class T, int kTile>
 struct SmallSmem {
   static constexpr int kPad = 32 / sizeof(T);
+  static constexpr int kStages = ring_stages<T>();
   T a[kStages][kBK][kTile + kPad];
   T b[kStages][kBK][kTile + kPad];
   T part[kTile * kTile];  // the second k slice's sums (8 x 8 form)
   int64_t row_a[kTile], col_b[kTile];
+  int64_t ka[kOffsets], kb[kOffsets];  // K offsets, a ring of two halves
 };
 
 // One output tile over the K range of `split`.  kTile: 16 or 8 rows and
@@ -98,21 +107,31 @@ __device__ __forceinline__ void small_tile(const GemmArgs& args, int64_t tile, i
     const int n = tid - kTile;
     colB[n] = n0 + n < N ? offs(args.csB, args.uB_n, n0 + n) : 0;
   }
-  __syncthreads();
 
   const bool a_kfast = args.uA_k == 1;
   const bool b_kfast = args.uB_k == 1 || args.uB_n != 1;
   constexpr int kPer = kTile * kBK / kThreads;
   static_assert(kPer * kThreads == kTile * kBK, "stage copies");
+  constexpr int kStages = ring_stages<T>();
+  // Offsets of k in [k0, k0 + n) into their places of the ring.
+  auto look = [&](int64_t k0, int n) {
+    for (int i = tid; i < n && k0 + i < K; i += kThreads) {
+      const int at = static_cast<int>((k0 + i - kb) % kOffsets);
+      sm.ka[at] = offs(args.csA, args.uA_k, k0 + i);
+      sm.kb[at] = offs(args.rsB, args.uB_k, k0 + i);
+    }
+  };
+  look(kb, kOffsets);
+  __syncthreads();
   auto issue = [&](int64_t k0, int buf) {
+    const int at = static_cast<int>((k0 - kb) % kOffsets);
 #pragma unroll
     for (int p = 0; p < kPer; ++p) {
       const int idx = tid + p * kThreads;
       const int m = a_kfast ? idx / kBK : idx % kTile;
       const int k = a_kfast ? idx % kBK : idx / kTile;
       const bool in = m0 + m < M && k0 + k < K;
-      cp_async_elem<sizeof(T)>(&As[buf][k][m],
-                               in ? A + rowA[m] + offs(args.csA, args.uA_k, k0 + k) : A, in);
+      cp_async_elem<sizeof(T)>(&As[buf][k][m], in ? A + rowA[m] + sm.ka[at + k] : A, in);
     }
 #pragma unroll
     for (int p = 0; p < kPer; ++p) {
@@ -120,8 +139,7 @@ __device__ __forceinline__ void small_tile(const GemmArgs& args, int64_t tile, i
       const int n = b_kfast ? idx / kBK : idx % kTile;
       const int k = b_kfast ? idx % kBK : idx / kTile;
       const bool in = n0 + n < N && k0 + k < K;
-      cp_async_elem<sizeof(T)>(&Bs[buf][k][n],
-                               in ? B + offs(args.rsB, args.uB_k, k0 + k) + colB[n] : B, in);
+      cp_async_elem<sizeof(T)>(&Bs[buf][k][n], in ? B + sm.kb[at + k] + colB[n] : B, in);
     }
   };
 
@@ -152,6 +170,10 @@ __device__ __forceinline__ void small_tile(const GemmArgs& args, int64_t tile, i
     cp_async_wait_group<kStages - 2>();
     __syncthreads();  // stage st has landed for every thread; stage st - 1 is consumed
     const int64_t nxt = st + kStages - 1;
+    // The copies enter a new half of the offsets: the other one is refilled
+    // (read again no earlier than 256 k later, stages of barriers away).
+    if (nxt * kBK % (kOffsets / 2) == 0 && nxt > 0)
+      look(kb + nxt * kBK + kOffsets / 2, kOffsets / 2);
     if (nxt < ksteps) issue(kb + nxt * kBK, static_cast<int>(nxt % kStages));
     cp_async_commit_group();
     const int kn = static_cast<int>(min(static_cast<int64_t>(kBK), K - kb - st * kBK));
@@ -309,17 +331,17 @@ cudaError_t launch_small(int dtype, int tile, const GemmArgs& g, int splits, cud
   }
 }
 
-cudaError_t launch_fp64_group(int dtype, const SimtProblem* dev, int nprob, int64_t total_tiles,
-                              cudaStream_t stream) {
+cudaError_t launch_small_group(int dtype, const SimtProblem* dev, int nprob, int64_t total_tiles,
+                               cudaStream_t stream) {
   if (total_tiles <= 0) return cudaSuccess;
   if (total_tiles > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
   const GemmArgs none{};
   const dim3 grid(static_cast<unsigned>(total_tiles));
-  return dtype == T1M_COMPLEX128
-             ? launch_dependent(small_contract<double2, kFp64Tile, true>, grid, dim3(kThreads), 0,
-                                stream, none, dev, nprob)
-             : launch_dependent(small_contract<double, kFp64Tile, true>, grid, dim3(kThreads), 0,
-                                stream, none, dev, nprob);
+  auto run = [&](auto kernel) {
+    return launch_dependent(kernel, grid, dim3(kThreads), 0, stream, none, dev, nprob);
+  };
+  return dtype == T1M_COMPLEX128 ? run(small_contract<double2, kSmallTile, true>)
+                                 : run(small_contract<double, kSmallTile, true>);
 }
 
 }  // namespace gb300

@@ -2697,6 +2697,7 @@ static cudaError_t launch_pieces(int method, int dtype, const GemmArgs& g, const
     ++*kernels;
   } else {
     for (int i = 0; i < n; ++i) {
+      ops[i].beside = i;
       const int64_t blocks = piece_split_blocks(real, ops[i]);
       e = launch_piece_split(P, real, &ops[i], 1, nullptr, blocks, stream);
       if (e != cudaSuccess) return e;
