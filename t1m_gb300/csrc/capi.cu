@@ -1981,7 +1981,7 @@ extern "C" int t1m_group_create(t1m_context* ctx, int dtype, int n, const t1m_gr
             piece_item_place(&pi, probe_pieces);
             le = cudaSuccess;
             for (int o = 0; o < 2 && le == cudaSuccess; ++o) {
-              const int64_t blocks = piece_split_blocks(false, pi.op[o]);
+              const int64_t blocks = piece_split_blocks(false, &pi.op[o]);
               le = launch_piece_split(3, false, &pi.op[o], 1, nullptr, blocks, ctx->stream);
             }
             if (le == cudaSuccess)
@@ -2180,7 +2180,7 @@ extern "C" int t1m_group_create(t1m_context* ctx, int dtype, int n, const t1m_gr
             PieceSplit& op = it.op[o];
             op.out = reinterpret_cast<uint8_t*>(used);  // offset until the workspace exists
             used += it.bytes[o];
-            const int64_t blocks = piece_split_blocks(false, op);
+            const int64_t blocks = piece_split_blocks(false, &op, true);
             if (op.mode == kSplitStep) {
               t1m_group::Launch T{kFamPieceStep, int64_t(g->steps.size()), 1, blocks};
               g->steps.push_back(op);

@@ -47,6 +47,28 @@ cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
 
+// Global -> shared copy of one element (4, 8 or 16 bytes) that does not pass
+// through registers; src_bytes 0 writes zeros (operands past the tile edge).
+template <int kBytes>
+__device__ __forceinline__ void cp_async_elem(void* dst, const void* src, bool in) {
+  const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
+  const uint32_t n = in ? kBytes : 0u;
+  if constexpr (kBytes == 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n)
+                 : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(d), "l"(src),
+                 "n"(kBytes), "r"(n)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async_commit_group() {
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+template <int N>
+__device__ __forceinline__ void cp_async_wait_group() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
 // Last of n descriptors (sorted by begin(i)) whose begin is at most x, found by
 // the whole block at once: a binary search is a chain of dependent loads that
 // a short block waits for (seven for a batch of 128).

@@ -103,72 +103,57 @@ constexpr int kSplitRowsPer = 32;                                // source rows 
 template <bool kReal>
 constexpr int split_k() { return kReal ? 64 : 32; }              // k per block: two stages
 
-// Blocks of 32 rows x two stages: read through shared memory along the
-// source's unit-stride direction, written as whole atoms (a warp writes the
-// four chunks of eight rows).  Bound by HBM; k past K is written as zeros, rows past
-// R are not written.
-template <int P, bool kReal>
-__global__ void __launch_bounds__(256)
+// Blocks of 32 rows x kper times two stages: read into shared memory along
+// the source's unit-stride direction, written as whole atoms (a warp writes
+// the four chunks of eight rows).  k past K is written as zeros, rows past R
+// are not written.  The next two stages are copied asynchronously while the
+// current ones are split: with two stages a block, its own start (finding the
+// operand, offsets) took longer than their data.  (Held in registers instead,
+// they left room for two to six blocks per SM of eight and the pass slowed
+// down by a third.)
+// kMany false: one k block (kper 1), eight blocks per SM, for operands that
+// leave no more than that to do.
+template <int P, bool kReal, bool kMany>
+__global__ void __launch_bounds__(256, kMany ? 6 : 8)
 split_pieces(const SplitPair pair, const PieceSplit* dev, int n) {
   using T = typename std::conditional<kReal, float, float2>::type;
   constexpr int KB = split_k<kReal>();
-  __shared__ T tile[kSplitRowsPer][KB + 1];
+  __shared__ T tile[kMany ? 2 : 1][kSplitRowsPer][KB + 1];
   __shared__ PieceSplit so;
   // The kernels ahead have finished once a block is past its wait: then the
   // next kernel may start (a second split reads and writes other memory).
   const bool beside = !dev && pair.op[0].beside;
   if (!beside) begin_dependent();
   release_dependents();
-  if (dev) {
+  if (kMany && dev) {
     const int lo = block_find(n, blockIdx.x, [&](int i) { return dev[i].block_begin; });
     block_copy(&so, dev + lo);
     __syncthreads();
   }
   const PieceSplit& o =
-      dev ? so : (pair.n > 1 && blockIdx.x >= pair.op[1].block_begin ? pair.op[1] : pair.op[0]);
+      kMany && dev ? so : (pair.n > 1 && blockIdx.x >= pair.op[1].block_begin ? pair.op[1] : pair.op[0]);
   // Block counts of a launch fit 32 bits (launch_piece_split).
   const int bid = static_cast<int>(blockIdx.x - o.block_begin);
-  const int kblocks = static_cast<int>((o.K + KB - 1) / KB);
+  const int kspan = kMany ? KB * o.kper : KB;
+  const int kblocks = static_cast<int>((o.K + kspan - 1) / kspan);
   const int rb = bid / kblocks;
-  const int64_t r0 = int64_t(rb) * kSplitRowsPer, k0 = int64_t(bid - rb * kblocks) * KB;
+  const int64_t r0 = int64_t(rb) * kSplitRowsPer, kbeg = int64_t(bid - rb * kblocks) * kspan;
+  const int64_t kend = min(o.K, kbeg + kspan);
   const T* __restrict__ src = static_cast<const T*>(o.src);
   const int t = threadIdx.x;
   constexpr int kPer = kSplitRowsPer * KB / 256;
-  if (o.mode == kSplitRows) {
-    const int r = t & 31;
-    const bool rin = r0 + r < o.R;
-    const T* __restrict__ row = src + (rin ? offs(o.ro, o.ur, r0 + r) : 0);
-#pragma unroll
-    for (int i = 0; i < kPer; ++i) {
-      const int k = (t >> 5) + 8 * i;
-      T v{};
-      if (rin && k0 + k < o.K) v = row[offs(o.ko, o.uk, k0 + k)];
-      tile[r][k] = v;
-    }
-  } else {
-    const int k = t & (KB - 1);
-    const bool kin = k0 + k < o.K;
-    const T* __restrict__ col = src + (kin ? offs(o.ko, o.uk, k0 + k) : 0);
-#pragma unroll
-    for (int i = 0; i < kPer; ++i) {
-      const int r = t / KB + (256 / KB) * i;
-      T v{};
-      if (kin && r0 + r < o.R) v = col[offs(o.ro, o.ur, r0 + r)];
-      tile[r][k] = v;
-    }
-  }
-  __syncthreads();
   // 32 rows x 8 chunks: thread t takes chunk t & 3 of row (t >> 2) & 31 in
-  // stage t >> 7 of the block's two.
+  // stage t >> 7 of the tile's two.
   const int c = t & 3, r = (t >> 2) & 31, st = t >> 7;
   constexpr int kStageE = kReal ? 32 : 16;  // elements per stage
-  const int64_t ks = k0 / kStageE + st;
-  if (r0 + r < o.R && ks * kStageE < o.K) {
+  constexpr int kChunkE = kReal ? 8 : 4;
+  auto put = [&](int64_t k0, int b) {
+    const int64_t ks = k0 / kStageE + st;
+    if (r0 + r >= o.R || ks * kStageE >= o.K) return;
     float v[8];
-    constexpr int kChunkE = kReal ? 8 : 4;
 #pragma unroll
     for (int j = 0; j < kChunkE; ++j) {
-      const T x = tile[r][st * kStageE + c * kChunkE + j];
+      const T x = tile[b][r][st * kStageE + c * kChunkE + j];
       if constexpr (kReal) {
         v[j] = x;
       } else {
@@ -177,6 +162,72 @@ split_pieces(const SplitPair pair, const PieceSplit* dev, int n) {
       }
     }
     split_row_chunk<P, kReal>(o, ks, r0 + r, c, v);
+  };
+  if constexpr (kMany) {
+    const bool by_rows = o.mode == kSplitRows;
+    auto fetch = [&](int64_t k0, int b) {
+      if (by_rows) {
+        const int r = t & 31;
+        const bool rin = r0 + r < o.R;
+        const T* __restrict__ row = src + (rin ? offs(o.ro, o.ur, r0 + r) : 0);
+#pragma unroll
+        for (int i = 0; i < kPer; ++i) {
+          const int k = (t >> 5) + 8 * i;
+          const bool in = rin && k0 + k < o.K;
+          cp_async_elem<sizeof(T)>(&tile[b][r][k], in ? row + offs(o.ko, o.uk, k0 + k) : src, in);
+        }
+      } else {
+        const int k = t & (KB - 1);
+        const bool kin = k0 + k < o.K;
+        const T* __restrict__ col = src + (kin ? offs(o.ko, o.uk, k0 + k) : 0);
+#pragma unroll
+        for (int i = 0; i < kPer; ++i) {
+          const int r = t / KB + (256 / KB) * i;
+          const bool in = kin && r0 + r < o.R;
+          cp_async_elem<sizeof(T)>(&tile[b][r][k], in ? col + offs(o.ro, o.ur, r0 + r) : src, in);
+        }
+      }
+      cp_async_commit_group();
+    };
+    fetch(kbeg, 0);
+    int b = 0;
+    for (int64_t k0 = kbeg; k0 < kend; k0 += KB, b ^= 1) {
+      if (k0 + KB < kend) {
+        fetch(k0 + KB, b ^ 1);
+        cp_async_wait_group<1>();
+      } else {
+        cp_async_wait_group<0>();
+      }
+      __syncthreads();
+      put(k0, b);
+      __syncthreads();  // this buffer is fetched into next
+    }
+  } else {
+    if (o.mode == kSplitRows) {
+      const int r = t & 31;
+      const bool rin = r0 + r < o.R;
+      const T* __restrict__ row = src + (rin ? offs(o.ro, o.ur, r0 + r) : 0);
+#pragma unroll
+      for (int i = 0; i < kPer; ++i) {
+        const int k = (t >> 5) + 8 * i;
+        T v{};
+        if (rin && kbeg + k < o.K) v = row[offs(o.ko, o.uk, kbeg + k)];
+        tile[0][r][k] = v;
+      }
+    } else {
+      const int k = t & (KB - 1);
+      const bool kin = kbeg + k < o.K;
+      const T* __restrict__ col = src + (kin ? offs(o.ko, o.uk, kbeg + k) : 0);
+#pragma unroll
+      for (int i = 0; i < kPer; ++i) {
+        const int r = t / KB + (256 / KB) * i;
+        T v{};
+        if (kin && r0 + r < o.R) v = col[offs(o.ro, o.ur, r0 + r)];
+        tile[0][r][k] = v;
+      }
+    }
+    __syncthreads();
+    put(kbeg, 0);
   }
   // This kernel's end stands for the other split's too.
   if (beside) begin_dependent();
@@ -815,19 +866,28 @@ cudaError_t launch_split_t(const PieceSplit* ops, int n, const PieceSplit* dev, 
     for (int i = 0; i < n; ++i) pair.op[i] = ops[i];
     pair.n = n;
   }
-  return launch_dependent(split_pieces<P, kReal>, dim3(static_cast<unsigned>(blocks)), dim3(256), 0,
-                          stream, pair, dev, n);
+  bool many = dev;
+  for (int i = 0; i < n && !dev; ++i) many = many || ops[i].kper > 1;
+  return launch_dependent(many ? split_pieces<P, kReal, true> : split_pieces<P, kReal, false>,
+                          dim3(static_cast<unsigned>(blocks)), dim3(256), 0, stream, pair, dev, n);
 }
 
 }  // namespace
 
-int64_t piece_split_blocks(bool real, const PieceSplit& s) {
-  if (s.mode == kSplitStep) {
-    const int64_t nhi = s.K / s.step, nlo = s.step / (real ? 32 : 16);
-    return (s.R + 7) / 8 * nlo * ((nhi + 31) / 32);
+int64_t piece_split_blocks(bool real, PieceSplit* s, bool batch) {
+  s->kper = 1;
+  if (s->mode == kSplitStep) {
+    const int64_t nhi = s->K / s->step, nlo = s->step / (real ? 32 : 16);
+    return (s->R + 7) / 8 * nlo * ((nhi + 31) / 32);
   }
   const int64_t kb = real ? split_k<true>() : split_k<false>();
-  return (s.R + kSplitRowsPer - 1) / kSplitRowsPer * ((s.K + kb - 1) / kb);
+  const int64_t rows = (s->R + kSplitRowsPer - 1) / kSplitRowsPer, kblocks = (s->K + kb - 1) / kb;
+  // Up to four k blocks a thread block, while the GPU (152 SMs x 8 blocks)
+  // keeps a round of them, counting four operands of a batch (4096^2 twice: 163 us with one, 140 with four;
+  // 1024^2: 9.5 us with one, 12.3 on the form for several).
+  s->kper = static_cast<int32_t>(
+      std::max<int64_t>(1, std::min<int64_t>(4, rows * kblocks / (batch ? 304 : 1216))));
+  return rows * ((kblocks + s->kper - 1) / s->kper);
 }
 
 cudaError_t launch_piece_split(int pieces, bool real, const PieceSplit* ops, int n,

@@ -49,6 +49,8 @@ struct PieceSplit {
   // Runs beside the split launched just before it, whose blocks let it start
   // once everything ahead of both has finished: it waits at its end instead.
   int32_t beside;
+  int32_t kper;            // two-stage k blocks of a thread block (piece_split_blocks)
+  int32_t pad;
 };
 
 // One product over pieces.  g: C, its offsets and epilogue, M, N, K,
@@ -79,8 +81,9 @@ void tc_piece_item(const GemmArgs& g, const HostPlan& plan, int splits, PieceIte
 // Put the item's pieces at ws (bytes[0] + bytes[1] bytes).
 void piece_item_place(PieceItem* it, void* ws);
 
-// Blocks of the split pass of one operand.
-int64_t piece_split_blocks(bool real, const PieceSplit& s);
+// Thread blocks of the split pass of one operand; sets its kper.  `batch`: one
+// of several operands in a launch.
+int64_t piece_split_blocks(bool real, PieceSplit* s, bool batch = false);
 // Split `n` operands in one launch (none of them kSplitStep when n > 1 or
 // dev is given): `ops` by value (n <= 2) or the device array `dev`.
 cudaError_t launch_piece_split(int pieces, bool real, const PieceSplit* ops, int n,

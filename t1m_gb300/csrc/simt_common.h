@@ -76,28 +76,6 @@ __device__ __forceinline__ double add(double a, double b) { return a + b; }
 __device__ __forceinline__ float2 add(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ double2 add(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
 
-// Global -> shared copy of one element (4, 8 or 16 bytes) that does not pass
-// through registers; src_bytes 0 writes zeros (operands past the tile edge).
-template <int kBytes>
-__device__ __forceinline__ void cp_async_elem(void* dst, const void* src, bool in) {
-  const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
-  const uint32_t n = in ? kBytes : 0u;
-  if constexpr (kBytes == 16)
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n)
-                 : "memory");
-  else
-    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(d), "l"(src),
-                 "n"(kBytes), "r"(n)
-                 : "memory");
-}
-__device__ __forceinline__ void cp_async_commit_group() {
-  asm volatile("cp.async.commit_group;" ::: "memory");
-}
-template <int N>
-__device__ __forceinline__ void cp_async_wait_group() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-
 }  // namespace
 }  // namespace gb300
 }  // namespace t1m

@@ -2553,7 +2553,7 @@ cudaError_t tc_split_operand(int dtype, int pieces, bool operand_a, const GemmAr
                              const HostPlan& plan, void* out, int64_t groups, cudaStream_t s) {
   PieceSplit op = piece_split_args(dtype, operand_a, false, g, plan, out, groups);
   const bool real = dtype == T1M_FLOAT32;
-  const int64_t blocks = piece_split_blocks(real, op);
+  const int64_t blocks = piece_split_blocks(real, &op);
   return launch_piece_split(pieces, real, &op, 1, nullptr, blocks, s);
 }
 
@@ -2690,15 +2690,15 @@ static cudaError_t launch_pieces(int method, int dtype, const GemmArgs& g, const
   const bool uniform = g.uA_m >= 0 && g.uA_k >= 0 && g.uB_k >= 0 && g.uB_n >= 0;
   cudaError_t e;
   if (n == 2 && uniform) {
-    ops[1].block_begin = piece_split_blocks(real, ops[0]);
-    const int64_t blocks = ops[1].block_begin + piece_split_blocks(real, ops[1]);
+    ops[1].block_begin = piece_split_blocks(real, &ops[0]);
+    const int64_t blocks = ops[1].block_begin + piece_split_blocks(real, &ops[1]);
     e = launch_piece_split(P, real, ops, 2, nullptr, blocks, stream);
     if (e != cudaSuccess) return e;
     ++*kernels;
   } else {
     for (int i = 0; i < n; ++i) {
       ops[i].beside = i;
-      const int64_t blocks = piece_split_blocks(real, ops[i]);
+      const int64_t blocks = piece_split_blocks(real, &ops[i]);
       e = launch_piece_split(P, real, &ops[i], 1, nullptr, blocks, stream);
       if (e != cudaSuccess) return e;
       ++*kernels;
