@@ -17,7 +17,7 @@
 // Steps past K are not computed, and a warp whose outputs all lie past the edge
 // computes nothing.
 // Measured (GB300): complex128 1024^3 8.23 -> 6.95 ms (1.24 TFLOP/s, 98% of
-// the two-FMA rate), float64 9216 x 96 x 96 281 -> 196 us a call.
+// the two-FMA rate), float64 9216 x 96 x 96 281 -> 190 us a call.
 //
 // Tiles are gathered through the scatter vectors as in simt.cu (the plain
 // form; replaces the reference's include/t1m/t1m.h:432-557 in FP64), each
@@ -25,6 +25,7 @@
 // three-stage cp.async ring.  Consecutive threads write along C's unit stride.
 #include <algorithm>
 #include <cstdint>
+#include <type_traits>
 
 #include "internal.h"
 #include "simt_common.h"
@@ -55,6 +56,48 @@ __device__ __forceinline__ double2 flip(double2 v, uint64_t sign) {
   return v;
 }
 
+// A sum of chains: FP32 values with the rounding errors of their additions
+// (Knuth's two-sum), so joining four short chains rounds once.  Plain
+// additions made outputs of few terms worse than one chain (float32, K = 5,
+// entries uniform in [-1, 1]: 5.0e-8 against 4.4e-8).  FP64 joins by plain
+// additions: two-sum would take the FP64 pipe longer than a small product.
+template <class T>
+struct ChainSum {
+  T v;
+  __device__ __forceinline__ void start(T x) { v = x; }
+  __device__ __forceinline__ void join(const ChainSum& o) { v = add(v, o.v); }
+  __device__ __forceinline__ T value() const { return v; }
+};
+__device__ __forceinline__ void two_sum(float& s, float& e, float x, float xe) {
+  const float t = __fadd_rn(s, x), u = __fsub_rn(t, s);
+  e = __fadd_rn(__fadd_rn(e, xe),
+                __fadd_rn(__fsub_rn(s, __fsub_rn(t, u)), __fsub_rn(x, u)));
+  s = t;
+}
+// An infinite, NaN or overflowing sum has no error term.
+__device__ __forceinline__ float two_value(float s, float e) {
+  return isfinite(e) ? __fadd_rn(s, e) : s;
+}
+template <>
+struct ChainSum<float> {
+  float v, e;
+  __device__ __forceinline__ void start(float x) { v = x; e = 0.f; }
+  __device__ __forceinline__ void join(const ChainSum& o) { two_sum(v, e, o.v, o.e); }
+  __device__ __forceinline__ float value() const { return two_value(v, e); }
+};
+template <>
+struct ChainSum<float2> {
+  float2 v, e;
+  __device__ __forceinline__ void start(float2 x) { v = x; e = make_float2(0.f, 0.f); }
+  __device__ __forceinline__ void join(const ChainSum& o) {
+    two_sum(v.x, e.x, o.v.x, o.e.x);
+    two_sum(v.y, e.y, o.v.y, o.e.y);
+  }
+  __device__ __forceinline__ float2 value() const {
+    return make_float2(two_value(v.x, e.x), two_value(v.y, e.y));
+  }
+};
+
 // K offsets held in shared memory: looked up per stage, each stage waited for
 // its offsets before its copies could start (a 16 x 16 x 512 block: 52 us).
 constexpr int kOffsets = 512;
@@ -65,7 +108,7 @@ struct SmallSmem {
   static constexpr int kStages = ring_stages<T>();
   T a[kStages][kBK][kTile + kPad];
   T b[kStages][kBK][kTile + kPad];
-  T part[kTile * kTile];  // the second k slice's sums (8 x 8 form)
+  ChainSum<T> part[kTile == 8 ? 64 : 1];  // the second k slice's sums (8 x 8 form)
   int64_t row_a[kTile], col_b[kTile];
   int64_t ka[kOffsets], kb[kOffsets];  // K offsets, a ring of two halves
 };
@@ -150,9 +193,17 @@ __device__ __forceinline__ void small_tile(const GemmArgs& args, int64_t tile, i
   bool live[kOut];
 #pragma unroll
   for (int j = 0; j < kOut; ++j) live[j] = f < fast_n && s + kSlow * j < slow_n;
-  // Four FMA chains per output (k mod 4, over the slices), added at the end:
-  // shorter chains than one per K range round less.
-  constexpr int kChains = 4 / kSlices;
+  // Several FMA chains per output (k modulo their number, over the slices),
+  // joined at the end: shorter chains than one per K range round less.  FP64
+  // takes eight, so that an unsplit K of 256 has chains of 32 terms.  Up to
+  // kSerial terms stay in one chain: there the products rounded apart and the
+  // sums that join them are more roundings than the chain's.
+  constexpr bool kWide = std::is_same_v<T, double> || std::is_same_v<T, double2>;
+  constexpr int kAll = kWide ? 8 : 4, kChains = kAll / kSlices;
+  constexpr int kSerial = std::is_same_v<T, double>    ? 8
+                          : std::is_same_v<T, double2> ? 3
+                          : std::is_same_v<T, float>   ? 2
+                                                       : 0;
   T part[kOut][kChains];
 #pragma unroll
   for (int j = 0; j < kOut; ++j)
@@ -189,11 +240,14 @@ __device__ __forceinline__ void small_tile(const GemmArgs& args, int64_t tile, i
     };
     if (kn == kBK) {
 #pragma unroll
-      for (int k = 0; k < kBK; k += 4)
+      for (int k = 0; k < kBK; k += kAll)
 #pragma unroll
         for (int u = 0; u < kChains; ++u) step(k + u * kSlices + slice, u);
+    } else if (K - kb <= kSerial) {
+      if (slice == 0)
+        for (int k = 0; k < kn; ++k) step(k, 0);
     } else {
-      for (int k = 0; k < kn; k += 4)
+      for (int k = 0; k < kn; k += kAll)
 #pragma unroll
         for (int u = 0; u < kChains; ++u)
           if (k + u * kSlices + slice < kn) step(k + u * kSlices + slice, u);
@@ -201,19 +255,24 @@ __device__ __forceinline__ void small_tile(const GemmArgs& args, int64_t tile, i
   }
   cp_async_wait_group<0>();
 
-  T acc[kOut];
+  ChainSum<T> acc[kOut];
 #pragma unroll
   for (int j = 0; j < kOut; ++j) {
-    acc[j] = part[j][0];
+    ChainSum<T> sum[kChains];
 #pragma unroll
-    for (int u = 1; u < kChains; ++u) acc[j] = add(acc[j], part[j][u]);
+    for (int u = 0; u < kChains; ++u) sum[u].start(part[j][u]);
+#pragma unroll
+    for (int w = kChains / 2; w > 0; w /= 2)
+#pragma unroll
+      for (int u = 0; u < w; ++u) sum[u].join(sum[u + w]);
+    acc[j] = sum[0];
   }
   if constexpr (kSlices > 1) {
     static_assert(kOut == 1 && kSlices == 2, "two k slices of one output per thread");
     if (slice > 0) sm.part[tid % (kTile * kTile)] = acc[0];
     __syncthreads();
     if (slice > 0) return;
-    acc[0] = add(acc[0], sm.part[tid]);
+    acc[0].join(sm.part[tid]);
   }
 
   const T alpha = scal<T>(args.alpha), beta = scal<T>(args.beta);
@@ -224,7 +283,7 @@ __device__ __forceinline__ void small_tile(const GemmArgs& args, int64_t tile, i
     if (!live[j]) continue;
     const int64_t m = m0 + (kNFast ? s + kSlow * j : f), n = n0 + (kNFast ? f : s + kSlow * j);
     T* p = C + offs(args.rsC, args.uC_m, m) + offs(args.csC, args.uC_n, n);
-    const T ab = mul(alpha, acc[j]);
+    const T ab = mul(alpha, acc[j].value());
     if (accumulate)
       *p = add(*p, ab);
     else if (beta_zero)

@@ -49,3 +49,58 @@ def test_small_tile_edges(ctx, torch_cuda, shape, dt, layout, splits):
     got = gc.cpu().numpy().reshape((M, N), order=order)
     bound = (4 * K + 8) * np.finfo(dt).eps / 2 * (abs(alpha) * (abs(A) @ abs(B)) * 2 + abs(beta) * abs(C) * 2)
     assert np.all(np.abs(got - ref.astype(dt)) <= bound)
+
+
+@pytest.mark.parametrize("mn", [80, 256])
+@pytest.mark.parametrize("K", [2, 3, 4, 5, 6, 9])
+@pytest.mark.parametrize("dt", [np.float64, np.float32])
+def test_few_terms_round_like_one_chain(ctx, torch_cuda, dt, K, mn):
+    """Outputs of few terms round no more than one FMA chain (rms; the chain
+    is evaluated with one rounding per term, 5% allowed for the sample)."""
+    import t1m_gb300 as t1m
+    torch = torch_cuda
+    rng = np.random.default_rng(K + mn)
+    A, B = (rng.uniform(-1, 1, s).astype(dt) for s in ((mn, K), (K, mn)))
+    wide = np.longdouble
+    chain = np.zeros((mn, mn), dt)
+    for k in range(K):
+        chain = (A[:, k:k + 1].astype(wide) * B[k].astype(wide) + chain.astype(wide)).astype(dt)
+    exact = A.astype(wide) @ B.astype(wide)
+    ga, gb = torch.from_numpy(A.ravel()).cuda(), torch.from_numpy(B.ravel()).cuda()
+    gc = torch.zeros(mn * mn, dtype=ga.dtype, device="cuda")
+    row = t1m.row_major
+    t1m.contract_scaled(1.0, t1m.tensor([mn, K], ga, row), "mk", t1m.tensor([K, mn], gb, row),
+                        "kn", 0.0, t1m.tensor([mn, mn], gc, row), "mn", ctx=ctx)
+    torch.cuda.synchronize()
+    got = gc.cpu().numpy().reshape(mn, mn)
+    rms = lambda x: float(np.sqrt(np.mean((x.astype(wide) - exact) ** 2)))
+    assert rms(got) <= 1.05 * rms(chain)
+
+
+@pytest.mark.parametrize("mn", [24, 256])
+@pytest.mark.parametrize("dt", [np.float32, np.complex64])
+def test_infinite_sums_stay_infinite(ctx, torch_cuda, dt, mn):
+    """Infinite, overflowing and NaN sums of the joined chains."""
+    import t1m_gb300 as t1m
+    torch = torch_cuda
+    K = 8
+    A, B = np.ones((mn, K), dt), np.ones((K, mn), dt)
+    A[0, 1] = np.inf                     # an infinite term
+    A[1, :] = np.finfo(np.float32).max   # overflow in the additions
+    A[2, 3] = np.nan
+    ga, gb = torch.from_numpy(A.ravel()).cuda(), torch.from_numpy(B.ravel()).cuda()
+    gc = torch.zeros(mn * mn, dtype=ga.dtype, device="cuda")
+    row = t1m.row_major
+    ctx.set_method("plain")
+    try:
+        t1m.contract_scaled(1.0, t1m.tensor([mn, K], ga, row), "mk", t1m.tensor([K, mn], gb, row),
+                            "kn", 0.0, t1m.tensor([mn, mn], gc, row), "mn", ctx=ctx)
+    finally:
+        ctx.set_method("auto")
+    torch.cuda.synchronize()
+    got = gc.cpu().numpy().reshape(mn, mn).real
+    if dt is np.float32:
+        assert np.all(np.isposinf(got[:2]))
+    else:
+        assert np.all(np.isposinf(got[1]))
+    assert np.all(np.isnan(got[2])) and np.all(got[3:] == K)
