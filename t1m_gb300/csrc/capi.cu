@@ -1082,6 +1082,10 @@ int t1m_contract(t1m_context* ctx, int dtype, const void* alpha, const t1m_tenso
     int st = build_plan(dtype, a->ndim, a->extents, sa, la, b->ndim, b->extents, sb, lb,
                         c->ndim, c->extents, sc, lc, &fresh.host, &err);
     if (st != T1M_OK) return fail(ctx, st, err);
+    int64_t per = 0;
+    if (dtype == T1M_COMPLEX64 &&
+        stream_splits(fresh.host.M, fresh.host.N, fresh.host.K, &per) > 0)
+      add_stream_order(&fresh.host);
     st = upload_plan(ctx, fresh.host, &fresh.dev);
     if (st != T1M_OK) return st;
     fresh.host.dev_stream_ka = fresh.dev.stream_ka;

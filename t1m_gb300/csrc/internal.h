@@ -53,7 +53,8 @@ struct HostPlan {
   // K offsets of A and B in an order that interleaves A's and B's unit-stride
   // K modes (4 x 8 or 8 x 4 elements first), where they are different modes of
   // such extents: a run of 32 k is then whole 32-byte sectors of both
-  // (stream.cu).  Empty otherwise.  dev_*: their device copies.
+  // (stream.cu).  Set by add_stream_order, empty otherwise.  dev_*: their
+  // device copies.
   std::vector<int64_t> stream_ka, stream_kb;
   const int64_t *dev_stream_ka = nullptr, *dev_stream_kb = nullptr;
   // Derived once per plan (the context caches plans across calls): results
@@ -84,6 +85,11 @@ int build_plan(int dtype, int na, const int64_t* ea, const int64_t* sa,
                const char* la, int nb, const int64_t* eb, const int64_t* sb,
                const char* lb, int nc, const int64_t* ec, const int64_t* sc,
                const char* lc, HostPlan* plan, std::string* err);
+
+// The streamed form's K order of a built plan.  Apart from build_plan, since
+// only single products of that form read it: built for every plan, it made
+// creating the two groups of a ring (bond 64, physical 8) take 2.6 ms, not 2.0.
+void add_stream_order(HostPlan* plan);
 
 // Device-resident copy of a plan's scatter vectors (one allocation).
 struct DevicePlan {

@@ -177,30 +177,6 @@ int build_plan(int dtype, int na, const int64_t* ea, const int64_t* sa,
   for (const Mode& m : plan->modes_k) k_by_b |= (m.s1 == 1 && m.extent > 1);
   order_modes(&plan->modes_k, k_by_b);
 
-  plan->stream_ka.clear();
-  plan->stream_kb.clear();
-  const Mode *ma = nullptr, *mb = nullptr;
-  for (const Mode& m : plan->modes_k) {
-    if (m.s0 == 1 && m.extent > 1) ma = &m;
-    if (m.s1 == 1 && m.extent > 1) mb = &m;
-  }
-  if (dtype == T1M_COMPLEX64 && ma && mb && ma != mb) {
-    const int64_t ta = ma->extent % 4 == 0 && mb->extent % 8 == 0 ? 4
-                       : ma->extent % 8 == 0 && mb->extent % 4 == 0 ? 8
-                                                                    : 0;
-    if (ta) {
-      const int64_t tb = 32 / ta;
-      std::vector<Mode> k = {{ta, ma->s0, ma->s1, ma->label},
-                             {tb, mb->s0, mb->s1, mb->label},
-                             {mb->extent / tb, mb->s0 * tb, mb->s1 * tb, mb->label},
-                             {ma->extent / ta, ma->s0 * ta, ma->s1 * ta, ma->label}};
-      for (const Mode& m : plan->modes_k)
-        if (&m != ma && &m != mb) k.push_back(m);
-      plan->stream_ka = scatter(k, false);
-      plan->stream_kb = scatter(k, true);
-    }
-  }
-
   plan->rsA = scatter(plan->modes_m, false);
   plan->rsC = scatter(plan->modes_m, true);
   plan->csB = scatter(plan->modes_n, false);
@@ -220,6 +196,30 @@ int build_plan(int dtype, int na, const int64_t* ea, const int64_t* sa,
   plan->spanB = span(nb, eb, sb);
   plan->spanC = span(nc, ec, sc);
   return T1M_OK;
+}
+
+void add_stream_order(HostPlan* plan) {
+  const Mode *ma = nullptr, *mb = nullptr;
+  for (const Mode& m : plan->modes_k) {
+    if (m.s0 == 1 && m.extent > 1) ma = &m;
+    if (m.s1 == 1 && m.extent > 1) mb = &m;
+  }
+  if (ma && mb && ma != mb) {
+    const int64_t ta = ma->extent % 4 == 0 && mb->extent % 8 == 0 ? 4
+                       : ma->extent % 8 == 0 && mb->extent % 4 == 0 ? 8
+                                                                    : 0;
+    if (ta) {
+      const int64_t tb = 32 / ta;
+      std::vector<Mode> k = {{ta, ma->s0, ma->s1, ma->label},
+                             {tb, mb->s0, mb->s1, mb->label},
+                             {mb->extent / tb, mb->s0 * tb, mb->s1 * tb, mb->label},
+                             {ma->extent / ta, ma->s0 * ta, ma->s1 * ta, ma->label}};
+      for (const Mode& m : plan->modes_k)
+        if (&m != ma && &m != mb) k.push_back(m);
+      plan->stream_ka = scatter(k, false);
+      plan->stream_kb = scatter(k, true);
+    }
+  }
 }
 
 }  // namespace gb300
