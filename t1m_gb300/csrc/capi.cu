@@ -1709,8 +1709,8 @@ extern "C" int t1m_group_destroy(t1m_group* g) {
   return T1M_OK;
 }
 
-extern "C" int t1m_group_create(t1m_context* ctx, int dtype, int n, const t1m_group_item* items,
-                                uint32_t options, t1m_group** out) {
+static int create_group(t1m_context* ctx, int dtype, int n, const t1m_group_item* items,
+                        uint32_t options, bool allow_pieces, t1m_group** out) {
   if (!ctx || !out || n < 0 || (n > 0 && !items)) return T1M_ERR_INVALID_ARGUMENT;
   *out = nullptr;
   const size_t es = elem_size(dtype);
@@ -1914,7 +1914,8 @@ extern "C" int t1m_group_create(t1m_context* ctx, int dtype, int n, const t1m_gr
 
   // Tensor-core items of family launches run over operand pieces (BF16x6)
   // where the automatic method or BF16x6 is set and workspaces are not capped.
-  const bool over_pieces = dtype == T1M_COMPLEX64 && !one_launch && ctx->opt_work_limit < 0 &&
+  const bool over_pieces = allow_pieces && dtype == T1M_COMPLEX64 && !one_launch &&
+                           ctx->opt_work_limit < 0 &&
                            (ctx->method == T1M_METHOD_AUTO ||
                             ctx->method == T1M_METHOD_TC_BF16X6);
 
@@ -2277,8 +2278,13 @@ extern "C" int t1m_group_create(t1m_context* ctx, int dtype, int n, const t1m_gr
     if (e != cudaSuccess) return fail(ctx, T1M_ERR_ALLOC, "group descriptors");
   }
   if (!pprobs.empty()) {
-    e = cudaMalloc(&g->pieces, piece_work);
-    if (e != cudaSuccess) return fail(ctx, T1M_ERR_ALLOC, "group operand pieces");
+    if (cudaMalloc(&g->pieces, piece_work) != cudaSuccess) {
+      // The pieces are an optimisation: without room for them the items run
+      // on the forms that split their operands in the kernel.
+      cudaGetLastError();
+      g.reset();
+      return create_group(ctx, dtype, n, items, options, false, out);
+    }
     uint8_t* const base = static_cast<uint8_t*>(g->pieces);
     auto place = [&](const uint8_t* off) { return base + reinterpret_cast<size_t>(off); };
     for (PieceSplit& x : psplits) x.out = place(x.out);
@@ -2333,6 +2339,11 @@ extern "C" int t1m_group_create(t1m_context* ctx, int dtype, int n, const t1m_gr
   }
   *out = g.release();
   return T1M_OK;
+}
+
+extern "C" int t1m_group_create(t1m_context* ctx, int dtype, int n, const t1m_group_item* items,
+                                uint32_t options, t1m_group** out) {
+  return create_group(ctx, dtype, n, items, options, true, out);
 }
 
 extern "C" int t1m_group_launch(t1m_group* g, t1m_report* report) {
