@@ -1336,9 +1336,10 @@ enum Family : int {
 
 // Workspace of a grouped launch's operand pieces.  Items run in batches whose
 // pieces fit it, each batch split and multiplied before the next overwrites
-// them: at half the L2 (129 MB) the pieces are mostly read, and overwritten,
-// before they reach HBM.
-constexpr size_t kGroupPieceBytes = size_t(64) << 20;
+// them.  Larger batches mean fewer launches and partial waves, smaller ones
+// pieces that stay in L2: a sweep of 128 two-site updates takes 8.26, 7.87,
+// 7.54, 7.26 and 7.20 ms at 24, 64, 128, 256 and 1024 MB.
+constexpr size_t kGroupPieceBytes = size_t(256) << 20;
 
 // Split-K inside a grouped launch: every tile covers at most kGroupKCap
 // complex (or real) K, so one long-K item (a skinny output over a big
