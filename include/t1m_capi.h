@@ -146,9 +146,11 @@ int t1m_set_method(t1m_context* ctx, int method);
  * (t1m.h:512-548); this is its parallel counterpart. */
 int t1m_set_split_k(t1m_context* ctx, int splits);
 /* Cap, in bytes, on each optional workspace of the tensor-core products: B
- * split once into panels, and dense repacks of operands that would otherwise
- * be gathered element by element.  Products whose workspace would exceed it
- * run without (same results, bit for bit; only speed changes).  -1 (the
+ * split once into panels, operand pieces, and dense repacks of operands that
+ * would otherwise be gathered element by element.  Products whose workspace
+ * would exceed it run without: the same results bit for bit under a set
+ * method; the automatic method may take another one (3xTF32 for gathered
+ * operands instead of BF16x6 over pieces).  -1 (the
  * default) = no cap, 0 = never use them.  For callers with a tight device
  * memory budget; the split-K workspace is not optional and not capped here.
  * No reference counterpart (the reference packs into one aligned_alloc'ed
@@ -163,13 +165,15 @@ int t1m_set_wait_limit(t1m_context* ctx, int64_t microseconds);
  * runs clusters of two CTAs whose MMAs (tcgen05 cta_group::2, 256 x 128 real
  * tiles) each read half of B from either CTA, where both operands load by
  * TMA; T1M_TILE_ONE keeps one 128 x 128 tile per CTA; T1M_TILE_AUTO (the
- * default) picks pairs where they apply.  The reference's counterpart is
+ * default) picks pieces, then pairs, where they apply.  The reference's counterpart is
  * BLIS's choice of micro-tile and cache blocking (bli/mappings.h:101-142). */
 #define T1M_TILE_AUTO 0
 #define T1M_TILE_ONE 1
 #define T1M_TILE_PAIR 2
-/* CTA pairs whose MMAs read both operands from shared memory, loaded by TMA
- * from copies split once into bf16 pieces (the bf16 methods; the copies
+/* CTA pairs whose MMAs read both operands from shared memory, loaded by bulk
+ * copies of operands split once into bf16 pieces (the bf16 methods, any
+ * layout; automatic where both operands load by TMA or the output is large
+ * enough, M N >= 64 (M + N); the copies
  * take the optional workspace: 2P bytes per real value of the 1M-expanded A
  * and of B, P = 3 pieces for BF16x6, 2 for BF16x3).  Same results as
  * T1M_TILE_PAIR, bit for bit.  Elsewhere it runs as T1M_TILE_PAIR. */

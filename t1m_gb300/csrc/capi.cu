@@ -1417,7 +1417,7 @@ struct TuneCache {
     cudaGetDeviceProperties(&prop, device);
     int drv = 0;
     cudaDriverGetVersion(&drv);
-    header = std::string("t1m_gb300-tune v2 ") + prop.name + " sms=" +
+    header = std::string("t1m_gb300-tune v3 ") + prop.name + " sms=" +
              std::to_string(prop.multiProcessorCount) + " driver=" + std::to_string(drv);
     for (char& ch : header)
       if (ch == '\n') ch = ' ';
@@ -1675,7 +1675,7 @@ int enqueue_group(t1m_group* g, cudaStream_t s) {
                                   static_cast<const SimtProblem*>(g->simt_dev) + l.offset, l.count,
                                   l.tiles, s);
         else
-          e = launch_simt_group(g->dtype, false,
+          e = launch_simt_group(g->dtype,
                                 static_cast<const SimtProblem*>(g->simt_dev) + l.offset, l.count,
                                 l.tiles, s);
         ++kernels;
@@ -1766,8 +1766,9 @@ static int create_group(t1m_context* ctx, int dtype, int n, const t1m_group_item
   // One persistent launch (T1M_GROUP_ONE_LAUNCH): a complex64 batch runs
   // every item on the persistent tensor-core kernel, each with its own tile;
   // dependencies and split-K reductions are resolved inside the kernel.
-  // Measured on the sweep batch of 1024 updates: 159 ms against 128 ms as
-  // family launches per level, because the second steps (N <= 4, A streamed
+  // Measured on the sweep batch of 1024 updates: 165 ms against 61 ms as
+  // family launches per level over operand pieces (128 ms without pieces):
+  // its first steps convert per tile, and the second steps (N <= 4, A streamed
   // once) run as SIMT tiles at 47 ms against 22 ms on the skinny kernel
   // (its two CTAs per SM keep 160 KB of A in flight; the persistent kernel's
   // four raw stages hold 32 KB), so the family launches stay the default.
@@ -2012,9 +2013,9 @@ static int create_group(t1m_context* ctx, int dtype, int n, const t1m_group_item
             SimtProblem sp{probe, 0};
             cudaMemcpy(pd, &sp, sizeof(sp), cudaMemcpyHostToDevice);
             int bm, bn;
-            simt_group_tile(dtype, false, &bm, &bn);
+            simt_group_tile(dtype, &bm, &bn);
             const int64_t tiles = nsp * ((hp.M + bm - 1) / bm) * ((hp.N + bn - 1) / bn);
-            le = launch_simt_group(dtype, false, static_cast<SimtProblem*>(pd), 1, tiles,
+            le = launch_simt_group(dtype, static_cast<SimtProblem*>(pd), 1, tiles,
                                    ctx->stream);
           }
           cudaEventRecord(ctx->ev[5], ctx->stream);
@@ -2244,7 +2245,7 @@ static int create_group(t1m_context* ctx, int dtype, int n, const t1m_group_item
           simts.push_back(sp);
         } else {
           int bm, bn;
-          simt_group_tile(dtype, false, &bm, &bn);
+          simt_group_tile(dtype, &bm, &bn);
           SimtProblem sp{main_args[i], L.tiles};
           L.tiles += splits[i] * ((hp.M + bm - 1) / bm) * ((hp.N + bn - 1) / bn);
           simts.push_back(sp);

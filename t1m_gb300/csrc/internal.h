@@ -133,8 +133,8 @@ constexpr uint32_t kFlagSkinnyAsync = 128u;
 constexpr int kSkinnyAsyncMaxK = 1024;
 
 // Internal method id: tensor cores, precision chosen per problem by the
-// launcher (BF16x6 where the one-tile kernel fetches both operands by TMA,
-// 3xTF32 elsewhere); the report carries the method that ran.
+// launcher (BF16x6 over operand pieces, streamed, or where the one-tile kernel
+// fetches both operands by TMA; 3xTF32 elsewhere); the report carries the method that ran.
 constexpr int kMethodTcAuto = 100;
 
 // Method of T1M_METHOD_AUTO for a planned contraction (capi.cu): the tensor
@@ -193,10 +193,9 @@ struct SimtProblem {
   GemmArgs g;
   int64_t tile_begin;
 };
-// Tile of a grouped plain launch: the regular tile, or a skinny one (128 x 16)
-// for contractions with few output columns.
-void simt_group_tile(int dtype, bool skinny, int* bm, int* bn);
-cudaError_t launch_simt_group(int dtype, bool skinny, const SimtProblem* dev, int nprob,
+// Tile of a grouped plain launch.
+void simt_group_tile(int dtype, int* bm, int* bn);
+cudaError_t launch_simt_group(int dtype, const SimtProblem* dev, int nprob,
                               int64_t total_tiles, cudaStream_t stream);
 
 // Skinny grouped launches (simt.cu): outputs of at most `nmax` (4 or 16)

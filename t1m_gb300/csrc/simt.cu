@@ -643,27 +643,13 @@ cudaError_t launch_skinny_group(int dtype, int nmax, const SimtProblem* dev, int
                    : launch_skinny_dtype<16>(dtype, dev, nprob, total_tiles, stream);
 }
 
-void simt_group_tile(int dtype, bool skinny, int* bm, int* bn) {
-  if (skinny) {
-    *bm = 128;
-    *bn = 16;
-    return;
-  }
+void simt_group_tile(int dtype, int* bm, int* bn) {
   int bk;
   simt_tile(dtype, bm, bn, &bk);
 }
 
-cudaError_t launch_simt_group(int dtype, bool skinny, const SimtProblem* dev, int nprob,
-                              int64_t total_tiles, cudaStream_t stream) {
-  if (skinny) {
-    switch (dtype) {
-      case 0: return launch_group<float, 8, 1, 16>(dev, nprob, total_tiles, stream);
-      case 1: return launch_group<double, 8, 1, 16>(dev, nprob, total_tiles, stream);
-      case 2: return launch_group<float2, 8, 1, 16>(dev, nprob, total_tiles, stream);
-      case 3: return launch_group<double2, 8, 1, 16>(dev, nprob, total_tiles, stream);
-    }
-    return cudaErrorInvalidValue;
-  }
+cudaError_t launch_simt_group(int dtype, const SimtProblem* dev, int nprob, int64_t total_tiles,
+                              cudaStream_t stream) {
   switch (dtype) {
     case 1: case 3: return launch_small_group(dtype, dev, nprob, total_tiles, stream);
     case 0: return launch_group<float, 8, 8, 8>(dev, nprob, total_tiles, stream);

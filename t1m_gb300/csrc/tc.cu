@@ -6,7 +6,8 @@
 // into real 2x2 blocks [re -im; im re] and complex B into re/im row pairs
 // (t1m.h:309-337), then runs a real GEMM of size 2M x N x 2K.  Here the same
 // real GEMM runs on the 5th-generation tensor cores, with no packed copy of
-// any tensor in HBM:
+// any tensor in HBM (products over operands split beforehand are in pieces.cu,
+// streamed ones in stream.cu):
 //
 //  1. Loader warps bring raw complex tiles into a ring of shared-memory
 //     stages.  Where the block-scatter blocks of an operand have unit stride
