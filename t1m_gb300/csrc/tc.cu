@@ -68,6 +68,7 @@
 #include "internal.h"
 #include "pieces.h"
 #include "ptx.h"
+#include "store_flags.h"
 #include "stream.h"
 #include "t1m_capi.h"
 #include "tc.h"
@@ -2159,46 +2160,6 @@ bool common_block_stride16(const std::vector<int64_t>& rows, const std::vector<i
   return true;
 }
 
-// Epilogue store flags of a problem (kFlagCPairs, kFlagCCol16) from C's row
-// and column offsets: the uniform strides where the arguments carry them (a
-// uniform bundle, the dense split-K workspace), else the plan's vectors.
-uint32_t c_store_flags(const GemmArgs& g, const std::vector<int64_t>& rsC,
-                       const std::vector<int64_t>& csC) {
-  auto col = [&](int64_t n) { return g.uC_n >= 0 ? n * g.uC_n : csC[n]; };
-  auto row = [&](int64_t m) { return g.uC_m >= 0 ? m * g.uC_m : rsC[m]; };
-  uint32_t f = 0;
-  bool col16 = true;
-  if (g.uC_n >= 0) {
-    col16 = g.uC_n == 1 || g.N <= 1;
-  } else {
-    for (int64_t b = 0; b < g.N && col16; b += 16)
-      for (int64_t i = b + 1; i < std::min<int64_t>(g.N, b + 16); ++i)
-        if (col(i) != col(b) + (i - b)) {
-          col16 = false;
-          break;
-        }
-  }
-  if (col16) f |= kFlagCCol16;
-  bool pairs = reinterpret_cast<uintptr_t>(g.C) % 16 == 0;
-  if (pairs) {
-    if (g.uC_m >= 0) {
-      pairs = g.uC_m % 2 == 0 || g.M <= 1;
-    } else {
-      for (int64_t m = 0; m < g.M && pairs; ++m) pairs = row(m) % 2 == 0;
-    }
-  }
-  if (pairs) {
-    if (g.uC_n >= 0) {
-      pairs = g.uC_n == 1;
-    } else {
-      for (int64_t n = 0; n + 1 < g.N && pairs; n += 2)
-        pairs = col(n) % 2 == 0 && col(n + 1) == col(n) + 1;
-    }
-  }
-  if (pairs) f |= kFlagCPairs;
-  return f;
-}
-
 bool make_map_f32(CUtensorMap* map, const void* base, int64_t inner, int64_t outer,
                   int64_t outer_stride, uint32_t box_inner, uint32_t box_outer, bool swizzle) {
   EncodeTiledFn fn = encode_fn();
@@ -2216,46 +2177,6 @@ bool make_map_f32(CUtensorMap* map, const void* base, int64_t inner, int64_t out
                   swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS;
-}
-
-// Real epilogue flags: kFlagCCol16 as for complex; kFlagCPairs for four
-// consecutive columns contiguous with 16-byte aligned starts.
-uint32_t c_store_flags_real(const GemmArgs& g, const std::vector<int64_t>& rsC,
-                            const std::vector<int64_t>& csC) {
-  auto col = [&](int64_t n) { return g.uC_n >= 0 ? n * g.uC_n : csC[n]; };
-  auto row = [&](int64_t m) { return g.uC_m >= 0 ? m * g.uC_m : rsC[m]; };
-  uint32_t f = 0;
-  bool col16 = true;
-  if (g.uC_n >= 0) {
-    col16 = g.uC_n == 1 || g.N <= 1;
-  } else {
-    for (int64_t b = 0; b < g.N && col16; b += 16)
-      for (int64_t i = b + 1; i < std::min<int64_t>(g.N, b + 16); ++i)
-        if (col(i) != col(b) + (i - b)) {
-          col16 = false;
-          break;
-        }
-  }
-  if (col16) f |= kFlagCCol16;
-  bool quads = reinterpret_cast<uintptr_t>(g.C) % 16 == 0;
-  if (quads) {
-    if (g.uC_m >= 0) {
-      quads = g.uC_m % 4 == 0 || g.M <= 1;
-    } else {
-      for (int64_t m = 0; m < g.M && quads; ++m) quads = row(m) % 4 == 0;
-    }
-  }
-  if (quads) {
-    if (g.uC_n >= 0) {
-      quads = g.uC_n == 1;
-    } else {
-      for (int64_t n = 0; n + 3 < g.N && quads; n += 4)
-        quads = col(n) % 4 == 0 && col(n + 1) == col(n) + 1 && col(n + 2) == col(n) + 2 &&
-                col(n + 3) == col(n) + 3;
-    }
-  }
-  if (quads) f |= kFlagCPairs;
-  return f;
 }
 
 bool tc_prepare_real(const GemmArgs& g, const HostPlan& plan, int splits, int* amode,
