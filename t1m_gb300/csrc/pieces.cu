@@ -296,7 +296,7 @@ constexpr int kPcEpiBase = 128;
 constexpr int kPcEpiWarps = 16;
 constexpr uint32_t kPcTmemCols = 512;
 constexpr int kPcBarriers = 512;
-constexpr int kPcARows = 128;          // real rows of A per CTA
+constexpr int kPcARows = kPieceCtaRows;  // real rows of A per CTA
 constexpr int kPcABytes = kPcARows * 64;
 constexpr int kPcFold = 8;             // stages per main chunk: 16 MMAs of K = 16
 
@@ -358,18 +358,13 @@ __device__ __forceinline__ void pc_fill(PcWork& w, const PieceProblem* single,
   constexpr int64_t f = kReal ? 1 : 2;
   const int64_t kb = int64_t(split) * g.k_per_split;
   const int64_t ke = min(g.K, kb + g.k_per_split);
-  const int64_t ks0 = f * kb / kPieceStageK;
-  // Row groups of this CTA's rows and columns that exist (the rest of a
-  // stage keeps old bytes: rows and columns nobody writes to C).
-  const int64_t ga = (2 * tm + rank) * (kPcARows / 8), gb = (n0 + rank * (tn / 2)) / 8;
-  const int64_t na = min(int64_t(kPcARows / 8), p->rg_a - ga);
-  const int64_t nb = min(int64_t(tn / 16), p->rg_b - gb);
-  w.a = p->a + (ks0 * P * p->rg_a + ga) * kPieceAtom;
-  w.b = p->b + (ks0 * P * p->rg_b + gb) * kPieceAtom;
+  const PieceLoads l = piece_loads(P, kReal, *p, tm, n0, rank, kb);
+  w.a = p->a + l.a;
+  w.b = p->b + l.b;
   w.pa = p->rg_a * kPieceAtom;
   w.pb = p->rg_b * kPieceAtom;
-  w.abytes = na > 0 ? static_cast<uint32_t>(na) * kPieceAtom : 0u;
-  w.bbytes = nb > 0 ? static_cast<uint32_t>(nb) * kPieceAtom : 0u;
+  w.abytes = l.abytes;
+  w.bbytes = l.bbytes;
   w.C = static_cast<uint8_t*>(g.C) + split * g.c_split_stride * (kReal ? 4 : 8);
   w.rsC = g.rsC;
   w.csC = g.csC;

@@ -59,7 +59,10 @@ struct PieceProblem {
   GemmArgs g;
   const uint8_t* a;
   const uint8_t* b;
-  int64_t rg_a, rg_b;
+  // Row groups of the arrays `a` and `b` point into (the distance from piece
+  // to piece) and of the operands themselves: an operand may be a part of its
+  // array, and nothing past its own groups is read (piece_operands).
+  int64_t rg_a, rg_b, gn_a, gn_b;
   int64_t tile_begin;      // first tile of this problem in the launch
   int32_t tiles_m, tiles_n, splits;
   int32_t tile_n;          // output columns of a tile, a multiple of 32 up to 256
@@ -69,6 +72,39 @@ struct PieceProblem {
   int32_t swapped;
   int32_t pad;
 };
+
+// Sets the row groups of a product's operands (from g's M and N); arrays of
+// `array_a` / `array_b` groups, 0: of the operand's own.
+inline void piece_operands(bool real, PieceProblem* p, int64_t array_a, int64_t array_b) {
+  p->gn_a = piece_groups((real ? 1 : 2) * p->g.M);
+  p->gn_b = piece_groups(p->g.N);
+  p->rg_a = array_a > 0 ? array_a : p->gn_a;
+  p->rg_b = array_b > 0 ? array_b : p->gn_b;
+}
+
+// What CTA `rank` of a pair loads for the tile of row tile tm and first
+// column n0, per stage and piece: 128 real rows of the first operand and half
+// of the tile's columns, as many of their row groups as exist (the rest of a
+// stage keeps old bytes: rows and columns nobody writes to C).
+constexpr int kPieceCtaRows = 128;
+struct PieceLoads {
+  int64_t a, b;             // byte offsets in the arrays at k = kb, piece 0
+  uint32_t abytes, bbytes;
+};
+__host__ __device__ inline PieceLoads piece_loads(int pieces, bool real, const PieceProblem& p,
+                                                  int64_t tm, int64_t n0, uint32_t rank,
+                                                  int64_t kb) {
+  const int64_t ks = (real ? 1 : 2) * kb / kPieceStageK;
+  const int64_t ga = (2 * tm + rank) * (kPieceCtaRows / 8), gb = (n0 + rank * (p.tile_n / 2)) / 8;
+  const int64_t la = p.gn_a - ga, lb = p.gn_b - gb, ta = kPieceCtaRows / 8, tb = p.tile_n / 16;
+  const int64_t na = la < ta ? la : ta, nb = lb < tb ? lb : tb;
+  PieceLoads l;
+  l.a = (ks * pieces * p.rg_a + ga) * kPieceAtom;
+  l.b = (ks * pieces * p.rg_b + gb) * kPieceAtom;
+  l.abytes = na > 0 ? static_cast<uint32_t>(na) * kPieceAtom : 0u;
+  l.bbytes = nb > 0 ? static_cast<uint32_t>(nb) * kPieceAtom : 0u;
+  return l;
+}
 
 // One product of a grouped launch (complex64, BF16x6): the product and the
 // split passes of its operands, without their workspace (piece_item_place).

@@ -2575,8 +2575,7 @@ void tc_piece_item(const GemmArgs& g, const HostPlan& plan, int splits, PieceIte
   const bool swap = swap_pieces(dtype, g, plan, nullptr);
   pieces_problem(dtype, g, plan, swap, &it->p);
   PieceProblem& p = it->p;
-  p.rg_a = tc_pieces_groups(dtype, true, p.g.M);
-  p.rg_b = tc_pieces_groups(dtype, false, p.g.N);
+  piece_operands(false, &p, 0, 0);
   it->op[0] = piece_split_args(dtype, !swap, swap, g, plan, nullptr, p.rg_a);
   it->op[1] = piece_split_args(dtype, swap, swap, g, plan, nullptr, p.rg_b);
   const int64_t kr = pieces_kreal(dtype, g.K);
@@ -2597,8 +2596,7 @@ static cudaError_t launch_pieces(int method, int dtype, const GemmArgs& g, const
   PieceProblem p{};
   const bool swap = swap_pieces(dtype, g, plan, ready);
   pieces_problem(dtype, g, plan, swap, &p);
-  p.rg_a = ra ? ready->a_groups : tc_pieces_groups(dtype, true, p.g.M);
-  p.rg_b = rb ? ready->b_groups : tc_pieces_groups(dtype, false, p.g.N);
+  piece_operands(real, &p, ra ? ready->a_groups : 0, rb ? ready->b_groups : 0);
   uint8_t* const w = static_cast<uint8_t*>(ws);
   const size_t abytes = ra ? 0 : piece_bytes(P, pieces_rows(dtype, true, p.g.M), pieces_kreal(dtype, g.K));
   uint8_t* const pa = ra ? static_cast<uint8_t*>(const_cast<void*>(ready->a)) : w;

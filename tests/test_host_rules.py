@@ -10,7 +10,7 @@ from t1m_gb300 import build
 ROOT = Path(__file__).resolve().parents[1]
 
 
-@pytest.mark.parametrize("name", ["store_flags"])
+@pytest.mark.parametrize("name", ["store_flags", "piece_loads"])
 def test_host_rule(name):
     out = ROOT / "tests" / "_build" / name
     out.parent.mkdir(parents=True, exist_ok=True)
