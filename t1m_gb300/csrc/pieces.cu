@@ -103,6 +103,20 @@ constexpr int kSplitRowsPer = 32;                                // source rows 
 template <bool kReal>
 constexpr int split_k() { return kReal ? 64 : 32; }              // k per block: two stages
 
+// Start of a split pass.  The kernels ahead have finished once a block is past
+// its wait: then the next kernel may start (a second split reads and writes
+// other memory than the first).  One that runs beside the split before it was
+// launched by blocks of that split past their wait, so everything ahead of
+// both has ended and written its results back; it takes them up by a fence of
+// its own (its SM may hold older lines of its source), and waits at its end.
+__device__ __forceinline__ void begin_split(bool beside) {
+  if (beside)
+    __threadfence();
+  else
+    begin_dependent();
+  release_dependents();
+}
+
 // Blocks of 32 rows x kper times two stages: read into shared memory along
 // the source's unit-stride direction, written as whole atoms (a warp writes
 // the four chunks of eight rows).  k past K is written as zeros, rows past R
@@ -120,11 +134,8 @@ split_pieces(const SplitPair pair, const PieceSplit* dev, int n) {
   constexpr int KB = split_k<kReal>();
   __shared__ T tile[kMany ? 2 : 1][kSplitRowsPer][KB + 1];
   __shared__ PieceSplit so;
-  // The kernels ahead have finished once a block is past its wait: then the
-  // next kernel may start (a second split reads and writes other memory).
   const bool beside = !dev && pair.op[0].beside;
-  if (!beside) begin_dependent();
-  release_dependents();
+  begin_split(beside);
   if (kMany && dev) {
     const int lo = block_find(n, blockIdx.x, [&](int i) { return dev[i].block_begin; });
     block_copy(&so, dev + lo);
@@ -245,8 +256,7 @@ split_pieces_step(const PieceSplit o) {
   // stores along k_hi nor the chunk reads conflict.
   constexpr int kRow = KL + 1, kPlane = R * kRow + 1;
   __shared__ T tile[KH * kPlane];
-  if (!o.beside) begin_dependent();
-  release_dependents();
+  begin_split(o.beside);
   const int64_t nhi = o.K / o.step, nlo = o.step / KL;
   const int64_t hblocks = (nhi + KH - 1) / KH;
   int64_t b = blockIdx.x;
