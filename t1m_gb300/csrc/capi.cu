@@ -266,9 +266,6 @@ int choose_method(const t1m_context* ctx, int dtype, const HostPlan& plan) {
   return ctx->method != T1M_METHOD_AUTO ? ctx->method : auto_method(dtype, plan);
 }
 
-// Workspace cap of split-K (bytes of partial products).
-constexpr size_t kMaxWorkBytes = size_t(2) << 30;
-
 // Number of K splits: enough CTAs for about one full wave when the output
 // has too few tiles, each split keeping at least four K-steps; forced by
 // t1m_set_split_k.  Returns the split count and its K length (a multiple of
@@ -385,12 +382,18 @@ int launch_product(t1m_context* ctx, int method, int dtype, size_t es, const Hos
                                          ctx->method == T1M_METHOD_AUTO)
                          : 1;
     int form = ctx->tile_form;
-    // Small outputs over long bundles stream both operands once.
+    // Small outputs over long bundles stream both operands once, where their
+    // partials (more than those of the other forms) have room.
     int64_t stream_kps = 0;
-    const int stream_s = allow_split && method == kMethodTcAuto && dtype == T1M_COMPLEX64 &&
-                                 ctx->split_k == 0 && form == T1M_TILE_AUTO && !ctx->autotune
-                             ? stream_splits(g.M, g.N, g.K, &stream_kps)
-                             : 0;
+    int stream_s = allow_split && method == kMethodTcAuto && dtype == T1M_COMPLEX64 &&
+                           ctx->split_k == 0 && form == T1M_TILE_AUTO && !ctx->autotune
+                       ? stream_splits(g.M, g.N, g.K, &stream_kps)
+                       : 0;
+    if (stream_s > 1 &&
+        ensure_work(ctx, size_t(stream_s) * size_t(g.M) * size_t(g.N) * es) != T1M_OK) {
+      cudaGetLastError();
+      stream_s = 0;
+    }
     if (stream_s > 0) {
       splits = stream_s;
       kps = stream_kps;

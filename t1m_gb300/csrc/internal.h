@@ -132,6 +132,9 @@ constexpr uint32_t kFlagCCol16 = 64u;
 constexpr uint32_t kFlagSkinnyAsync = 128u;
 constexpr int kSkinnyAsyncMaxK = 1024;
 
+// Cap on the split-K workspace of a product (bytes of partial products).
+constexpr size_t kMaxWorkBytes = size_t(2) << 30;
+
 // Internal method id: tensor cores, precision chosen per problem by the
 // launcher (BF16x6 over operand pieces, streamed, or where the one-tile kernel
 // fetches both operands by TMA; 3xTF32 elsewhere); the report carries the method that ran.

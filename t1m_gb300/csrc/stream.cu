@@ -406,11 +406,16 @@ int stream_splits(int64_t M, int64_t N, int64_t K, int64_t* k_per_split) {
     if (per <= most) break;
   }
   per = std::max<int64_t>(2, per);
-  // The partial products, written and read back, stay below the operands.
+  // The partial products, written and read back, stay below the operands, and
+  // within the split-K workspace.
   auto splits_of = [&](int64_t p) { return (stages + p - 1) / p; };
-  while (per < most && splits_of(per) * M * N * 2 > (M + N) * K) ++per;
+  auto fits = [&](int64_t s) {
+    return s * M * N * 2 <= (M + N) * K &&
+           (s == 1 || size_t(s) * size_t(M) * size_t(N) * 8 <= kMaxWorkBytes);
+  };
+  while (per < most && !fits(splits_of(per))) ++per;
   const int64_t splits = splits_of(per);
-  if (splits * M * N * 2 > (M + N) * K || splits > 65535 || tiles > 0x7fffffffLL) return 0;
+  if (!fits(splits) || splits > 65535 || tiles > 0x7fffffffLL) return 0;
   *k_per_split = per * kStK;
   return static_cast<int>(splits);
 }
