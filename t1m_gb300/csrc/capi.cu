@@ -2052,9 +2052,15 @@ static int create_group(t1m_context* ctx, int dtype, int n, const t1m_group_item
   std::vector<int> splits(n, 1);
   std::vector<int64_t> kps(n, 0), work_off(n, -1);
   size_t work_bytes = 0;
+  // A batch whose items all run on the tensor cores is one persistent launch,
+  // which splits its operands itself: no pieces there.
+  const bool all_tc =
+      n > 0 && std::all_of(family.begin(), family.end(), [](int f) { return f == kFamTC; });
   // Items of a level with few tiles (a chain's steps) split further, to
   // occupy the 76 pairs (over pieces, at least 64 complex k each) or the SMs
-  // (skinny, at least 128): as one tile, a 64 x 64 x 512 step took 72 us.
+  // (skinny, at least 128): as one tile, a 64 x 64 x 512 step took 72 us.  Not
+  // in the persistent launch, whose tiles pay more for a split than they
+  // gain: 8 items of 200 x 100 x 300 take 38 us unsplit, 223 as 5 ranges each.
   std::vector<double> level_tc(n ? *std::max_element(level.begin(), level.end()) + 1 : 1, 0.0);
   std::vector<double> level_skinny(level_tc.size(), 0.0);
   for (int i = 0; i < n; ++i) {
@@ -2067,7 +2073,7 @@ static int create_group(t1m_context* ctx, int dtype, int n, const t1m_group_item
     const HostPlan& hp = plans[i];
     if (hp.M == 0 || hp.N == 0 || hp.K == 0) continue;
     int64_t cap = kGroupKCap;
-    if (over_pieces && family[i] == kFamTC)
+    if (over_pieces && !all_tc && family[i] == kFamTC)
       cap = std::max<int64_t>(64, static_cast<int64_t>(level_tc[level[i]] / 76));
     else if (family[i] == kFamSimtSkinny)
       cap = std::max<int64_t>(128, static_cast<int64_t>(level_skinny[level[i]] / ctx->num_sms));
@@ -2096,8 +2102,6 @@ static int create_group(t1m_context* ctx, int dtype, int n, const t1m_group_item
   // the tensor cores) is ONE persistent launch: dependencies and split-K
   // reductions resolved in the kernel.  Otherwise per level one launch per
   // family, then one grouped split-K reduction.
-  bool all_tc = n > 0;
-  for (int i = 0; i < n; ++i) all_tc = all_tc && family[i] == kFamTC;
   int max_level = 0;
   for (int i = 0; i < n; ++i) max_level = std::max(max_level, level[i]);
   std::vector<TcProblem> tcs;
