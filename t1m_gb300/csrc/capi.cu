@@ -2009,6 +2009,8 @@ static int create_group(t1m_context* ctx, int dtype, int n, const t1m_group_item
             SimtProblem sp{probe, 0};
             const int nmax = hp.N <= 4 ? 4 : 16;
             if (skinny_async_ok(sp.g, hp.rsA, es, nmax)) sp.g.flags |= kFlagSkinnyAsync;
+            if (skinny_may_tall(sp.g) && skinny_tall(skinny_tall_blocks(sp.g, nsp), ctx->num_sms))
+              sp.g.flags |= kFlagSkinnyTall;
             cudaMemcpy(pd, &sp, sizeof(sp), cudaMemcpyHostToDevice);
             le = launch_skinny_group(dtype, nmax, static_cast<SimtProblem*>(pd), 1,
                                      skinny_tiles(sp.g, nsp, nmax), ctx->stream);
@@ -2227,6 +2229,15 @@ static int create_group(t1m_context* ctx, int dtype, int n, const t1m_group_item
         for (int i = 0; i < n; ++i)
           if (level[i] == lv && family[i] == fam && plans[i].N > 4) L.nmax = 16;
       }
+      int64_t tall_blocks = 0;  // of the launch, were its large items tall
+      if (fam == kFamSimtSkinny)
+        for (int i = 0; i < n; ++i) {
+          if (level[i] != lv || family[i] != fam) continue;
+          GemmArgs a = main_args[i];
+          if (skinny_async_ok(a, plans[i].rsA, es, L.nmax)) a.flags |= kFlagSkinnyAsync;
+          tall_blocks += skinny_may_tall(a) ? skinny_tall_blocks(a, splits[i])
+                                            : skinny_tiles(a, splits[i], L.nmax);
+        }
       for (int i = 0; i < n; ++i) {
         if (level[i] != lv || family[i] != fam) continue;
         const HostPlan& hp = plans[i];
@@ -2248,6 +2259,8 @@ static int create_group(t1m_context* ctx, int dtype, int n, const t1m_group_item
         } else if (fam == kFamSimtSkinny) {
           SimtProblem sp{main_args[i], L.tiles};
           if (skinny_async_ok(sp.g, hp.rsA, es, L.nmax)) sp.g.flags |= kFlagSkinnyAsync;
+          if (skinny_may_tall(sp.g) && skinny_tall(tall_blocks, ctx->num_sms))
+            sp.g.flags |= kFlagSkinnyTall;
           L.tiles += skinny_tiles(sp.g, splits[i], L.nmax);
           simts.push_back(sp);
         } else {

@@ -130,6 +130,7 @@ constexpr uint32_t kFlagCCol16 = 64u;
 // the host where A has unit K stride, 8-byte elements, 16-byte aligned rows,
 // a K chunk of at most kSkinnyAsyncMaxK and N <= 4).
 constexpr uint32_t kFlagSkinnyAsync = 128u;
+constexpr uint32_t kFlagSkinnyTall = 2048u;  // its blocks take 128 rows (skinny_async_rows)
 constexpr int kSkinnyAsyncMaxK = 1024;
 
 // Cap on the split-K workspace of a product (bytes of partial products).
@@ -216,9 +217,22 @@ __host__ __device__ constexpr int skinny_rows(bool k_unit, int nmax) {
 // kFlagSkinnyAsync for an item of a skinny launch of column bound nmax
 // (rs: the plan's A row offsets; uniform stride uA_m where >= 0).
 bool skinny_async_ok(const GemmArgs& g, const std::vector<int64_t>& rsA, size_t elem, int nmax);
-// Rows per block of the asynchronous form: several 32-row tiles share one
-// staged B chunk where there are enough of them.
-__host__ __device__ constexpr int skinny_async_rows(int64_t rows) { return rows >= 256 ? 128 : 32; }
+// Rows per block of the asynchronous form.  Tall blocks (kFlagSkinnyTall) run
+// four 32-row tiles over one staged B chunk, where a launch has enough of them
+// for two per SM (skinny_tall); 8 items of 256 x 4 x 4096 are 64 tall blocks
+// and took 59 us (float64: 171), as 256 blocks of 32 rows 42 (102), while 64
+// such items take 168 us in tall blocks and 225 in others.
+__host__ __device__ constexpr int skinny_async_rows(uint32_t flags) {
+  return flags & kFlagSkinnyTall ? 128 : 32;
+}
+inline bool skinny_tall(int64_t tall_blocks, int num_sms) { return tall_blocks >= 2 * num_sms; }
+// Items that may be tall, and their blocks.
+inline bool skinny_may_tall(const GemmArgs& g) {
+  return (g.flags & kFlagSkinnyAsync) && g.M >= 256;
+}
+inline int64_t skinny_tall_blocks(const GemmArgs& g, int splits) {
+  return int64_t(splits) * ((g.M + 127) / 128);
+}
 // Tiles of one skinny problem: splits x ceil(M / rows).
 int64_t skinny_tiles(const GemmArgs& g, int splits, int nmax);
 cudaError_t launch_skinny_group(int dtype, int nmax, const SimtProblem* dev, int nprob,

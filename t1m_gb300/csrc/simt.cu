@@ -401,9 +401,9 @@ __device__ __forceinline__ void skinny_body(const GemmArgs& g, int64_t tile, T (
 // (at most kSkinnyAsyncMaxK) is staged once, after the first A stages are
 // issued.  Warp w reduces rows 4w..4w+3, lanes over k as in skinny_body.
 // Five stages of 16 KB with two CTAs per SM keep up to 128 KB of A in flight
-// per SM.  A block runs up to four 32-row tiles over one staged B chunk, their
-// copies in one continuous ring: with one tile per block (256 KB of A) its
-// start and the B staging took a third of its time.
+// per SM.  A tall block runs up to four 32-row tiles over one staged B chunk,
+// their copies in one continuous ring: with one tile per block (256 KB of A)
+// its start and the B staging took a third of its time.
 constexpr int kSkStages = 5;
 constexpr int kSkKS = 64;  // k per stage
 constexpr size_t kSkAsyncSmem =
@@ -436,7 +436,7 @@ __device__ __forceinline__ void skinny_async_body(const GemmArgs& g, int64_t til
   T (*Bs)[kSkinnyAsyncMaxK] =
       reinterpret_cast<T (*)[kSkinnyAsyncMaxK]>(dsmem + size_t(kSkStages) * 32 * kSkKS * 8);
   const int64_t M = g.M, N = g.N, K = g.K;
-  const int rows_per = skinny_async_rows(M);
+  const int rows_per = skinny_async_rows(g.flags);
   const int64_t tiles_m = (M + rows_per - 1) / rows_per;
   const int64_t split = tile / tiles_m;
   const int64_t m0 = (tile - split * tiles_m) * rows_per;
@@ -632,7 +632,7 @@ bool skinny_async_ok(const GemmArgs& g, const std::vector<int64_t>& rsA, size_t 
 }
 
 int64_t skinny_tiles(const GemmArgs& g, int splits, int nmax) {
-  const int64_t rows = g.flags & kFlagSkinnyAsync ? skinny_async_rows(g.M)
+  const int64_t rows = g.flags & kFlagSkinnyAsync ? skinny_async_rows(g.flags)
                                                   : skinny_rows(skinny_k_lanes(g.uA_k, g.M), nmax);
   return int64_t(splits) * ((g.M + rows - 1) / rows);
 }

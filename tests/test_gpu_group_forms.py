@@ -46,3 +46,21 @@ def test_tensor_core_batch_is_not_split(ctx, torch_cuda, size, count):
         np.testing.assert_array_equal(x, y)
         ref = a.astype(np.complex128) @ b.astype(np.complex128)
         assert np.abs(x - ref).max() <= 1e-6 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("count", [1, 8, 80])
+@pytest.mark.parametrize("dtype", [np.complex64, np.float64])
+def test_skinny_rows_per_block(ctx, torch_cuda, dtype, count):
+    """Items of a few columns around the 256 rows from which a block may take
+    128 of them: few items in blocks of 32 rows, many in tall ones."""
+    import t1m_gb300 as t1m
+    torch = torch_cuda
+    shapes = [((255, 256, 257, 383, 1000)[i % 5], 1 + i % 4, 500 + 2 * i) for i in range(count)]
+    items, keep, outs = _items(t1m, torch, np.random.default_rng(71), shapes, dtype)
+    g = t1m.Group(items, ctx=ctx, graph=False)
+    g.launch()
+    torch.cuda.synchronize()
+    for (a, b), out in zip(keep, outs):
+        ref = a.astype(np.complex128) @ b.astype(np.complex128)
+        bound = 1e-6 if dtype == np.complex64 else 1e-13
+        assert np.abs(out[2].cpu().numpy() - ref).max() <= bound * np.abs(ref).max()
