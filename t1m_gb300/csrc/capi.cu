@@ -1344,12 +1344,11 @@ enum Family : int {
 // 7.54, 7.26 and 7.20 ms at 24, 64, 128, 256 and 1024 MB.
 constexpr size_t kGroupPieceBytes = size_t(256) << 20;
 
-// Split-K inside a grouped launch: every tile covers at most kGroupKCap
+// Split-K inside a grouped launch: every tile covers at most kGroupKCap (1024)
 // complex (or real) K, so one long-K item (a skinny output over a big
 // contracted bundle) spreads over many CTAs instead of leaving a tail of
 // serial tiles; partials go to the group's workspace and one reduction per
 // dependency level applies the epilogues.
-constexpr int64_t kGroupKCap = 1024;
 constexpr size_t kGroupWorkBytes = size_t(2) << 30;
 constexpr size_t kGroupItemWorkBytes = size_t(256) << 20;
 
@@ -2060,16 +2059,21 @@ static int create_group(t1m_context* ctx, int dtype, int n, const t1m_group_item
       n > 0 && std::all_of(family.begin(), family.end(), [](int f) { return f == kFamTC; });
   // Items of a level with few tiles (a chain's steps) split further, to
   // occupy the 76 pairs (over pieces, at least 64 complex k each) or the SMs
-  // (skinny, at least 128): as one tile, a 64 x 64 x 512 step took 72 us.  Not
+  // (skinny_k_cap): as one tile, a 64 x 64 x 512 step took 72 us.  Not
   // in the persistent launch, whose tiles pay more for a split than they
   // gain: 8 items of 200 x 100 x 300 take 38 us unsplit, 223 as 5 ranges each.
   std::vector<double> level_tc(n ? *std::max_element(level.begin(), level.end()) + 1 : 1, 0.0);
   std::vector<double> level_skinny(level_tc.size(), 0.0);
+  std::vector<int> level_nmax(level_tc.size(), 4);
+  for (int i = 0; i < n; ++i)
+    if (family[i] == kFamSimtSkinny && plans[i].N > 4) level_nmax[level[i]] = 16;
   for (int i = 0; i < n; ++i) {
     const HostPlan& hp = plans[i];
     if (family[i] == kFamTC)
       level_tc[level[i]] += double((hp.M + 127) / 128) * double((hp.N + 127) / 128) * double(hp.K);
-    if (family[i] == kFamSimtSkinny) level_skinny[level[i]] += double((hp.M + 31) / 32) * double(hp.K);
+    if (family[i] == kFamSimtSkinny)
+      level_skinny[level[i]] +=
+          double(skinny_tiles(args[i], 1, level_nmax[level[i]])) * double(hp.K);
   }
   for (int i = 0; i < n; ++i) {
     const HostPlan& hp = plans[i];
@@ -2078,7 +2082,7 @@ static int create_group(t1m_context* ctx, int dtype, int n, const t1m_group_item
     if (over_pieces && !all_tc && family[i] == kFamTC)
       cap = std::max<int64_t>(64, static_cast<int64_t>(level_tc[level[i]] / 76));
     else if (family[i] == kFamSimtSkinny)
-      cap = std::max<int64_t>(128, static_cast<int64_t>(level_skinny[level[i]] / ctx->num_sms));
+      cap = skinny_k_cap(dtype == T1M_COMPLEX128, args[i], level_skinny[level[i]], ctx->num_sms);
     splits[i] = group_splits(dtype, family[i], hp, es, &kps[i], cap);
     if (splits[i] > 1) {
       work_off[i] = static_cast<int64_t>(work_bytes);
@@ -2225,9 +2229,7 @@ static int create_group(t1m_context* ctx, int dtype, int n, const t1m_group_item
       if (fam == kFamSimtSkinny) {
         // One kernel instance per launch: the smallest column bound that
         // covers every item of the launch.
-        L.nmax = 4;
-        for (int i = 0; i < n; ++i)
-          if (level[i] == lv && family[i] == fam && plans[i].N > 4) L.nmax = 16;
+        L.nmax = level_nmax[lv];
       }
       int64_t tall_blocks = 0;  // of the launch, were its large items tall
       if (fam == kFamSimtSkinny)

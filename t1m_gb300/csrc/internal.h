@@ -235,6 +235,21 @@ inline int64_t skinny_tall_blocks(const GemmArgs& g, int splits) {
 }
 // Tiles of one skinny problem: splits x ceil(M / rows).
 int64_t skinny_tiles(const GemmArgs& g, int splits, int nmax);
+// Longest K a block of a grouped launch covers.
+constexpr int64_t kGroupKCap = 1024;
+// K a block of a skinny item covers at most, in a level whose blocks cover
+// `work` k in all (unsplit): levels that leave SMs idle split further, into no
+// more blocks than SMs (one more wave costs what the split gained: 8 items of
+// 64 x 16 x 2048, 64 blocks of 8 rows, take 48 us as two ranges each and 55 as
+// ten), at least 128 k each.  A split adds a reduction launch, more than the
+// lanes along k take over 512 k (1000 x 3 x 500: 17 us unsplit, 20 split).
+inline int64_t skinny_k_cap(bool complex128, const GemmArgs& g, double work, int num_sms) {
+  if (g.K <= 512 && !complex128 && skinny_k_lanes(g.uA_k, g.M)) return kGroupKCap;
+  const int64_t ranges = work > 0 ? static_cast<int64_t>(double(num_sms) * double(g.K) / work) : 1;
+  if (ranges <= 1) return kGroupKCap;
+  const int64_t steps = (g.K + 15) / 16, cap = (steps + ranges - 1) / ranges * 16;
+  return cap < 128 ? 128 : cap < kGroupKCap ? cap : kGroupKCap;
+}
 cudaError_t launch_skinny_group(int dtype, int nmax, const SimtProblem* dev, int nprob,
                                 int64_t total_tiles, cudaStream_t stream);
 
