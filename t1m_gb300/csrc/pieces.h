@@ -117,6 +117,32 @@ void tc_piece_item(const GemmArgs& g, const HostPlan& plan, int splits, PieceIte
 // Put the item's pieces at ws (bytes[0] + bytes[1] bytes).
 void piece_item_place(PieceItem* it, void* ws);
 
+// Whether a product of the automatic form runs over pieces.  `tma`: both
+// operands are plain views that the one-tile kernels load by TMA; otherwise
+// those gather them element by element, and pieces pay from 128 products per
+// element on (2 M N / (M + N)): abcd,ebfd->aecf at 1024^3 77 -> 56 us, float32
+// 1999 x 2503 x 1531 1012 -> 119; abcd,dbea->ec (96 x 64, K = 36864) 70
+// without, 86 over pieces.  Complex products that load by TMA all do.
+// float32 ones (one-tile / pieces, us, cold): the pieces are three times the
+// bytes of the operands, written and read, for a product that is a quarter
+// of a complex one.
+//   few products per element   4000 x 4 x 4000 58 / 84, 4000 x 256 x 4000
+//                              121 / 127, 2000 x 384 x 4000 102 / 97;
+//   short K                    1000 x 1024 x 256 45 / 52, x 2000 93 / 87;
+//   one wave of one-tile CTAs  4000 x 512 x 2000 60 / 72, 2000 x 768 x 4000
+//   (76 to 152 tiles)          103 / 91, 2000 x 1024 x 2000 60 / 68;
+//   more than one wave         4000 x 768 x 512 46 / 40, x 256 35 / 36.
+inline bool pieces_pay(bool real, bool tma, int64_t M, int64_t N, int64_t K) {
+  if (!tma) return M * N >= 64 * (M + N);
+  if (!real) return true;
+  if (M * N < 320 * (M + N)) return false;
+  // One-tile CTAs, with the K ranges that the precision rule asks for.
+  const int64_t tiles = ((M + 127) / 128) * ((N + 127) / 128) * ((K + 8191) / 8192);
+  if (tiles > 152) return K >= 512;
+  if (tiles >= 76) return K >= 4000 && M * N >= 500 * (M + N);
+  return K >= 1024;
+}
+
 // Thread blocks of the split pass of one operand; sets its kper.  `batch`: one
 // of several operands in a launch.
 int64_t piece_split_blocks(bool real, PieceSplit* s, bool batch = false);

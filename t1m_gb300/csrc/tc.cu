@@ -2489,19 +2489,17 @@ size_t tc_panel_bytes(int dtype, int64_t M, int64_t N, int64_t K) {
 
 // Method of the pieces form for a product, 0 where it does not run: the
 // bf16 methods (the automatic method as BF16x6).  T1M_TILE_PIECES takes it
-// for two or more 64-row M tiles; T1M_TILE_AUTO, unless both operands load
-// by TMA (`tma`), where the output is large enough that writing the pieces
-// and reading them back costs less than gathering and splitting per tile:
-// abcd,dbea->ec (96 x 64, K = 36864) takes 86 us over pieces, 70 packed and
-// split in the kernel; abcd,ebfd->aecf (1024^3) 56 against 77.
-static int pieces_method(int method, int dtype, int form, int64_t M, int64_t N, bool tma) {
+// for two or more 64-row M tiles; T1M_TILE_AUTO where they pay (pieces_pay).
+static int pieces_method(int method, int dtype, int form, int64_t M, int64_t N, int64_t K,
+                         bool tma) {
   if (M <= (dtype == T1M_COMPLEX64 ? kTileMc : 2 * kTileMc)) return 0;
   const int pm = method == kMethodTcAuto ? T1M_METHOD_TC_BF16X6 : method;
   if (pm != T1M_METHOD_TC_BF16X3 && pm != T1M_METHOD_TC_BF16X6) return 0;
   if (form == T1M_TILE_PIECES) return pm;
   if (form != T1M_TILE_AUTO) return 0;
-  // 2 M N / (M + N) >= 128: enough products per split element.
-  return tma || M * N >= 64 * (M + N) ? pm : 0;
+  // A set method keeps the size rule alone for float32 (the same bits).
+  const bool real = dtype == T1M_FLOAT32;
+  return pieces_pay(real, tma && (!real || method == kMethodTcAuto), M, N, K) ? pm : 0;
 }
 
 // Both operands a uniform view with a unit-stride direction that TMA loads.
@@ -2522,8 +2520,13 @@ int tc_pieces_count(int method, int dtype, const GemmArgs& g, const HostPlan& pl
   if (dtype == T1M_COMPLEX64) {
     TcProblem p;
     tma = tc_prepare(g, plan, 1, &p) && plain_tma(p);
+  } else {
+    int am, bm;
+    TmaMaps maps;
+    GemmArgs gr;
+    tma = tc_prepare_real(g, plan, 1, &am, &bm, &maps, &gr) && am != kGatherMK && bm != kGatherNK;
   }
-  return pieces_of(pieces_method(method, dtype, form, g.M, g.N, tma));
+  return pieces_of(pieces_method(method, dtype, form, g.M, g.N, g.K, tma));
 }
 
 // Whether the product runs with its operands exchanged: the kernel's rows
@@ -2762,7 +2765,7 @@ cudaError_t launch_tc(int method, int dtype, const GemmArgs& args, const HostPla
     GemmArgs gr;
     if (!tc_prepare_real(args, plan, splits, &am, &bm, &maps, &gr))
       return cudaErrorInvalidConfiguration;
-    if (const int pm = pieces_method(method, dtype, form, args.M, args.N,
+    if (const int pm = pieces_method(method, dtype, form, args.M, args.N, args.K,
                                      am != kGatherMK && bm != kGatherNK)) {
       if (pieces_ws_ok(pm)) {
         if (used_method) *used_method = pm;
@@ -2800,7 +2803,7 @@ cudaError_t launch_tc(int method, int dtype, const GemmArgs& args, const HostPla
   }
   TcProblem p;
   if (!tc_prepare(args, plan, splits, &p)) return cudaErrorInvalidConfiguration;
-  if (const int pm = pieces_method(method, dtype, form, args.M, args.N, plain_tma(p))) {
+  if (const int pm = pieces_method(method, dtype, form, args.M, args.N, args.K, plain_tma(p))) {
     // Operand pieces: split once (the operands not in `ready`) into the
     // panel workspace, then CTA pairs with both MMA operands in shared
     // memory.  Without the workspace the product takes the forms below.

@@ -11,7 +11,8 @@ from t1m_gb300 import build
 ROOT = Path(__file__).resolve().parents[1]
 
 
-@pytest.mark.parametrize("name", ["store_flags", "piece_loads", "stream_splits", "skinny_blocks"])
+@pytest.mark.parametrize("name", ["store_flags", "piece_loads", "stream_splits", "skinny_blocks",
+                                  "pieces_pay"])
 def test_host_rule(built_lib, name):
     out = ROOT / "tests" / "_build" / name
     out.parent.mkdir(parents=True, exist_ok=True)
