@@ -389,6 +389,9 @@ int launch_product(t1m_context* ctx, int method, int dtype, size_t es, const Hos
                            ctx->split_k == 0 && form == T1M_TILE_AUTO && !ctx->autotune
                        ? stream_splits(g.M, g.N, g.K, &stream_kps)
                        : 0;
+    if (stream_s > 0 && !stream_pays(stream_fetch(g, hp), g.M, g.N, g.K, stream_s, stream_kps,
+                                     splits, splits > 1 ? kps : g.K))
+      stream_s = 0;
     if (stream_s > 1 &&
         ensure_work(ctx, size_t(stream_s) * size_t(g.M) * size_t(g.N) * es) != T1M_OK) {
       cudaGetLastError();

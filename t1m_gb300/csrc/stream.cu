@@ -420,6 +420,20 @@ int stream_splits(int64_t M, int64_t N, int64_t K, int64_t* k_per_split) {
   return static_cast<int>(splits);
 }
 
+bool stream_pays(int fetch, int64_t M, int64_t N, int64_t K, int splits, int64_t kps, int other,
+                 int64_t other_kps) {
+  if (fetch == kStreamGathered) return true;
+  const int64_t rows = std::min(M, N), cols = std::max(M, N);
+  const int64_t tiles = ((rows + kStRows - 1) / kStRows) * ((cols + kStCols - 1) / kStCols);
+  if (fetch == kStreamSectors)
+    return tiles > 1 ? K <= 8192 : M * N <= 5000 || K <= 20000;
+  if (tiles == 1) return true;
+  auto busiest = [](int64_t ctas, int64_t k) { return double((ctas + 151) / 152 * k); };
+  const int64_t other_tiles = ((M + 63) / 64) * ((N + 127) / 128);
+  return busiest(tiles * splits, kps) * (1.25 + double(rows) / 90) <=
+         busiest(other_tiles * other, other_kps) + 140;
+}
+
 cudaError_t launch_stream(const GemmArgs& g, const StreamLayout& lay, int splits,
                           cudaStream_t stream, int* err_flag) {
   StreamArgs s;

@@ -2560,6 +2560,16 @@ static void pieces_problem(int dtype, const GemmArgs& g, const HostPlan& plan, b
   p->g.flags |= dtype == T1M_FLOAT32 ? c_store_flags_real(p->g, r, c) : c_store_flags(p->g, r, c);
 }
 
+int stream_fetch(const GemmArgs& g, const HostPlan& plan) {
+  if (g.uA_m >= 0 && g.uA_k >= 0 && g.uB_k >= 0 && g.uB_n >= 0) {
+    TcProblem p;
+    return tc_prepare(g, plan, 1, &p) && plain_tma(p) ? kStreamTma : kStreamGathered;
+  }
+  const bool apart = pack_step(plan.modes_k, false, plan.modes_m) > 0 ||
+                     pack_step(plan.modes_k, true, plan.modes_n) > 0;
+  return apart && !plan.dev_stream_ka ? kStreamSectors : kStreamGathered;
+}
+
 StreamLayout stream_layout(const GemmArgs& g, const HostPlan& plan) {
   StreamLayout l{};
   l.a_rows = pack_step(plan.modes_k, false, plan.modes_m) == 0;
