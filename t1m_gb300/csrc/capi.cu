@@ -344,6 +344,9 @@ bool ensure_opt_work(cudaStream_t user, void** buf, size_t* have, size_t bytes) 
   return true;
 }
 
+// The streamed form among the tuned ones (not a T1M_TILE_* that a caller sets).
+constexpr int kTileStream = 9;
+
 // Tuned tile form and split count of a single tensor-core product (defined
 // with the tuning cache below); false when none applies.
 bool tuned_product(t1m_context* ctx, int method, int dtype, size_t es, const HostPlan& hp,
@@ -382,16 +385,31 @@ int launch_product(t1m_context* ctx, int method, int dtype, size_t es, const Hos
                                          ctx->method == T1M_METHOD_AUTO)
                          : 1;
     int form = ctx->tile_form;
-    // Small outputs over long bundles stream both operands once, where their
-    // partials (more than those of the other forms) have room.
+    // Small outputs over long bundles stream both operands once.
     int64_t stream_kps = 0;
     int stream_s = allow_split && method == kMethodTcAuto && dtype == T1M_COMPLEX64 &&
-                           ctx->split_k == 0 && form == T1M_TILE_AUTO && !ctx->autotune
+                           ctx->split_k == 0 && form == T1M_TILE_AUTO
                        ? stream_splits(g.M, g.N, g.K, &stream_kps)
                        : 0;
     if (stream_s > 0 && !stream_pays(stream_fetch(g, hp), g.M, g.N, g.K, stream_s, stream_kps,
                                      splits, splits > 1 ? kps : g.K))
       stream_s = 0;
+    if (allow_split && ctx->autotune && ctx->split_k == 0 && ctx->tile_form == T1M_TILE_AUTO &&
+        method != T1M_METHOD_PLAIN && method != T1M_METHOD_DMMA) {
+      int tf = 0, ts = 0;
+      int64_t tk = 0;
+      if (tuned_product(ctx, method, dtype, es, hp, g, s, slot, &tf, &ts, &tk)) {
+        stream_s = tf == kTileStream ? ts : 0;
+        if (stream_s > 0) {
+          stream_kps = tk;
+        } else {
+          form = tf;
+          splits = ts;
+          kps = tk;
+        }
+      }
+    }
+    // Its partials (more than those of the other forms) may have no room.
     if (stream_s > 1 &&
         ensure_work(ctx, size_t(stream_s) * size_t(g.M) * size_t(g.N) * es) != T1M_OK) {
       cudaGetLastError();
@@ -400,16 +418,6 @@ int launch_product(t1m_context* ctx, int method, int dtype, size_t es, const Hos
     if (stream_s > 0) {
       splits = stream_s;
       kps = stream_kps;
-    }
-    if (allow_split && ctx->autotune && ctx->split_k == 0 && ctx->tile_form == T1M_TILE_AUTO &&
-        method != T1M_METHOD_PLAIN && method != T1M_METHOD_DMMA) {
-      int tf = 0, ts = 0;
-      int64_t tk = 0;
-      if (tuned_product(ctx, method, dtype, es, hp, g, s, slot, &tf, &ts, &tk)) {
-        form = tf;
-        splits = ts;
-        kps = tk;
-      }
     }
     // Split-K: the main kernel writes raw partial products (alpha = 1,
     // beta = 0) into dense workspace slices, m fastest; the reduction sums
@@ -1422,7 +1430,7 @@ struct TuneCache {
     cudaGetDeviceProperties(&prop, device);
     int drv = 0;
     cudaDriverGetVersion(&drv);
-    header = std::string("t1m_gb300-tune v3 ") + prop.name + " sms=" +
+    header = std::string("t1m_gb300-tune v4 ") + prop.name + " sms=" +
              std::to_string(prop.multiProcessorCount) + " driver=" + std::to_string(drv);
     for (char& ch : header)
       if (ch == '\n') ch = ' ';
@@ -1464,8 +1472,9 @@ std::string shape_class(int dtype, const HostPlan& hp) {
 }
 
 // Single tensor-core products: per shape class (dtype, method, log2 of M, N,
-// K, which operand directions have unit stride), the tile form (one CTA or
-// CTA pairs) and the split count (the heuristic one, half or twice it, never
+// K, which operand directions have unit stride, for complex64 how both are
+// fetched), the tile form (one CTA, CTA pairs, pieces or streamed) and the
+// split count (the heuristic one, half or twice it, never
 // below the precision rule's minimum) that ran fastest, measured once on
 // the call's own operands into scratch outputs (the split workspace: the
 // partials and a dense M x N result), three runs each after a warm-up.
@@ -1494,7 +1503,12 @@ bool tuned_product(t1m_context* ctx, int method, int dtype, size_t es, const Hos
                           std::to_string(log2_bucket(g.M)) + "," + std::to_string(log2_bucket(g.N)) +
                           "," + std::to_string(log2_bucket(g.K)) + ":" +
                           std::to_string(int(hp.uA_m == 1)) + std::to_string(int(hp.uA_k == 1)) +
-                          std::to_string(int(hp.uB_k == 1)) + std::to_string(int(hp.uB_n == 1));
+                          std::to_string(int(hp.uB_k == 1)) + std::to_string(int(hp.uB_n == 1)) +
+                          (dtype == T1M_COMPLEX64 ? std::to_string(stream_fetch(g, hp)) : "");
+  int64_t stream_kps = 0;
+  const int stream_s = method == kMethodTcAuto && dtype == T1M_COMPLEX64
+                           ? stream_splits(g.M, g.N, g.K, &stream_kps)
+                           : 0;
   std::lock_guard<std::mutex> lock(g_tune.mu);
   g_tune.load(ctx->device);
   auto it = g_tune.choice.find(key);
@@ -1502,7 +1516,46 @@ bool tuned_product(t1m_context* ctx, int method, int dtype, size_t es, const Hos
   if (it != g_tune.choice.end()) {
     code = it->second;
   } else {
+    // Raw partials (or the one dense result) into the workspace; the reduction
+    // writes a dense M x N scratch after them.
+    auto scratch_args = [&](int sp, int64_t kps, GemmArgs* gm, GemmArgs* red) {
+      const size_t slice = size_t(g.M) * size_t(g.N) * es;
+      if (ensure_work(ctx, size_t(sp + 1) * slice) != T1M_OK) return false;
+      *gm = g;
+      gm->C = ctx->work;
+      gm->rsC = gm->csC = nullptr;
+      gm->uC_m = 1;
+      gm->uC_n = g.M;
+      gm->alpha[0] = 1.0;
+      gm->alpha[1] = 0.0;
+      gm->beta[0] = gm->beta[1] = 0.0;
+      gm->flags = (g.flags & (kFlagConjA | kFlagConjB)) | kFlagBetaZero;
+      gm->k_per_split = sp > 1 ? kps : g.K;
+      gm->c_split_stride = sp > 1 ? g.M * g.N : 0;
+      *red = *gm;
+      red->C = static_cast<char*>(ctx->work) + size_t(sp) * slice;
+      return true;
+    };
     float best = 1e30f;
+    auto time_form = [&](int form_code, auto run) {
+      float total = 0;
+      for (int rep = 0; rep < 4; ++rep) {
+        cudaEventRecord(ctx->ev[4], s);
+        const cudaError_t e = run();
+        cudaEventRecord(ctx->ev[5], s);
+        if (e != cudaSuccess || cudaEventSynchronize(ctx->ev[5]) != cudaSuccess) {
+          cudaGetLastError();
+          return;
+        }
+        float ms = 0;
+        cudaEventElapsedTime(&ms, ctx->ev[4], ctx->ev[5]);
+        if (rep > 0) total += ms;  // the first run warms up
+      }
+      if (total < best) {
+        best = total;
+        code = form_code;
+      }
+    };
     for (int f : {T1M_TILE_ONE, T1M_TILE_PAIR, T1M_TILE_PIECES}) {
       // Pieces only where they run (else the same as pairs).
       if (f == T1M_TILE_PIECES && tc_pieces_count(method, dtype, g, hp, f) == 0) continue;
@@ -1512,24 +1565,8 @@ bool tuned_product(t1m_context* ctx, int method, int dtype, size_t es, const Hos
         const int64_t kps = *k_per_split;
         if (sp == last_sp) continue;
         last_sp = sp;
-        const size_t need = size_t(sp + 1) * size_t(g.M) * size_t(g.N) * es;
-        if (ensure_work(ctx, need) != T1M_OK) return false;
-        char* work = static_cast<char*>(ctx->work);
-        // Raw partials (or the one dense result) into the workspace; the
-        // reduction writes a dense M x N scratch after them.
-        GemmArgs gm = g;
-        gm.C = work;
-        gm.rsC = gm.csC = nullptr;
-        gm.uC_m = 1;
-        gm.uC_n = g.M;
-        gm.alpha[0] = 1.0;
-        gm.alpha[1] = 0.0;
-        gm.beta[0] = gm.beta[1] = 0.0;
-        gm.flags = (g.flags & (kFlagConjA | kFlagConjB)) | kFlagBetaZero;
-        gm.k_per_split = sp > 1 ? kps : g.K;
-        gm.c_split_stride = sp > 1 ? g.M * g.N : 0;
-        GemmArgs red = gm;
-        red.C = work + size_t(sp) * size_t(g.M) * size_t(g.N) * es;
+        GemmArgs gm, red;
+        if (!scratch_args(sp, kps, &gm, &red)) return false;
         const size_t pb =
             std::max(tc_panel_bytes(dtype, gm.M, gm.N, gm.K),
                      tc_pieces_bytes(dtype, tc_pieces_count(method, dtype, gm, hp, f), gm.M, gm.N,
@@ -1539,10 +1576,7 @@ bool tuned_product(t1m_context* ctx, int method, int dtype, size_t es, const Hos
         const size_t kb = tc_pack_bytes(dtype, hp);
         const bool pk = kb > 0 && (ctx->opt_work_limit < 0 || kb <= size_t(ctx->opt_work_limit)) &&
                         ensure_opt_work(s, &ctx->pack[slot], &ctx->pack_bytes[slot], kb);
-        float total = 0;
-        bool ok = true;
-        for (int rep = 0; rep < 4 && ok; ++rep) {
-          cudaEventRecord(ctx->ev[4], s);
+        time_form(f * 100 + v, [&] {
           int nk = 0, ran = method;
           std::string err;
           cudaError_t e = launch_tc(method, dtype, gm, hp, sp, s, ctx->d_err, &nk, &err, &ran,
@@ -1550,21 +1584,22 @@ bool tuned_product(t1m_context* ctx, int method, int dtype, size_t es, const Hos
                                     pan ? ctx->panel_bytes[slot] : 0,
                                     pk ? ctx->pack[slot] : nullptr, pk ? ctx->pack_bytes[slot] : 0,
                                     nullptr, f);
-          if (e == cudaSuccess && sp > 1) e = launch_splitk_reduce(dtype, work, sp, red, s);
-          cudaEventRecord(ctx->ev[5], s);
-          if (e != cudaSuccess || cudaEventSynchronize(ctx->ev[5]) != cudaSuccess) {
-            cudaGetLastError();
-            ok = false;
-            break;
-          }
-          float ms = 0;
-          cudaEventElapsedTime(&ms, ctx->ev[4], ctx->ev[5]);
-          if (rep > 0) total += ms;  // the first run warms up
-        }
-        if (ok && total < best) {
-          best = total;
-          code = f * 100 + v;
-        }
+          if (e == cudaSuccess && sp > 1) e = launch_splitk_reduce(dtype, ctx->work, sp, red, s);
+          return e;
+        });
+      }
+    }
+    if (stream_s > 0) {
+      GemmArgs gm, red;
+      if (scratch_args(stream_s, stream_kps, &gm, &red)) {
+        time_form(kTileStream * 100, [&] {
+          cudaError_t e = launch_stream(gm, stream_layout(gm, hp), stream_s, s, ctx->d_err);
+          if (e == cudaSuccess && stream_s > 1)
+            e = launch_splitk_reduce(dtype, ctx->work, stream_s, red, s);
+          return e;
+        });
+      } else {
+        cudaGetLastError();
       }
     }
     if (code < 0) return false;
@@ -1573,6 +1608,13 @@ bool tuned_product(t1m_context* ctx, int method, int dtype, size_t es, const Hos
     g_tune.save();
   }
   *form = code / 100;
+  if (*form == kTileStream) {
+    // A shape class spans sizes that do not stream.
+    if (stream_s == 0) return false;
+    *splits = stream_s;
+    *k_per_split = stream_kps;
+    return true;
+  }
   *splits = variant(code % 100);
   return true;
 }
