@@ -1968,17 +1968,57 @@ static int create_group(t1m_context* ctx, int dtype, int n, const t1m_group_item
                            (ctx->method == T1M_METHOD_AUTO ||
                             ctx->method == T1M_METHOD_TC_BF16X6);
 
+  // A batch whose items all run on the tensor cores is one persistent launch,
+  // which splits its operands itself: no pieces there.
+  // Items of a level with few tiles (a chain's steps) split further, to
+  // occupy the 76 pairs (over pieces, at least 64 complex k each) or the SMs
+  // (skinny_k_cap): as one tile, a 64 x 64 x 512 step took 72 us.  Not
+  // in the persistent launch, whose tiles pay more for a split than they
+  // gain: 8 items of 200 x 100 x 300 take 38 us unsplit, 223 as 5 ranges each.
+  bool all_tc = false;
+  const size_t nlevels = n ? size_t(*std::max_element(level.begin(), level.end()) + 1) : 1;
+  std::vector<double> level_tc, level_skinny;
+  std::vector<int> level_nmax;
+  auto sum_levels = [&] {  // from the items' families
+    all_tc = n > 0 && std::all_of(family.begin(), family.end(), [](int f) { return f == kFamTC; });
+    level_tc.assign(nlevels, 0.0);
+    level_skinny.assign(nlevels, 0.0);
+    level_nmax.assign(nlevels, 4);
+    for (int i = 0; i < n; ++i)
+      if (family[i] == kFamSimtSkinny && plans[i].N > 4) level_nmax[level[i]] = 16;
+    for (int i = 0; i < n; ++i) {
+      const HostPlan& hp = plans[i];
+      if (family[i] == kFamTC)
+        level_tc[level[i]] +=
+            double((hp.M + 127) / 128) * double((hp.N + 127) / 128) * double(hp.K);
+      if (family[i] == kFamSimtSkinny)
+        level_skinny[level[i]] +=
+            double(skinny_tiles(args[i], 1, level_nmax[level[i]])) * double(hp.K);
+    }
+  };
+  // Longest K range of item i, run as family f.
+  auto item_cap = [&](int i, int f) -> int64_t {
+    if (over_pieces && !all_tc && f == kFamTC)
+      return std::max<int64_t>(64, static_cast<int64_t>(level_tc[level[i]] / 76));
+    if (f == kFamSimtSkinny)
+      return skinny_k_cap(dtype == T1M_COMPLEX128, args[i], level_skinny[level[i]], ctx->num_sms);
+    return kGroupKCap;
+  };
+  sum_levels();
+
   // Autotuning of family launches: per shape class, time the candidate
-  // families once on a representative item (into a scratch output) and keep
-  // the fastest.
+  // families once on a representative item (into a scratch output, its K
+  // ranges those of the level before tuning) and keep the fastest.  The class
+  // says whether the tensor-core candidate runs over pieces.
   if (!one_launch && (options & T1M_GROUP_AUTOTUNE)) {
+    const bool tune_pieces = over_pieces && !all_tc;
     std::lock_guard<std::mutex> lock(g_tune.mu);
     g_tune.load(ctx->device);
     bool changed = false;
     for (int i = 0; i < n; ++i) {
       const HostPlan& hp = plans[i];
       if (hp.M == 0 || hp.N == 0 || hp.K == 0) continue;
-      const std::string key = shape_class(dtype, hp);
+      const std::string key = (tune_pieces ? "p" : "") + shape_class(dtype, hp);
       auto it = g_tune.choice.find(key);
       if (it != g_tune.choice.end()) {
         // A shape class spans N up to twice its bucket: the skinny kernel
@@ -1994,7 +2034,7 @@ static int create_group(t1m_context* ctx, int dtype, int n, const t1m_group_item
       size_t scratch_bytes = 0;
       for (int f : cands) {
         int64_t kps = 0;
-        const int sp = group_splits(dtype, f, hp, es, &kps);
+        const int sp = group_splits(dtype, f, hp, es, &kps, item_cap(i, f));
         scratch_bytes = std::max(scratch_bytes, size_t(sp) * size_t(hp.M) * size_t(hp.N) * es);
       }
       void* scratch = nullptr;
@@ -2008,9 +2048,9 @@ static int create_group(t1m_context* ctx, int dtype, int n, const t1m_group_item
       // Pieces of the tensor-core candidate, as it is launched below: into the
       // scratch partials, whose layout may order the operands differently.
       void* probe_pieces = nullptr;
-      if (over_pieces) {
+      if (tune_pieces) {
         int64_t kps = 0;
-        const int sp = group_splits(dtype, kFamTC, hp, es, &kps);
+        const int sp = group_splits(dtype, kFamTC, hp, es, &kps, item_cap(i, kFamTC));
         PieceItem pi;
         tc_piece_item(split_args(args[i], scratch, kps), hp, sp, &pi);
         if (cudaMalloc(&probe_pieces, pi.bytes[0] + pi.bytes[1]) != cudaSuccess) {
@@ -2024,7 +2064,7 @@ static int create_group(t1m_context* ctx, int dtype, int n, const t1m_group_item
         float total = 0;
         bool ok = true;
         int64_t kps = 0;
-        const int nsp = group_splits(dtype, f, hp, es, &kps);
+        const int nsp = group_splits(dtype, f, hp, es, &kps, item_cap(i, f));
         const GemmArgs probe = split_args(args[i], scratch, kps);
         for (int rep = 0; rep < 3 && ok; ++rep) {
           cudaEventRecord(ctx->ev[4], ctx->stream);
@@ -2098,36 +2138,11 @@ static int create_group(t1m_context* ctx, int dtype, int n, const t1m_group_item
   std::vector<int> splits(n, 1);
   std::vector<int64_t> kps(n, 0), work_off(n, -1);
   size_t work_bytes = 0;
-  // A batch whose items all run on the tensor cores is one persistent launch,
-  // which splits its operands itself: no pieces there.
-  const bool all_tc =
-      n > 0 && std::all_of(family.begin(), family.end(), [](int f) { return f == kFamTC; });
-  // Items of a level with few tiles (a chain's steps) split further, to
-  // occupy the 76 pairs (over pieces, at least 64 complex k each) or the SMs
-  // (skinny_k_cap): as one tile, a 64 x 64 x 512 step took 72 us.  Not
-  // in the persistent launch, whose tiles pay more for a split than they
-  // gain: 8 items of 200 x 100 x 300 take 38 us unsplit, 223 as 5 ranges each.
-  std::vector<double> level_tc(n ? *std::max_element(level.begin(), level.end()) + 1 : 1, 0.0);
-  std::vector<double> level_skinny(level_tc.size(), 0.0);
-  std::vector<int> level_nmax(level_tc.size(), 4);
-  for (int i = 0; i < n; ++i)
-    if (family[i] == kFamSimtSkinny && plans[i].N > 4) level_nmax[level[i]] = 16;
-  for (int i = 0; i < n; ++i) {
-    const HostPlan& hp = plans[i];
-    if (family[i] == kFamTC)
-      level_tc[level[i]] += double((hp.M + 127) / 128) * double((hp.N + 127) / 128) * double(hp.K);
-    if (family[i] == kFamSimtSkinny)
-      level_skinny[level[i]] +=
-          double(skinny_tiles(args[i], 1, level_nmax[level[i]])) * double(hp.K);
-  }
+  sum_levels();
   for (int i = 0; i < n; ++i) {
     const HostPlan& hp = plans[i];
     if (hp.M == 0 || hp.N == 0 || hp.K == 0) continue;
-    int64_t cap = kGroupKCap;
-    if (over_pieces && !all_tc && family[i] == kFamTC)
-      cap = std::max<int64_t>(64, static_cast<int64_t>(level_tc[level[i]] / 76));
-    else if (family[i] == kFamSimtSkinny)
-      cap = skinny_k_cap(dtype == T1M_COMPLEX128, args[i], level_skinny[level[i]], ctx->num_sms);
+    const int64_t cap = item_cap(i, family[i]);
     splits[i] = group_splits(dtype, family[i], hp, es, &kps[i], cap);
     if (splits[i] > 1) {
       work_off[i] = static_cast<int64_t>(work_bytes);
