@@ -360,8 +360,10 @@ SmallForm small_form(int dtype, int64_t M, int64_t N, int64_t K, int64_t forced)
       best = {tile, static_cast<int>(used)};
     }
   };
-  for (int64_t s = forced > 0 ? forced : 1; s <= (forced > 0 ? forced : 64); ++s) {
-    if (s > 1 && s > ksteps) break;
+  // More forced ranges than k steps of 16 (other kernels count shorter steps):
+  // the tile of as many ranges as there are steps.
+  const int64_t first = forced > 0 ? std::min(forced, ksteps) : 1;
+  for (int64_t s = first; s <= (forced > 0 ? first : std::min<int64_t>(64, ksteps)); ++s) {
     for (int tile : {16, 8}) {
       const double tiles = double((M + tile - 1) / tile) * double((N + tile - 1) / tile);
       // A block's clocks per k: its FMAs (FP64: two per clock, four per

@@ -12,7 +12,7 @@ ROOT = Path(__file__).resolve().parents[1]
 
 
 @pytest.mark.parametrize("name", ["store_flags", "piece_loads", "stream_splits", "skinny_blocks",
-                                  "pieces_pay", "stream_pays"])
+                                  "pieces_pay", "stream_pays", "small_form"])
 def test_host_rule(built_lib, name):
     out = ROOT / "tests" / "_build" / name
     out.parent.mkdir(parents=True, exist_ok=True)
