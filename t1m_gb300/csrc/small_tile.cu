@@ -193,13 +193,14 @@ __device__ __forceinline__ void small_tile(const GemmArgs& args, int64_t tile, i
   bool live[kOut];
 #pragma unroll
   for (int j = 0; j < kOut; ++j) live[j] = f < fast_n && s + kSlow * j < slow_n;
-  // Several FMA chains per output (k modulo their number, over the slices),
-  // joined at the end: shorter chains than one per K range round less.  FP64
-  // takes eight, so that an unsplit K of 256 has chains of 32 terms.  Up to
+  // Eight FMA chains per output (k modulo their number, over the slices),
+  // joined at the end: shorter chains than one per K range round less, and an
+  // unsplit K of 256 has chains of 32 terms, as short as the K ranges that
+  // larger tiles split such products into (FP32 with four chains: 20 x 248
+  // over 262 3.0e-7 off, 1.5e-7 as seven ranges).  Up to
   // kSerial terms stay in one chain: there the products rounded apart and the
   // sums that join them are more roundings than the chain's.
-  constexpr bool kWide = std::is_same_v<T, double> || std::is_same_v<T, double2>;
-  constexpr int kAll = kWide ? 8 : 4, kChains = kAll / kSlices;
+  constexpr int kAll = 8, kChains = kAll / kSlices;
   constexpr int kSerial = std::is_same_v<T, double>    ? 8
                           : std::is_same_v<T, double2> ? 3
                           : std::is_same_v<T, float>   ? 2
