@@ -676,6 +676,7 @@ cudaError_t launch_simt(int dtype, const GemmArgs& args, int splits, cudaStream_
                                                  : small_form(dtype, args.M, args.N, args.K, splits).tile;
   if (tile > 0) return launch_small(dtype, tile, args, splits, stream);
   if (dtype == 0) return launch<float, 8, 8, 8>(args, splits, stream);
+  if (dtype == 1) return launch<double, 8, 4, 8>(args, splits, stream);
   if (dtype == 2) return launch<float2, 4, 8, 8>(args, splits, stream);
   return cudaErrorInvalidValue;
 }

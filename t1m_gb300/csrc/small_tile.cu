@@ -342,6 +342,10 @@ SmallForm small_form(int dtype, int64_t M, int64_t N, int64_t K, int64_t forced)
   const double es = (cplx ? 2 : 1) * (wide ? 8 : 4);
   constexpr double kSms = 152;
   const int64_t ksteps = std::max<int64_t>(1, (K + kBK - 1) / kBK);
+  // Large float64 outputs over few k: hundreds of small blocks per SM are all
+  // start and end (4000 x 4000 over 8: 498 us against 270 on simt.cu's tile,
+  // 1000 x 1000 43 against 28).  Up to 8 k both sum one chain: the same bits.
+  const bool brief = dtype == T1M_FLOAT64 && K > 0 && K <= 8;
   SmallForm best{16, 1};
   double best_cost = 1e300;
   // Clocks of the busiest SM: whole blocks per SM times a block's k steps,
@@ -371,7 +375,13 @@ SmallForm small_form(int dtype, int64_t M, int64_t N, int64_t K, int64_t forced)
       // complex product) or the shared-memory reads of its four warps; a
       // stage of 16 k takes at least its latency.
       const double per_k = wide ? double(tile) * tile * (cplx ? 4 : 1) / 2 : (tile == 16 ? 18 : 9);
-      consider(tile, tiles, per_k, wide ? 0 : 20, s);
+      // Float64 over at most 8 k: the start and end of a block, 2100 clocks.
+      consider(tile, tiles, brief ? std::max(per_k, 2100.0 / double(K)) : per_k, wide ? 0 : 20, s);
+    }
+    if (brief) {
+      // simt.cu's tile: 8192 products per k, always 8 k of them.
+      const double tiles = double((M + 127) / 128) * double((N + 63) / 64);
+      consider(0, tiles, 8 * 8192 / 2 / double(K), 0, s);
     }
     if (!wide) {
       // simt.cu's tile: 8192 (complex, four FMAs) or 16384 products per k on

@@ -24,6 +24,12 @@ int main() {
       }
   // A large FP32 product keeps the large tile.
   if (small_form(T1M_FLOAT32, 4096, 4096, 64, 8).tile != 0) ++failures;
+  // Float64 over at most 8 k: large outputs on the large tile, small ones not.
+  if (small_form(T1M_FLOAT64, 4000, 4000, 8, 0).tile != 0) ++failures;
+  if (small_form(T1M_FLOAT64, 1000, 1000, 1, 0).tile != 0) ++failures;
+  if (small_form(T1M_FLOAT64, 200, 300, 8, 0).tile == 0) ++failures;
+  if (small_form(T1M_FLOAT64, 4000, 4000, 9, 0).tile == 0) ++failures;
+  if (small_form(T1M_COMPLEX128, 4000, 4000, 8, 0).tile == 0) ++failures;
   std::printf("%d failures\n", failures);
   return failures != 0;
 }
