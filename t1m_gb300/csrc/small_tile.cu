@@ -200,15 +200,11 @@ __device__ __forceinline__ void small_tile(const GemmArgs& args, int64_t tile, i
   // over 262 3.0e-7 off, 1.5e-7 as seven ranges).  Up to
   // kSerial terms stay in one chain: there the products rounded apart and the
   // sums that join them are more roundings than the chain's.
-  // FP32 ranges of up to 32 take four, eight terms each: joining eight adds to
-  // the latency that such a product is.
-  constexpr bool kWide = std::is_same_v<T, double> || std::is_same_v<T, double2>;
-  constexpr int kAll = 8, kChains = kAll / kSlices, kFew = 4 / kSlices;
+  constexpr int kAll = 8, kChains = kAll / kSlices;
   constexpr int kSerial = std::is_same_v<T, double>    ? 8
                           : std::is_same_v<T, double2> ? 3
                           : std::is_same_v<T, float>   ? 2
                                                        : 0;
-  const bool few = !kWide && K - kb <= 32;
   T part[kOut][kChains];
 #pragma unroll
   for (int j = 0; j < kOut; ++j)
@@ -243,27 +239,20 @@ __device__ __forceinline__ void small_tile(const GemmArgs& args, int64_t tile, i
         if (kNFast) mac(part[j][u], y, x); else mac(part[j][u], x, y);
       }
     };
-    auto steps = [&](auto count) {  // chains of the block's slices together
-      constexpr int n = decltype(count)::value;
-      if (kn == kBK) {
+    if (kn == kBK) {
 #pragma unroll
-        for (int k = 0; k < kBK; k += n)
+      for (int k = 0; k < kBK; k += kAll)
 #pragma unroll
-          for (int u = 0; u < n / kSlices; ++u) step(k + u * kSlices + slice, u);
-      } else if (K - kb <= kSerial) {
-        if (slice == 0)
-          for (int k = 0; k < kn; ++k) step(k, 0);
-      } else {
-        for (int k = 0; k < kn; k += n)
+        for (int u = 0; u < kChains; ++u) step(k + u * kSlices + slice, u);
+    } else if (K - kb <= kSerial) {
+      if (slice == 0)
+        for (int k = 0; k < kn; ++k) step(k, 0);
+    } else {
+      for (int k = 0; k < kn; k += kAll)
 #pragma unroll
-          for (int u = 0; u < n / kSlices; ++u)
-            if (k + u * kSlices + slice < kn) step(k + u * kSlices + slice, u);
-      }
-    };
-    if (few)
-      steps(std::integral_constant<int, 4>{});
-    else
-      steps(std::integral_constant<int, kAll>{});
+        for (int u = 0; u < kChains; ++u)
+          if (k + u * kSlices + slice < kn) step(k + u * kSlices + slice, u);
+    }
   }
   cp_async_wait_group<0>();
 
@@ -275,10 +264,8 @@ __device__ __forceinline__ void small_tile(const GemmArgs& args, int64_t tile, i
     for (int u = 0; u < kChains; ++u) sum[u].start(part[j][u]);
 #pragma unroll
     for (int w = kChains / 2; w > 0; w /= 2)
-      if (w < kFew || !few) {
 #pragma unroll
-        for (int u = 0; u < w; ++u) sum[u].join(sum[u + w]);
-      }
+      for (int u = 0; u < w; ++u) sum[u].join(sum[u + w]);
     acc[j] = sum[0];
   }
   if constexpr (kSlices > 1) {
