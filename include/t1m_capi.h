@@ -149,8 +149,9 @@ int t1m_set_split_k(t1m_context* ctx, int splits);
  * split once into panels, operand pieces, and dense repacks of operands that
  * would otherwise be gathered element by element.  Products whose workspace
  * would exceed it run without: the same results bit for bit under a set
- * method; the automatic method may take another one (3xTF32 for gathered
- * operands instead of BF16x6 over pieces).  -1 (the
+ * method; the automatic method may take another one (3xTF32 instead of BF16x6
+ * where operands that are not plain TMA views have no room for pieces, packs
+ * or panels; the same where their allocation fails).  -1 (the
  * default) = no cap, 0 = never use them.  For callers with a tight device
  * memory budget; the split-K workspace is not optional and not capped here.
  * No reference counterpart (the reference packs into one aligned_alloc'ed
@@ -172,8 +173,9 @@ int t1m_set_wait_limit(t1m_context* ctx, int64_t microseconds);
 #define T1M_TILE_PAIR 2
 /* CTA pairs whose MMAs read both operands from shared memory, loaded by bulk
  * copies of operands split once into bf16 pieces (the bf16 methods, any
- * layout; automatic where both operands load by TMA or the output is large
- * enough, M N >= 64 (M + N); the copies
+ * layout; automatic where the output is large enough, M N >= 64 (M + N), and
+ * for all complex64 operands that load by TMA, for float32 ones where the
+ * products per element and K are large enough to pay; the copies
  * take the optional workspace: 2P bytes per real value of the 1M-expanded A
  * and of B, P = 3 pieces for BF16x6, 2 for BF16x3).  Same results as
  * T1M_TILE_PAIR, bit for bit.  Elsewhere it runs as T1M_TILE_PAIR. */
@@ -181,11 +183,12 @@ int t1m_set_wait_limit(t1m_context* ctx, int64_t microseconds);
 int t1m_set_tile_form(t1m_context* ctx, int form);
 /* Autotuning of single tensor-core contractions (on != 0; default off): per
  * shape class (element type, method, log2 of M, N and K, which operand
- * directions have unit stride) the tile form (one CTA or CTA pairs) and the
- * split-K count (the heuristic count, half or twice it, never below the
- * automatic method's precision minimum) are measured once on the call's own
- * operands, into scratch outputs, and the fastest is cached in the same file
- * as the grouped launches' choices ($T1M_TUNE_CACHE).  Applies when the tile
+ * directions have unit stride, how complex64 operands are fetched) the tile
+ * form (one CTA, CTA pairs, pieces, or streamed) and the split-K count (the
+ * heuristic count, half or twice it, never below the automatic method's
+ * precision minimum) are measured once on the call's own operands, into scratch
+ * outputs, and the fastest is cached in the same file as the grouped launches'
+ * choices ($T1M_TUNE_CACHE).  Applies when the tile
  * form and the split count are automatic.  The reference's counterpart is
  * BLIS's fixed block sizes (bli/mappings.h:101-142). */
 int t1m_set_autotune(t1m_context* ctx, int on);

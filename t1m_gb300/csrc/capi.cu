@@ -1323,13 +1323,14 @@ extern "C" int t1m_contract_vjp(t1m_context* ctx, int dtype, const t1m_tensor* d
 
 // ------------------------------------------------------------ grouped ---
 // A batch of contractions (e.g. the updates of a tensor-network sweep) run
-// as grouped launches: every complex64 contraction with enough rows and
-// columns is a list of tiles of ONE persistent tensor-core launch; the rest
-// (other dtypes, skinny outputs) are tiles of one grouped plain launch per
-// tile shape.  Items may read the C of an earlier item (depends_on); when all
-// items are tensor-core items the dependencies are resolved inside the one
-// persistent launch, otherwise items run in dependency levels.  Optionally
-// the whole batch is captured once in a CUDA graph.  The reference has no
+// as grouped launches.  Items may read the C of an earlier item (depends_on).
+// When all items are tensor-core items (complex64 with enough rows and columns)
+// they are the tiles of one persistent launch, which resolves the dependencies.
+// Otherwise items run in dependency levels: the tensor-core items over operand
+// pieces in batches (a split pass and a product launch each; without pieces one
+// persistent launch per level), the rest (other dtypes, skinny outputs) as tiles
+// of one grouped launch per family, then one reduction.  Optionally the whole
+// batch is captured once in a CUDA graph.  The reference has no
 // batching; its counterpart is a loop of t1m::contract calls.
 #include "pieces.h"
 #include "tc.h"
@@ -2166,8 +2167,8 @@ static int create_group(t1m_context* ctx, int dtype, int n, const t1m_group_item
 
   // Launch lists.  A one-launch batch (and any batch whose items all run on
   // the tensor cores) is ONE persistent launch: dependencies and split-K
-  // reductions resolved in the kernel.  Otherwise per level one launch per
-  // family, then one grouped split-K reduction.
+  // reductions resolved in the kernel.  Otherwise per level the batches over
+  // pieces, one launch per other family, then one grouped split-K reduction.
   int max_level = 0;
   for (int i = 0; i < n; ++i) max_level = std::max(max_level, level[i]);
   std::vector<TcProblem> tcs;

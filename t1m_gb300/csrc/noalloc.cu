@@ -196,10 +196,11 @@ extern "C" int t1m_contract_noalloc(void* stream_ptr, int method, int dtype, con
   if (e != cudaSuccess) return finish(err, err_len, T1M_ERR_CUDA, cudaGetErrorString(e));
 
   // The method asked for, or t1m_contract's automatic choice (the same rule,
-  // auto_method).  Its tensor-core form picks BF16x6 or 3xTF32 per operand
-  // layout exactly as t1m_contract does; only the B panels and dense operand
-  // packs, which would need workspace, are not used here (they change
-  // speed, not results).
+  // auto_method).  Its tensor-core form picks BF16x6 or 3xTF32 by how the
+  // operands are fetched, without the forms that need workspace (operand
+  // pieces, streamed products, B panels, dense packs): t1m_contract may run
+  // BF16x6 over pieces, packs or panels, or in other K ranges, where this runs
+  // 3xTF32.  Both meet the automatic method's bound; the bits can differ.
   const bool cplx = dtype == T1M_COMPLEX64 || dtype == T1M_COMPLEX128;
   const bool is_auto = method == T1M_METHOD_AUTO;
   if (is_auto) method = auto_method(dtype, hp);

@@ -398,8 +398,9 @@ __device__ __forceinline__ void pc_fill(PcWork& w, const PieceProblem* single,
 // SMs.  Warp 0 (even CTA, one lane) issues every MMA; warp 1 (one lane per
 // CTA) loads the CTA's 128 rows of A and half of the tile's columns of B;
 // warp 2 (odd CTA, one lane) relays the arrival of its stage to the MMA
-// thread; warp 3 (one lane per CTA) finds the tiles; warps 4-19 fold chunks and write C (one TMEM lane per thread, the
-// four warpgroups each a quarter of the columns).
+// thread; warp 3 (one lane per CTA) finds the tiles; warps 4-19 fold chunks
+// and write C (one TMEM lane per thread, the four warpgroups each a quarter of
+// the columns).
 //
 // Overlap.  Loads run ahead over tile borders.  With tiles of up to 128
 // columns both chunk and correction accumulators are doubled, so a tile's
@@ -888,8 +889,9 @@ int64_t piece_split_blocks(bool real, PieceSplit* s, bool batch) {
   const int64_t kb = real ? split_k<true>() : split_k<false>();
   const int64_t rows = (s->R + kSplitRowsPer - 1) / kSplitRowsPer, kblocks = (s->K + kb - 1) / kb;
   // Up to four k blocks a thread block, while the GPU (152 SMs x 8 blocks)
-  // keeps a round of them, counting four operands of a batch (4096^2 twice: 163 us with one, 140 with four;
-  // 1024^2: 9.5 us with one, 12.3 on the form for several).
+  // keeps a round of them, counting four operands of a batch (4096^2 twice:
+  // 163 us with one, 140 with four; 1024^2: 9.5 us with one, 12.3 on the form
+  // for several).
   s->kper = static_cast<int32_t>(
       std::max<int64_t>(1, std::min<int64_t>(4, rows * kblocks / (batch ? 304 : 1216))));
   return rows * ((kblocks + s->kper - 1) / s->kper);

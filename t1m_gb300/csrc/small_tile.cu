@@ -22,7 +22,7 @@
 // Tiles are gathered through the scatter vectors as in simt.cu (the plain
 // form; replaces the reference's include/t1m/t1m.h:432-557 in FP64), each
 // operand's unit-stride direction on consecutive threads, through a
-// three-stage cp.async ring.  Consecutive threads write along C's unit stride.
+// cp.async ring (ring_stages).  Consecutive threads write along C's unit stride.
 #include <algorithm>
 #include <cstdint>
 #include <type_traits>

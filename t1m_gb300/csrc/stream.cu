@@ -16,9 +16,10 @@
 // A stage is 32 complex k.  Where each operand has its unit stride along
 // another K mode, the K order interleaves them (HostPlan::stream_k: 4 x 8 or 8
 // x 4), so a stage is whole 32-byte sectors of both.  K ranges hold at most 12
-// stages: three main chunk accumulators of 16 MMAs each and the corrections
-// fill TMEM, and nothing is folded before the end (the precision of pieces.cu,
-// whose chunks are as long).
+// stages (outputs of up to 64 columns: 28): three (seven) main chunk
+// accumulators of 16 MMAs each and the corrections fill TMEM, and nothing is
+// folded before the end (the precision of pieces.cu, whose chunks are as long).
+// Which products run so: stream_pays (stream.h).
 #include <cuda_runtime.h>
 
 #include <algorithm>
