@@ -123,24 +123,26 @@ void piece_item_place(PieceItem* it, void* ws);
 // element on (2 M N / (M + N)): abcd,ebfd->aecf at 1024^3 77 -> 56 us, float32
 // 1999 x 2503 x 1531 1012 -> 119; abcd,dbea->ec (96 x 64, K = 36864) 70
 // without, 86 over pieces.  Complex products that load by TMA all do.
-// float32 ones (one-tile / pieces, us, cold): the pieces are three times the
-// bytes of the operands, written and read, for a product that is a quarter
-// of a complex one.
-//   few products per element   4000 x 4 x 4000 58 / 84, 4000 x 256 x 4000
-//                              121 / 127, 2000 x 384 x 4000 102 / 97;
-//   short K                    1000 x 1024 x 256 45 / 52, x 2000 93 / 87;
-//   one wave of one-tile CTAs  4000 x 512 x 2000 60 / 72, 2000 x 768 x 4000
-//   (76 to 152 tiles)          103 / 91, 2000 x 1024 x 2000 60 / 68;
-//   more than one wave         4000 x 768 x 512 46 / 40, x 256 35 / 36.
+// float32 ones (one-tile / pieces, us a call queued among others over 260 MB of
+// inputs): the pieces are three times the bytes of the operands, written and
+// read, for a product that is a quarter of a complex one.
+//   short K                     1000 x 1024 x 100 13.3 / 15.0, x 512 19.2 / 16.4;
+//   few products per element    4000 x 4 x 4000 0.75 times as fast over pieces,
+//                               1000 x 128 x 512 1.12, x 4000 0.86 times,
+//                               1000 x 400 x 4000 1.10;
+//   one wave of one-tile CTAs   4000 x 512 x 1024 0.92 times, 2000 x 768 x 1024
+//   (76 to 152 tiles)           1.12, 2000 x 1024 x 256 0.86, x 4000 1.11;
+//   more than one wave          4000 x 768 x 100 1.34, 2000 x 2000 x 2000 1.27.
+// (After a flush of L2, code included, and alone, the pieces' extra launches
+// cost up to 10 us more; calls of a program in a row do not see that.)
 inline bool pieces_pay(bool real, bool tma, int64_t M, int64_t N, int64_t K) {
   if (!tma) return M * N >= 64 * (M + N);
   if (!real) return true;
-  if (M * N < 320 * (M + N)) return false;
   // One-tile CTAs, with the K ranges that the precision rule asks for.
   const int64_t tiles = ((M + 127) / 128) * ((N + 127) / 128) * ((K + 8191) / 8192);
-  if (tiles > 152) return K >= 512;
-  if (tiles >= 76) return K >= 4000 && M * N >= 500 * (M + N);
-  return K >= 1024;
+  if (tiles > 152) return K >= 96;
+  if (tiles >= 76) return K >= 1024 && M * N >= 500 * (M + N);
+  return K >= 300 && (M * N >= 220 * (M + N) || (M * N >= 50 * (M + N) && K <= 1536));
 }
 
 // Thread blocks of the split pass of one operand; sets its kper.  `batch`: one

@@ -427,12 +427,12 @@ bool stream_pays(int fetch, int64_t M, int64_t N, int64_t K, int splits, int64_t
   const int64_t rows = std::min(M, N), cols = std::max(M, N);
   const int64_t tiles = ((rows + kStRows - 1) / kStRows) * ((cols + kStCols - 1) / kStCols);
   if (fetch == kStreamSectors)
-    return tiles > 1 ? K <= 8192 : M * N <= 5000 || K <= 20000;
-  if (tiles == 1) return true;
+    return tiles > 1 ? K <= 14000 : M * N <= 5000 || K <= 24000;
+  if (M > 64 || tiles == 1 || tiles * ((K + kStK - 1) / kStK) <= 7 * 152) return true;
   auto busiest = [](int64_t ctas, int64_t k) { return double((ctas + 151) / 152 * k); };
-  const int64_t other_tiles = ((M + 63) / 64) * ((N + 127) / 128);
-  return busiest(tiles * splits, kps) * (1.25 + double(rows) / 90) <=
-         busiest(other_tiles * other, other_kps) + 140;
+  const int64_t other_tiles = (N + 127) / 128;  // 64 rows: one tile
+  return busiest(tiles * splits, kps) * (1.1 + double(rows) / 90) <=
+         busiest(other_tiles * other, other_kps);
 }
 
 cudaError_t launch_stream(const GemmArgs& g, const StreamLayout& lay, int splits,

@@ -24,19 +24,21 @@ enum : int {
 };
 // Whether a product for which stream_splits gives `splits` ranges of `kps` runs
 // streamed; `other`, `other_kps`: the K ranges it has otherwise (tiles of 64
-// x 128).  Measured in us, other form / streamed, cold:
-//   gathered: always (96 x 64, K = 36864 interleaved 84 / 59; 500 x 33 210 / 140;
-//     63 x 1001 over 40001 593 / 223; 8 x 16001 over 8191 1980 / 421);
-//   TMA: outputs of one tile (64 x 128 over 40000 51 / 51, 8 x 64 over 1024 1.2
-//     times), and larger ones while the k that the busiest SM goes through,
-//     1.25 (one row) to 2 (64 rows) times as long each as in the other form,
-//     cost no more than the launch saves (140 k): 64 x 1000 over 2048
-//     1.04 times, over 40000 131 / 220; 64 x 16000 over 1024 62 / 147,
-//     16000 x 33 over 1024 124 / 113;
-//   sectors: outputs of one tile, over K up to 20000 where they are large
-//     (95 x 63: 48 / 49 over 6061, 82 / 90 over 33511; 64 x 64 67 / 57 there),
-//     larger ones up to 8192 (97 x 65: 48 / 46 over 6061, 56 / 75 over 16983;
-//     500 x 33: 64 / 67, 125 / 179).
+// x 128).  Measured as speed against the other form, calls queued among others
+// over 260 MB of inputs:
+//   gathered: always (96 x 64, K = 36864 interleaved 1.7; 500 x 33 1.6; 64 x
+//     129 over 40000 2.1);
+//   TMA, more than 64 rows of A (the other form runs over pieces): always (96 x
+//     96 over 40000 1.5, 4000 x 33 over 1024 1.8; worst 65 x 4000 0.9);
+//   TMA, otherwise: outputs of one tile (64 x 128 over 40000 1.1) and up to
+//     seven stages of an SM (64 x 1000 over 4096 1.1, 8 x 4000 over 1024 1.5),
+//     beyond only while the k that the busiest SM goes through, 1.1 (one row) to
+//     1.8 (64 rows) times as long each, are fewer than in the other form (64 x
+//     1000 over 8192 0.8, 64 x 16000 over 1024 0.4, 8 x 4000 over 8192 1.5);
+//   sectors: outputs of one tile, large ones over K up to 24000 (64 x 64 over
+//     40425 1.1; 95 x 63 over 16983 1.0, 40425 0.85), larger ones up to 14000
+//     (70 x 70 over 13824 1.2, 23693 0.9; 97 x 65 1.0 over 8645, 0.8 over
+//     16983; 500 x 33 1.1 over 13824, 0.5 over 23693).
 bool stream_pays(int fetch, int64_t M, int64_t N, int64_t K, int splits, int64_t kps, int other,
                  int64_t other_kps);
 

@@ -16,14 +16,18 @@ int main() {
         ++failures;
       }
   };
-  for (int64_t n : {1, 4, 16, 64, 128, 256}) {
+  for (int64_t n : {1, 4, 16, 64}) {
     expect(false, true, true, 4000, n, 4000);
     expect(false, true, true, 300, n, 20000);
   }
-  expect(false, true, true, 4000, 512, 256);
+  expect(false, true, true, 4000, 128, 4000);
+  expect(false, true, true, 300, 256, 20000);
+  expect(false, true, true, 1000, 1024, 100);
+  expect(false, true, true, 4000, 512, 1024);
   expect(false, true, true, 2000, 1024, 512);
-  expect(true, true, true, 2000, 768, 4000);
-  expect(true, true, true, 4000, 768, 2000);
+  expect(true, true, true, 1000, 128, 512);
+  expect(true, true, true, 2000, 768, 2000);
+  expect(true, true, true, 4000, 768, 100);
   expect(true, true, true, 2048, 2048, 2048);
   expect(true, true, true, 1000, 1024, 4000);
   expect(true, true, false, 1999, 2503, 1531);

@@ -22,7 +22,9 @@ int main() {
     expect(true, kStreamTma, 96, 64, k, 76);
     expect(true, kStreamSectors, 64, 64, k, 75);
   }
-  expect(true, kStreamTma, 64, 1000, 2048, 19);
+  expect(true, kStreamTma, 64, 1000, 4096, 19);
+  expect(true, kStreamTma, 96, 96, 40000, 38);
+  expect(true, kStreamTma, 65, 1000, 40000, 10);
   expect(false, kStreamTma, 64, 1000, 40000, 19);
   expect(false, kStreamTma, 64, 256, 40000, 76);
   expect(false, kStreamTma, 64, 16000, 1024, 1);
@@ -31,6 +33,7 @@ int main() {
   expect(true, kStreamSectors, 95, 63, 6061, 75);
   expect(false, kStreamSectors, 95, 63, 33511, 75);
   expect(true, kStreamSectors, 97, 65, 6061, 75);
+  expect(true, kStreamSectors, 70, 70, 13824, 75);
   expect(false, kStreamSectors, 97, 65, 16983, 75);
   expect(false, kStreamSectors, 500, 33, 40425, 19);
   std::printf("%d failures\n", failures);
