@@ -1814,7 +1814,7 @@ static int create_group(t1m_context* ctx, int dtype, int n, const t1m_group_item
   // One persistent launch (T1M_GROUP_ONE_LAUNCH): a complex64 batch runs
   // every item on the persistent tensor-core kernel, each with its own tile;
   // dependencies and split-K reductions are resolved inside the kernel.
-  // Measured on the sweep batch of 1024 updates: 165 ms against 61 ms as
+  // Measured on the sweep batch of 1024 updates: 165 ms against 58 ms as
   // family launches per level over operand pieces (128 ms without pieces):
   // its first steps convert per tile, and the second steps (N <= 4, A streamed
   // once) run as SIMT tiles at 47 ms against 22 ms on the skinny kernel
