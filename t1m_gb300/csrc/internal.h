@@ -220,8 +220,8 @@ bool skinny_async_ok(const GemmArgs& g, const std::vector<int64_t>& rsA, size_t 
 // Rows per block of the asynchronous form.  Tall blocks (kFlagSkinnyTall) run
 // four 32-row tiles over one staged B chunk, where a launch has enough of them
 // for two per SM (skinny_tall); 8 items of 256 x 4 x 4096 are 64 tall blocks
-// and took 59 us (float64: 171), as 256 blocks of 32 rows 42 (102), while 64
-// such items take 168 us in tall blocks and 225 in others.
+// and took 58 us (float64: 172), as 256 blocks of 32 rows 36 (89), while 64
+// such items take 165 us in tall blocks and took 224 in others.
 __host__ __device__ constexpr int skinny_async_rows(uint32_t flags) {
   return flags & kFlagSkinnyTall ? 128 : 32;
 }

@@ -126,7 +126,7 @@ void piece_item_place(PieceItem* it, void* ws);
 // float32 ones (one-tile / pieces, us a call queued among others over 260 MB of
 // inputs): the pieces are three times the bytes of the operands, written and
 // read, for a product that is a quarter of a complex one.
-//   short K                     1000 x 1024 x 100 13.3 / 15.0, x 512 19.2 / 16.4;
+//   short K                     1000 x 1024 x 100 12.8 / 14.4, x 512 59 / 51;
 //   few products per element    4000 x 4 x 4000 0.75 times as fast over pieces,
 //                               1000 x 128 x 512 1.12, x 4000 0.86 times,
 //                               1000 x 400 x 4000 1.10;
