@@ -427,7 +427,7 @@ bool stream_pays(int fetch, int64_t M, int64_t N, int64_t K, int splits, int64_t
   const int64_t rows = std::min(M, N), cols = std::max(M, N);
   const int64_t tiles = ((rows + kStRows - 1) / kStRows) * ((cols + kStCols - 1) / kStCols);
   if (fetch == kStreamSectors)
-    return tiles > 1 ? K <= 14000 : M * N <= 5000 || K <= 24000;
+    return tiles == 1 || K <= 14000;
   if (M > 64 || tiles == 1 || tiles * ((K + kStK - 1) / kStK) <= 7 * 152) return true;
   auto busiest = [](int64_t ctas, int64_t k) { return double((ctas + 151) / 152 * k); };
   const int64_t other_tiles = (N + 127) / 128;  // 64 rows: one tile

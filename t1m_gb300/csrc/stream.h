@@ -35,10 +35,10 @@ enum : int {
 //     beyond only while the k that the busiest SM goes through, 1.1 (one row) to
 //     1.8 (64 rows) times as long each, are fewer than in the other form (64 x
 //     1000 over 8192 0.8, 64 x 16000 over 1024 0.4, 8 x 4000 over 8192 1.5);
-//   sectors: outputs of one tile, large ones over K up to 24000 (64 x 64 over
-//     40425 1.1; 95 x 63 over 16983 1.0, 40425 0.85), larger ones up to 14000
-//     (70 x 70 over 13824 1.2, 23693 0.9; 97 x 65 1.0 over 8645, 0.8 over
-//     16983; 500 x 33 1.1 over 13824, 0.5 over 23693).
+//   sectors: outputs of one tile (64 x 64 over 40425 1.1; 95 x 63 over 16983 1.0,
+//     33511 0.9, kept for its error, 1.7e-7 against 1.9e-7), larger ones over K
+//     up to 14000 (70 x 70 over 13824 1.2, 23693 0.9; 97 x 65 1.0 over 8645,
+//     0.8 over 16983; 500 x 33 1.1 over 13824, 0.5 over 23693).
 bool stream_pays(int fetch, int64_t M, int64_t N, int64_t K, int splits, int64_t kps, int other,
                  int64_t other_kps);
 

@@ -31,7 +31,7 @@ int main() {
   expect(false, kStreamTma, 8, 16000, 1024, 1);
   expect(true, kStreamTma, 16000, 33, 1024, 1);
   expect(true, kStreamSectors, 95, 63, 6061, 75);
-  expect(false, kStreamSectors, 95, 63, 33511, 75);
+  expect(true, kStreamSectors, 95, 63, 33511, 75);
   expect(true, kStreamSectors, 97, 65, 6061, 75);
   expect(true, kStreamSectors, 70, 70, 13824, 75);
   expect(false, kStreamSectors, 97, 65, 16983, 75);
